@@ -63,30 +63,288 @@ __device__ ArgMax block_argmax(ArgMax a, ArgMax* scratch) {
   return scratch[32];
 }
 
-// One block per row.  params per row: temperature[m], top_k[m], stream[m] (request's random stream),
-// counter[m] (request's step).  Rows with temperature <= 1e-3 take the argmax.
-__global__ void __launch_bounds__(1024)
-sample_kernel(const float* __restrict__ logits, int V, long long ld, const float* __restrict__ temperature,
-              const int* __restrict__ top_k, const unsigned long long* __restrict__ streams,
-              const unsigned long long* __restrict__ counters, unsigned long long seed, int* __restrict__ out) {
-  JLX_TL(TL_SAMPLE);
-  __shared__ ArgMax scratch[33];
-  __shared__ float fscratch[33];
-  __shared__ float topv[SAMPLE_MAX_K];
-  __shared__ int topi[SAMPLE_MAX_K];
-  __shared__ float partial[1024];
-  const int m = blockIdx.x;
-  const float* row = logits + (size_t)m * ld;
-  const float temp = temperature ? temperature[m] : 0.f;
+// ---- sampling in three launches.  A row's logits are read once, by several blocks:
+//
+//   sample_top_kernel     (row, chunk): the chunk's `k` largest (value, index), in no order; one for rows that need only
+//                         their largest (greedy rows, and rows that draw from the whole vocabulary).
+//   sample_spans_kernel   (row, spans): for rows that draw from the whole vocabulary, the sums of exp over SAMPLE_SPANS
+//                         contiguous spans of the row; blocks of other rows leave at once.
+//   sample_pick_kernel    (row): the chunks' lists merged, the draw, the choice.
+//
+// What bounds it: the one pass over the logits (64 rows x 202048: 52 MB, 8 us at the copy rate), then the latency of three
+// dependent launches and of the counts that find the k-th largest.  The kernel that was here walked a row once per chosen
+// token in one block: 64 rows, top 64: 3630 us; these three: 48 us (greedy rows 24 us, the whole vocabulary 93 us: the
+// sums of the spans, a sequential prefix over them and one over the chosen span).
+// Every sum runs in the order it had there (the chosen tokens in descending order; the spans each in index order, then
+// the tree over the spans), so the drawn tokens are the same.
+#define SAMPLE_THREADS 512        // of sample_top_kernel: a block's threads, and so the strands it cuts a chunk into
+#define SAMPLE_STRAND 64          // values that one thread reads at most
+#define SAMPLE_MAX_CANDIDATES (SAMPLE_MAX_K * SAMPLE_STRAND)
+#define SAMPLE_SPANS 1024
+#define SAMPLE_SPANS_PER_BLOCK 64
+#define SAMPLE_PIECE 64           // values of each span that a block holds at once
 
-  ArgMax best{0.f, -1};
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    const float v = row[i];
-    if (!isnan(v)) best = better(best, ArgMax{v, i});
+// (value, index) as one number: larger values first, equal values by the lower index; 0: no entry (no number maps there).
+typedef unsigned long long SampleKey;
+__device__ __forceinline__ unsigned sample_order(float v) {  // 0 for what is not a number; -0 counts as +0
+  const unsigned u = __float_as_uint(v + 0.f);
+  return isnan(v) ? 0u : ((u & 0x80000000u) ? ~u : (u | 0x80000000u));
+}
+__device__ __forceinline__ SampleKey sample_key(unsigned order, int i) {
+  return order == 0u ? 0ull : ((SampleKey)order << 32) | (unsigned)(0xffffffffu - (unsigned)i);
+}
+__device__ __forceinline__ float sample_value(SampleKey k) {
+  const unsigned o = (unsigned)(k >> 32);
+  return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
+}
+__device__ __forceinline__ int sample_index(SampleKey k) { return (int)(0xffffffffu - (unsigned)k); }
+
+// Sorts n keys (a power of two) in shared memory, largest first; all threads of the block call it.
+__device__ __forceinline__ void sample_sort(SampleKey* a, int n) {
+  for (int size = 2; size <= n; size <<= 1)
+    for (int step = size >> 1; step > 0; step >>= 1) {
+      __syncthreads();
+      for (int t = threadIdx.x; t < (n >> 1); t += blockDim.x) {
+        const int i = 2 * t - (t & (step - 1)), j = i + step;
+        const SampleKey x = a[i], y = a[j];
+        if (((i & size) == 0) == (x < y)) {
+          a[i] = y;
+          a[j] = x;
+        }
+      }
+    }
+  __syncthreads();
+}
+
+__device__ __forceinline__ int sample_pow2(int n) {
+  int p = 2;
+  while (p < n) p <<= 1;
+  return p;
+}
+
+// The candidates a row's draw chooses among: its largest alone, all (0), or the k largest.
+__device__ __forceinline__ int sample_k(const float* temperature, const int* top_k, int m, int V) {
+  if (!temperature || temperature[m] <= 1e-3f) return 1;
+  const int k = top_k ? top_k[m] : 0;
+  return k <= 0 ? 0 : min(min(k, V), SAMPLE_MAX_K);  // the host refuses larger k before the launch
+}
+
+// The largest key `from` that at least k of the block's keys (one per thread, all different or 0) reach: bit by bit, each
+// bit one count over the block, until exactly k reach it (a dozen or two bits; a sort of the 512 keys was a third of the
+// kernel).  Fewer than k keys that are not 0: 1.
+__device__ __forceinline__ SampleKey sample_kth(SampleKey mine, int k) {
+  SampleKey from = 0ull;
+  if (__syncthreads_count(mine != 0ull) <= k) return 1ull;
+  for (int bit = 63; bit >= 0; --bit) {
+    const SampleKey t = from | (1ull << bit);
+    const int reach = __syncthreads_count(mine >= t);
+    if (reach >= k) from = t;
+    if (reach == k) break;
   }
-  best = block_argmax(best, scratch);
-  if (temp <= 1e-3f || best.i < 0) {
-    if (threadIdx.x == 0) out[m] = best.i < 0 ? 0 : best.i;
+  return from;
+}
+
+// A chunk's k largest, in no order: every thread finds the largest of its strand; a value among the chunk's k largest lies
+// in a strand whose largest is among the k largest of those, so only these k threads read their strand again (at most
+// SAMPLE_STRAND values each: the list of candidates cannot overflow) and keep what reaches the k-th strand's largest.
+__global__ void __launch_bounds__(SAMPLE_THREADS, 4)  // 64 rows of 202048 are 512 blocks: all resident at once
+sample_top_kernel(const float* __restrict__ logits, int V, long long ld, int chunk, const float* __restrict__ temperature,
+                  const int* __restrict__ top_k, SampleKey* __restrict__ lists) {
+  JLX_TL(TL_SAMPLE);
+  __shared__ SampleKey keys[SAMPLE_MAX_CANDIDATES];
+  __shared__ int count, kept;
+  const int m = blockIdx.x, tid = threadIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int k = max(1, sample_k(temperature, top_k, m, V));
+  const float* row = logits + (size_t)m * ld;
+  const int lo = blockIdx.y * chunk, hi = min(V, lo + chunk);
+  SampleKey* list = lists + ((size_t)m * gridDim.y + blockIdx.y) * SAMPLE_MAX_K;
+  // one strand: every SAMPLE_THREADS-th group of four values, then every SAMPLE_THREADS-th of the rest; AHEAD groups are
+  // in flight together
+  float best = -INFINITY;
+  int at = -1;
+  const bool vec = (ld & 3) == 0 && ((uintptr_t)logits & 15) == 0;  // chunks are multiples of 4
+  const int hi4 = vec ? lo + ((hi - lo) & ~3) : lo;
+  constexpr int AHEAD = 4, STEP = 4 * SAMPLE_THREADS;
+  for (int i0 = lo + 4 * tid; i0 < hi4; i0 += AHEAD * STEP) {
+    float4 v[AHEAD];
+#pragma unroll
+    for (int g = 0; g < AHEAD; ++g)
+      v[g] = i0 + g * STEP < hi4 ? *reinterpret_cast<const float4*>(row + i0 + g * STEP) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+#pragma unroll
+    for (int g = 0; g < AHEAD; ++g) {
+      const int i = i0 + g * STEP;
+      if (v[g].x > best) { best = v[g].x; at = i; }
+      if (v[g].y > best) { best = v[g].y; at = i + 1; }
+      if (v[g].z > best) { best = v[g].z; at = i + 2; }
+      if (v[g].w > best) { best = v[g].w; at = i + 3; }
+    }
+  }
+#pragma unroll 4
+  for (int i = hi4 + tid; i < hi; i += SAMPLE_THREADS) {
+    const float v = row[i];
+    if (v > best) { best = v; at = i; }
+  }
+  if (at < 0) {  // nothing above minus infinity: its first place, if the strand has one
+    for (int i = lo + 4 * tid; i < hi4 && at < 0; i += STEP)
+      for (int c = 3; c >= 0; --c)
+        if (!isnan(row[i + c])) at = i + c;
+    for (int i = hi4 + tid; i < hi && at < 0; i += SAMPLE_THREADS)
+      if (!isnan(row[i])) at = i;
+  }
+  const SampleKey mine = at < 0 ? 0ull : sample_key(sample_order(best), at);
+  if (k == 1) {
+    SampleKey w = mine;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const SampleKey x = __shfl_xor_sync(0xffffffffu, w, o);
+      w = x > w ? x : w;
+    }
+    if ((tid & 31) == 0) keys[tid >> 5] = w;
+    __syncthreads();
+    if (tid == 0) {
+      for (int i = 1; i < SAMPLE_THREADS / 32; ++i) w = keys[i] > w ? keys[i] : w;
+      list[0] = w;
+    }
+    return;
+  }
+  const SampleKey from = sample_kth(mine, k);
+  if (tid == 0) count = kept = 0;
+  __syncthreads();
+  if (mine >= from) {
+    for (int i0 = lo + 4 * tid; i0 < hi4; i0 += AHEAD * STEP) {
+      float4 v[AHEAD];
+#pragma unroll
+      for (int g = 0; g < AHEAD; ++g)
+        v[g] = i0 + g * STEP < hi4 ? *reinterpret_cast<const float4*>(row + i0 + g * STEP) : make_float4(NAN, NAN, NAN, NAN);
+#pragma unroll
+      for (int g = 0; g < AHEAD; ++g) {
+        const float vv[4] = {v[g].x, v[g].y, v[g].z, v[g].w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const SampleKey x = sample_key(sample_order(vv[c]), i0 + g * STEP + c);
+          if (x >= from) keys[atomicAdd(&count, 1)] = x;
+        }
+      }
+    }
+    for (int i = hi4 + tid; i < hi; i += SAMPLE_THREADS) {
+      const SampleKey x = sample_key(sample_order(row[i]), i);
+      if (x >= from) keys[atomicAdd(&count, 1)] = x;
+    }
+  }
+  __syncthreads();
+  const int n = count;
+  if (n > SAMPLE_THREADS) {  // many large values in few strands
+    const int p = sample_pow2(n);
+    for (int i = n + tid; i < p; i += SAMPLE_THREADS) keys[i] = 0ull;
+    sample_sort(keys, p);
+    if (tid < k) list[tid] = keys[tid];
+    return;
+  }
+  const SampleKey x = tid < n ? keys[tid] : 0ull;
+  const SampleKey reach = sample_kth(x, k);
+  if (x >= reach) list[atomicAdd(&kept, 1)] = x;
+  __syncthreads();
+  if (tid >= kept && tid < k) list[tid] = 0ull;
+}
+
+// The largest entry of a row whose chunks list only theirs; every thread gets it.
+__device__ __forceinline__ SampleKey sample_best(const SampleKey* lists, int m, int chunks) {
+  SampleKey w = 0ull;
+  for (int c = threadIdx.x & 31; c < chunks; c += 32) {
+    const SampleKey x = lists[((size_t)m * chunks + c) * SAMPLE_MAX_K];
+    w = x > w ? x : w;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const SampleKey x = __shfl_xor_sync(0xffffffffu, w, o);
+    w = x > w ? x : w;
+  }
+  return w;
+}
+
+__global__ void __launch_bounds__(256)
+sample_spans_kernel(const float* __restrict__ logits, int V, long long ld, int chunks, const float* __restrict__ temperature,
+                    const int* __restrict__ top_k, const SampleKey* __restrict__ lists, float* __restrict__ sums) {
+  JLX_TL(TL_SAMPLE);
+  __shared__ float piece[SAMPLE_SPANS_PER_BLOCK][SAMPLE_PIECE + 1];
+  const int m = blockIdx.x, tid = threadIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
+  if (sample_k(temperature, top_k, m, V) != 0) return;
+  const SampleKey best = sample_best(lists, m, chunks);
+  if (best == 0ull) return;
+  const float mx = sample_value(best), inv_t = 1.f / temperature[m];
+  const float* row = logits + (size_t)m * ld;
+  const int span = (V + SAMPLE_SPANS - 1) / SAMPLE_SPANS, first = blockIdx.y * SAMPLE_SPANS_PER_BLOCK;
+  float s = 0.f;
+  for (int off = 0; off < span; off += SAMPLE_PIECE) {
+    const int width = min(SAMPLE_PIECE, span - off);
+    __syncthreads();
+    for (int idx = tid; idx < SAMPLE_SPANS_PER_BLOCK * SAMPLE_PIECE; idx += 256) {
+      const int t = idx / SAMPLE_PIECE, i = idx % SAMPLE_PIECE;
+      const long long at = (long long)(first + t) * span + off + i;
+      float e = 0.f;
+      if (i < width && at < V) {
+        const float v = row[at];
+        if (!isnan(v)) e = expf((v - mx) * inv_t);
+      }
+      piece[t][i] = e;
+    }
+    __syncthreads();
+    if (tid < SAMPLE_SPANS_PER_BLOCK)
+      for (int i = 0; i < width; ++i) s += piece[tid][i];
+  }
+  if (tid < SAMPLE_SPANS_PER_BLOCK) sums[(size_t)m * SAMPLE_SPANS + first + tid] = s;
+}
+
+// One block of SAMPLE_SPANS threads per row.  params per row: temperature[m], top_k[m], stream[m] (request's random
+// stream), counter[m] (request's step).  Rows with temperature <= 1e-3 take the argmax.
+__global__ void __launch_bounds__(SAMPLE_SPANS)
+sample_pick_kernel(const float* __restrict__ logits, int V, long long ld, int chunks, const float* __restrict__ temperature,
+                   const int* __restrict__ top_k, const unsigned long long* __restrict__ streams,
+                   const unsigned long long* __restrict__ counters, unsigned long long seed,
+                   const SampleKey* __restrict__ lists, const float* __restrict__ sums, int* __restrict__ out) {
+  JLX_TL(TL_SAMPLE);
+  __shared__ SampleKey keys[SAMPLE_MAX_K];
+  __shared__ float weight[SAMPLE_SPANS], upto[SAMPLE_SPANS], fscratch[33];
+  __shared__ int pick;
+  const int m = blockIdx.x, tid = threadIdx.x;
+  pdl_wait();
+  const int want = sample_k(temperature, top_k, m, V);
+  const float temp = temperature ? temperature[m] : 0.f;
+  int kept = 0;
+  if (want > 1) {
+    // merge: the best `want` so far stay while the other lists pass by, then each finds its place by counting the larger
+    const int total_keys = chunks * want;
+    for (int from = 0; from < total_keys;) {
+      const int take = min(SAMPLE_SPANS - kept, total_keys - from);
+      const int e = from + tid - kept;
+      SampleKey x = 0ull;
+      if (tid < kept) x = keys[tid];
+      else if (tid < kept + take) x = lists[((size_t)m * chunks + e / want) * SAMPLE_MAX_K + e % want];
+      const SampleKey reach = sample_kth(x, want);
+      if (tid == 0) pick = 0;
+      __syncthreads();
+      if (x >= reach) keys[atomicAdd(&pick, 1)] = x;
+      __syncthreads();
+      kept = pick;
+      from += take;
+      __syncthreads();
+    }
+    const SampleKey x = tid < kept ? keys[tid] : 0ull;
+    int place = 0;
+    if (tid < kept)
+      for (int j = 0; j < kept; ++j) place += keys[j] > x;
+    __syncthreads();
+    if (tid < kept) keys[place] = x;
+    if (tid == 0 && kept == 0) keys[0] = 0ull;
+    __syncthreads();
+  }
+  const SampleKey best = want > 1 ? keys[0] : sample_best(lists, m, chunks);
+  if (want == 1 || best == 0ull) {  // greedy, or the one candidate
+    if (tid == 0) out[m] = best == 0ull ? 0 : sample_index(best);
     return;
   }
   // uniform draw for this (request stream, step)
@@ -94,81 +352,86 @@ sample_kernel(const float* __restrict__ logits, int V, long long ld, const float
   philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
   const float u = (float)(c[0] >> 8) * (1.0f / 16777216.0f);
   const float inv_t = 1.f / temp;
-  const float mx = best.v;
-  int k = top_k ? top_k[m] : 0;
-  if (k > V) k = V;
-  if (k > SAMPLE_MAX_K) k = SAMPLE_MAX_K;  // the host refuses larger k before the launch
+  const float mx = sample_value(best);
 
-  if (k > 0) {
-    // k rounds of argmax over what is not yet taken: (value, index) strictly below the last pick
-    // in the order "larger value first, lower index first".
-    float lastv = INFINITY;
-    int lasti = -1;
-    for (int j = 0; j < k; ++j) {
-      ArgMax b{0.f, -1};
-      for (int i = threadIdx.x; i < V; i += blockDim.x) {
-        const float v = row[i];
-        if (isnan(v)) continue;
-        const bool after = (v < lastv) || (v == lastv && i > lasti);
-        if (after) b = better(b, ArgMax{v, i});
-      }
-      b = block_argmax(b, scratch);
-      if (b.i < 0) { k = j; break; }
-      if (threadIdx.x == 0) {
-        topv[j] = expf((b.v - mx) * inv_t);
-        topi[j] = b.i;
-      }
-      lastv = b.v;
-      lasti = b.i;
-    }
+  if (want > 0) {
+    const int k = kept;  // a row may hold fewer numbers than were asked for
+    if (tid < k) weight[tid] = expf((sample_value(keys[tid]) - mx) * inv_t);
     __syncthreads();
-    if (threadIdx.x == 0) {
-      float total = 0.f;
-      for (int j = 0; j < k; ++j) total += topv[j];
-      float run = 0.f;
-      int pick = topi[k - 1];
-      for (int j = 0; j < k; ++j) {
-        run += topv[j];
-        if (u <= run / total) { pick = topi[j]; break; }
+    if (tid < 32) {
+      if (tid == 0) {
+        float run = 0.f;
+#pragma unroll 8
+        for (int j = 0; j < k; ++j) {  // in descending order of the weights
+          run += weight[j];
+          upto[j] = run;
+        }
       }
-      out[m] = pick;
+      __syncwarp();
+      const float total = upto[k - 1];
+      int first = k - 1;
+      for (int j = tid; j < k; j += 32)
+        if (u <= upto[j] / total) { first = min(first, j); break; }
+      first = __reduce_min_sync(0xffffffffu, first);
+      if (tid == 0) out[m] = sample_index(keys[first]);
     }
     return;
   }
-  // whole vocabulary, cumulative sum in index order: thread t owns one contiguous span
-  const int span = (V + blockDim.x - 1) / blockDim.x;
-  const int lo = min(V, (int)threadIdx.x * span), hi = min(V, lo + span);
-  float s = 0.f;
-  for (int i = lo; i < hi; ++i) {
-    const float v = row[i];
-    if (!isnan(v)) s += expf((v - mx) * inv_t);
-  }
-  partial[threadIdx.x] = s;
-  const float total = block_sum(s, fscratch);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    // find the span, then the index inside it
+  // whole vocabulary, cumulative sum in index order: thread t stands for one contiguous span
+  const float* row = logits + (size_t)m * ld;
+  const int span = (V + SAMPLE_SPANS - 1) / SAMPLE_SPANS;
+  weight[tid] = sums[(size_t)m * SAMPLE_SPANS + tid];
+  const float total = block_sum(weight[tid], fscratch);
+  if (tid == 0) {
+    pick = SAMPLE_SPANS - 1;
     float run = 0.f;
-    int t = 0;
-    for (; t < (int)blockDim.x - 1; ++t) {
-      if (u <= (run + partial[t]) / total) break;
-      run += partial[t];
+#pragma unroll 8
+    for (int t = 0; t < SAMPLE_SPANS; ++t) {
+      run += weight[t];
+      upto[t] = run;
     }
-    const int l2 = min(V, t * span), h2 = min(V, l2 + span);
-    int pick = -1;
-    for (int i = l2; i < h2; ++i) {
-      const float v = row[i];
-      if (isnan(v)) continue;
-      run += expf((v - mx) * inv_t);
-      if (u <= run / total) { pick = i; break; }
-    }
-    if (pick < 0) {  // rounding at the very end of the range: last token with weight
-      pick = best.i;
-      for (int i = V - 1; i >= 0; --i)
-        if (!isnan(row[i]) && expf((row[i] - mx) * inv_t) > 0.f) { pick = i; break; }
-    }
-    out[m] = pick;
   }
+  __syncthreads();
+  if (u <= upto[tid] / total) atomicMin(&pick, tid);
+  __syncthreads();
+  const int t = pick;  // the span that the draw falls into; then the index inside it
+  float run = t > 0 ? upto[t - 1] : 0.f;
+  const int l2 = (int)min((long long)V, (long long)t * span), h2 = min(V, l2 + span);
+  __syncthreads();
+  if (tid == 0) pick = V;
+  for (int i0 = l2; i0 < h2; i0 += SAMPLE_SPANS) {
+    const int i = i0 + tid, n = min(SAMPLE_SPANS, h2 - i0);
+    const float v = i < h2 ? row[i] : 0.f;
+    const bool number = i < h2 && !isnan(v);
+    weight[tid] = number ? expf((v - mx) * inv_t) : 0.f;
+    __syncthreads();
+    if (tid == 0) {
+      float r = run;
+#pragma unroll 8
+      for (int j = 0; j < n; ++j) {
+        r += weight[j];
+        upto[j] = r;
+      }
+    }
+    __syncthreads();
+    if (number && u <= upto[tid] / total) atomicMin(&pick, i);
+    run = upto[n - 1];
+    __syncthreads();
+    if (pick < V) break;
+  }
+  if (pick >= V) {  // rounding at the very end of the range: last token with weight
+    __syncthreads();
+    if (tid == 0) pick = -1;
+    __syncthreads();
+    int last = -1;
+    for (int i = tid; i < V; i += SAMPLE_SPANS)
+      if (!isnan(row[i]) && expf((row[i] - mx) * inv_t) > 0.f) last = i;
+    if (last >= 0) atomicMax(&pick, last);
+    __syncthreads();
+    if (tid == 0 && pick < 0) pick = sample_index(best);
+  }
+  __syncthreads();
+  if (tid == 0) out[m] = pick;
 }
 
 // Greedy choice in two stages so that a handful of rows still uses the whole GPU: each block finds the
@@ -294,13 +557,41 @@ JLX_API int jlx_argmax_noalloc(const float* logits, int M, int V, long long ld, 
 
 JLX_API int jlx_sample_max_top_k() { return SAMPLE_MAX_K; }
 
+// Chunks of a row for sample_top_kernel.  At most SAMPLE_STRAND values per thread (the bound of its candidate list).  8 from
+// 16 rows on: 64 rows are then 512 blocks, all resident at once (four an SM).  16 below, where blocks are few: one row of
+// 202048, top 64, takes 24 us of which three launches' latency is most.
+static int sample_chunk(int M, int V) {
+  const int chunks = M < 16 ? 16 : 8;
+  const int size = ((V + chunks - 1) / chunks + 3) / 4 * 4;
+  const int most = SAMPLE_THREADS * (SAMPLE_STRAND - 4);  // whole vectors, and one of the last 1..3 values, per thread
+  return size < most ? size : most;
+}
+static long long sample_chunks(int M, int V) { return ((long long)V + sample_chunk(M, V) - 1) / sample_chunk(M, V); }
+
+// Bytes of scratch that jlx_sample needs: the chunks' lists, then the sums of the spans.
+JLX_API long long jlx_sample_scratch(int M, int V) {
+  if (M <= 0 || V <= 0) return 0;
+  return M * (sample_chunks(M, V) * SAMPLE_MAX_K * (long long)sizeof(SampleKey) + SAMPLE_SPANS * (long long)sizeof(float));
+}
+
 JLX_API int jlx_sample(const float* logits, int M, int V, long long ld, const float* temperature, const int* top_k,
                        const unsigned long long* streams, const unsigned long long* counters, unsigned long long seed,
-                       int* out, cudaStream_t stream) {
+                       int* out, void* scratch, cudaStream_t stream) {
   JLX_REQUIRE(M >= 0 && V > 0 && ld >= V, "sample: bad sizes M=%d V=%d", M, V);
   JLX_REQUIRE(!temperature || (streams && counters), "sample: temperature sampling needs streams and counters");
   if (M == 0) return 0;
-  sample_kernel<<<M, 1024, 0, stream>>>(logits, V, ld, temperature, top_k, streams, counters, seed, out);
+  JLX_REQUIRE(scratch && ((uintptr_t)scratch & 15) == 0, "sample: scratch missing or not on a 16-byte boundary");
+  const long long chunks = sample_chunks(M, V);
+  JLX_REQUIRE(chunks <= 65535, "sample: a vocabulary of %d is too large", V);
+  SampleKey* lists = (SampleKey*)scratch;
+  float* sums = (float*)(lists + (size_t)M * chunks * SAMPLE_MAX_K);
+  JLX_CUDA(jlx_launch_pdl(sample_top_kernel, dim3(M, (unsigned)chunks), dim3(SAMPLE_THREADS), 0, stream, logits, V, ld, sample_chunk(M, V),
+                          temperature, top_k, lists));
+  if (temperature)
+    JLX_CUDA(jlx_launch_pdl(sample_spans_kernel, dim3(M, SAMPLE_SPANS / SAMPLE_SPANS_PER_BLOCK), dim3(256), 0, stream, logits, V, ld, (int)chunks,
+                            temperature, top_k, lists, sums));
+  JLX_CUDA(jlx_launch_pdl(sample_pick_kernel, dim3(M), dim3(SAMPLE_SPANS), 0, stream, logits, V, ld, (int)chunks, temperature, top_k, streams,
+                          counters, seed, lists, sums, out));
   JLX_LAUNCH_CHECK("sample");
   return 0;
 }

@@ -1105,6 +1105,12 @@ def sample_max_top_k() -> int:
     return int(library("sampling").jlx_sample_max_top_k())
 
 
+def _sample_scratch(rows: int, vocab: int) -> int:
+    fn = library("sampling").jlx_sample_scratch
+    fn.restype = c_longlong
+    return fn(c_int(rows), c_int(vocab))
+
+
 def argmax(logits: torch.Tensor, out: torch.Tensor, part_v: torch.Tensor, part_i: torch.Tensor) -> None:
     """out[m] = index of the largest logit (lowest index on ties).  part_v (float32), part_i (int32): [M * 32] scratch."""
     _contig(logits, out, part_v, part_i)
@@ -1125,5 +1131,7 @@ def sample(logits: torch.Tensor, out: torch.Tensor, temperature: torch.Tensor | 
     if logits.dtype != torch.float32:
         raise KernelError("sample: logits must be float32")
     M, V = logits.shape
+    # made per call: the caching allocator ties it to this stream, so calls on other streams and threads have their own
+    scratch = torch.empty(_sample_scratch(M, V), dtype=torch.uint8, device=logits.device)
     _run("sampling", "jlx_sample", _ptr(logits), c_int(M), c_int(V), c_longlong(V), _ptr(temperature), _ptr(top_k),
-         _ptr(streams), _ptr(counters), c_ulonglong(seed & 0xFFFFFFFFFFFFFFFF), _ptr(out), _stream())
+         _ptr(streams), _ptr(counters), c_ulonglong(seed & 0xFFFFFFFFFFFFFFFF), _ptr(out), _ptr(scratch), _stream())

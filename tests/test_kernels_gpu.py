@@ -432,6 +432,41 @@ def test_sampling_argmax_and_draws():
     assert (freq - torch.softmax(small[0], -1)).abs().max() < 0.03
 
 
+@pytest.mark.parametrize("rows, vocab", [(1, 1), (3, 2), (2, 511), (16, 513), (5, 2049), (17, 8191), (2, 30720 * 16 + 5), (1, 202048)])
+def test_sampling_at_the_edges_of_its_chunks(rows, vocab):
+    """The lists of a row's chunks merged: rows whose values all tie, rise, hold few numbers, lie together in one thread's
+    strand, or are infinite; every k from one to more than there is.  The draw's sums are float32 in a fixed order; the
+    oracle's are float64, so a draw within 4e-6 (64 sums of 6e-8) of a boundary may fall on either side."""
+    from tests.plain import llama4_plain as plain
+
+    torch.manual_seed(rows + vocab)
+    kinds = [lambda r: r, lambda r: r * 0 + 1.5, lambda r: torch.arange(vocab, device=DEV).float() / vocab,
+             lambda r: torch.where(torch.arange(vocab, device=DEV) % 2048 == min(7, vocab - 1), r.abs() + 9, r),
+             lambda r: torch.where(torch.rand(vocab, device=DEV) < 0.99, torch.full_like(r, float("nan")), r),
+             lambda r: torch.where(torch.rand(vocab, device=DEV) < 0.9, torch.full_like(r, float("-inf")), r)]
+    ks = torch.tensor([(1, 2, 16, 63, 64, 0)[m % 6] for m in range(rows)], device=DEV, dtype=torch.int32)
+    temps = torch.tensor([(0.7, 1.3, 0.0)[m % 3] for m in range(rows)], device=DEV)
+    streams, counters = torch.arange(rows, device=DEV), torch.arange(rows, device=DEV) + 5
+    out = torch.empty(rows, device=DEV, dtype=torch.int32)
+    for kind in kinds:
+        logits = torch.stack([kind(torch.randn(vocab, device=DEV) * 2) for _ in range(rows)])
+        K().sample(logits, out, temps, ks, streams, counters, seed=77)
+        for m, got in enumerate(out.tolist()):
+            row, t = logits[m].cpu(), float(temps[m])
+            numbers = torch.nonzero(~torch.isnan(row))[:, 0]
+            if numbers.numel() == 0:
+                assert got == 0
+                continue
+            row = row[numbers]  # what is not a number is never drawn
+            if bool((row == float("-inf")).all()):
+                assert got in numbers.tolist()
+                continue
+            bits = plain.philox4x32((m + 5, 0, m, 0), (77, 0))
+            u = plain.uniform_from_bits(bits[0])
+            refs = {int(numbers[plain.sample_top(row, t, int(ks[m]), min(max(u + d, 0.0), 0.99999994))]) for d in (-4e-6, 0.0, 4e-6)}
+            assert got in refs, (m, got, refs)
+
+
 @pytest.mark.parametrize("Hq, Hkv, dh, page, chunk, window, temp", [
     (40, 8, 128, 64, 0, 0, False), (6, 2, 64, 16, 512, 0, False), (16, 1, 128, 32, 0, 300, True), (4, 4, 64, 128, 0, 0, True),
     (10, 2, 128, 16, 1024, 0, False)])
