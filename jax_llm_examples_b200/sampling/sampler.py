@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import dataclasses
 
+import numpy as np
 import torch
 
 from ..kernels import api as K
@@ -62,10 +63,12 @@ class Sampler:
         if max(top_ks) > self._max_k:
             raise ValueError(f"top_k {max(top_ks)} is above the sampler's maximum {self._max_k}")
         dev = logits.device
-        # one host->device copy: temperatures (as int bits), top_k, then streams and counters (uint64 as 2 x int32)
-        t = torch.tensor(temperatures, dtype=torch.float32).to(dev, non_blocking=True)
-        k = torch.tensor(top_ks, dtype=torch.int32).to(dev, non_blocking=True)
-        s = torch.tensor([x & 0x7FFFFFFFFFFFFFFF for x in streams], dtype=torch.int64).to(dev, non_blocking=True)
-        c = torch.tensor(counters, dtype=torch.int64).to(dev, non_blocking=True)
-        K.sample(logits, out, t, k, s, c, self.seed)
+        # one host->device copy of eight bytes thrice per row: streams, counters, then temperatures and top_k side by side
+        host = np.empty(3 * M, dtype=np.int64)
+        host[:M] = [x & 0x7FFFFFFFFFFFFFFF for x in streams]
+        host[M:2 * M] = counters
+        host[2 * M:].view(np.float32)[:M] = temperatures
+        host[2 * M:].view(np.int32)[M:] = top_ks
+        row = torch.from_numpy(host).to(dev, non_blocking=True)
+        K.sample(logits, out, row[2 * M:].view(torch.float32)[:M], row[2 * M:].view(torch.int32)[M:], row[:M], row[M:2 * M], self.seed)
         return out
