@@ -938,8 +938,12 @@ def attention_prefill_tc(q: torch.Tensor, pages: torch.Tensor, block_table: torc
 
 
 # ------------------------------------------------------------------------------------- GEMMs
-def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, offsets: torch.Tensor | None = None) -> None:
-    """out = a @ w^T.  a: [M, K]; w: [N, K], or [E, N, K] with row-group offsets [E + 1] on the device."""
+GEMM_FORMS = {"rule": 0, "general": 1, "tile": 2, "rows": 3}  # csrc/gemm_simt.cu
+
+
+def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, offsets: torch.Tensor | None = None, form: str = "rule") -> None:
+    """out = a @ w^T.  a: [M, K]; w: [N, K], or [E, N, K] with row-group offsets [E + 1] on the device.  ``form``: which of
+    the file's kernels (by the sizes, unless a test names one)."""
     _contig(a, w, out, offsets)
     M, K = a.shape
     if offsets is None:
@@ -951,7 +955,7 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, offsets: torc
         raise KernelError(f"gemm: shapes do not fit: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
     _run("gemm_simt", "jlx_gemm_simt", _ptr(a), c_int(code(a.dtype)), _ptr(w), c_int(code(w.dtype)), _ptr(out),
          c_int(code(out.dtype)), c_int(M), c_int(N), c_int(K), c_longlong(K), c_longlong(K), c_longlong(N),
-         _ptr(offsets), c_int(E), c_longlong(stride), _stream())
+         _ptr(offsets), c_int(E), c_longlong(stride), c_int(GEMM_FORMS[form]), _stream())
 
 
 def gemm_stream_supported(a: torch.Tensor, w: torch.Tensor) -> bool:

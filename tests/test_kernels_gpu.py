@@ -236,6 +236,36 @@ def _groups(E, sizes_seed, total):
     return torch.tensor([0] + cuts + [total], dtype=torch.int32)
 
 
+@pytest.mark.parametrize("form", ["rule", "tile", "rows"])
+@pytest.mark.parametrize("M, N, Kd", [(1, 16, 4), (7, 17, 36), (8, 128, 32), (9, 129, 68), (33, 130, 100), (64, 127, 512), (65, 256, 2052),
+                                      (130, 64, 516), (300, 515, 1028)])
+def test_gemm_f32_forms_at_the_edges_of_their_tiles(form, M, N, Kd):
+    """The float32 kernels at the remainders of rows, columns and K slices, with K cut over a cluster where it is long
+    enough.  A sum of Kd products in float32 is off by at most Kd 2^-24 of the sum of their sizes; strands stay below."""
+    a, w = torch.randn(M, Kd, device=DEV), torch.randn(N, Kd, device=DEV)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    K().gemm_simt(a, w, out, form=form)
+    ref, size = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+    assert bool(((out.double() - ref).abs() <= Kd * 2.0 ** -24 * size).all())
+
+
+@pytest.mark.parametrize("form", ["rule", "tile", "rows"])
+@pytest.mark.parametrize("E, rows, N, Kd", [(3, [0, 5, 1], 20, 40), (40, None, 132, 64), (4, [64, 0, 65, 33], 129, 516), (2, [0, 0], 16, 8)])
+def test_gemm_f32_forms_in_groups(form, E, rows, N, Kd):
+    """Groups without rows, with more than one tile, and more than 32 of them (a warp looks at 32 at a time)."""
+    rows = rows or [(7 * e) % 5 for e in range(E)]
+    off = torch.tensor([sum(rows[:e]) for e in range(E + 1)], device=DEV, dtype=torch.int32)
+    M = max(sum(rows), 1)
+    a, w, out = torch.randn(M, Kd, device=DEV), torch.randn(E, N, Kd, device=DEV), torch.zeros(M, N, device=DEV)
+    K().gemm_simt(a, w, out, off, form=form)
+    at = 0
+    for e, n in enumerate(rows):
+        ref = a[at:at + n].double() @ w[e].double().t()
+        size = a[at:at + n].double().abs() @ w[e].double().abs().t()
+        assert bool(((out[at:at + n].double() - ref).abs() <= Kd * 2.0 ** -24 * size).all())
+        at += n
+
+
 @pytest.mark.parametrize("E, rows, N, Kd", [(4, 37, 70, 50), (8, 300, 130, 64), (3, 5, 64, 129)])
 def test_gemm_simt_grouped(E, rows, N, Kd):
     a, w = torch.randn(rows, Kd, device=DEV), torch.randn(E, N, Kd, device=DEV)
