@@ -14,8 +14,10 @@
 //   gemm_f32_tile   many rows: tiles of 64 (or 32) x 128 outputs, 8 (4) x 8 per thread; bound by the FMA pipe.
 //   gemm_simt       everything that is not float32 throughout or not in whole 16-byte pieces.
 //
-// The order in which an output's K products are added is a function of the sizes of the product: in order, or in strands
-// (of lanes and warps, or of blocks) that are added in a fixed order.  The other rows' values never enter a row's result.
+// The order in which an output's K products are added follows from K alone, so that a position's result does not depend on
+// how its prompt was cut into steps.  gemm_simt adds them one by one.  The other two cut K into four parts of whole 32s;
+// a part has a strand of its even and one of its odd K, each one by one; the strands are added, then the parts in order.
+
 #include "common.cuh"
 
 #define BM 64
@@ -139,54 +141,61 @@ __device__ __forceinline__ bool find_row_tile(const int* __restrict__ offsets, i
   return false;
 }
 
-// 8 RM x 128 outputs per block of 128 threads: a warp 4 RM x 64, a thread RM rows by 8 columns.  A packed FMA takes two
-// neighbouring K of a row of A and of a row of W as they lie in memory, so an output has two strands (even and odd K) that
-// are added at the end, nothing is transposed, and the K slices come by 16-byte asynchronous copies into a ring of three.
-// A thread's rows are every fourth, its columns every eighth, and a row of a slice is 144 bytes: the lanes that read
-// together read different banks.  Four K of RM = 8 are sixteen 16-byte reads for 128 packed FMAs.
-// Where the tiles are too few for the GPU, a cluster of blocks cuts K and adds its sums, in the blocks' order, through
-// distributed shared memory.
-// Bound by the FMA pipe, whose rate with such operands is about 60 TFLOP/s (32 independent accumulators in registers,
-// nothing else), and by the reads beside it: 1024 x 8192 x 2048 takes 752 us (45.7 TFLOP/s; the kernel with 64 x 64 tiles
-// and scalar loads, below, 1360), 1024 x 3072 x 2048 311 us (600).
-#define TN 128
-#define TK 32
-#define TILE_LD 36  // floats per row of a slice
-#define TILE_STAGES 3
+#define GEMM_PARTS 4
+__host__ __device__ __forceinline__ int gemm_part(int K) { return ((K + GEMM_PARTS - 1) / GEMM_PARTS + 31) / 32 * 32; }
+
 __device__ __forceinline__ void copy16_or_zero(float* dst, const float* src, bool there) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
 }
+
+// 8 RM x 128 outputs per block of 128 threads: a warp 4 RM x 64, a thread RM rows by 8 columns.  A packed FMA takes two
+// neighbouring K of a row of A and of a row of W as they lie in memory (the two strands), nothing is transposed, and the K
+// slices come by 16-byte asynchronous copies into a ring of four.  A thread's rows are every fourth, its columns every
+// eighth, and a row of a slice is 80 bytes: the lanes that read together read different banks.  Four K of RM = 8 are sixteen
+// 16-byte reads for 128 packed FMAs.  The parts before a block's last are added up in a place beside the ring.
+// Where the tiles are too few for the GPU, a cluster of two or four blocks shares the parts and adds them through
+// distributed shared memory.
+// Bound by the FMA pipe, whose rate with such operands is about 60 TFLOP/s (32 independent accumulators in registers,
+// nothing else), and by the reads beside it: 1024 x 8192 x 2048 takes
+// 817 us (42 TFLOP/s; the kernel with 64 x 64 tiles and scalar loads, above, 1360), 1024 x 3072 x 2048 338 us (600).
+#define TN 128
+#define TK 16
+#define TILE_LD 20  // floats per row of a slice
+#define TILE_STAGES 4
+#define SUM_LD (TN + 4)
 template <int RM>
 __global__ void __launch_bounds__(128, 2)
 gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K, long long lda,
-                     long long ldw, long long ldc, const int* __restrict__ offsets, int E, long long w_group_stride, int k_share) {
+                     long long ldw, long long ldc, const int* __restrict__ offsets, int E, long long w_group_stride) {
   JLX_TL(TL_GEMM_SIMT);
   constexpr int TM = 8 * RM, STAGE = (TM + TN) * TILE_LD;
-  extern __shared__ __align__(16) float ring[];  // [TILE_STAGES][TM rows of A, then TN rows of W][TILE_LD]
+  extern __shared__ __align__(16) float ring[];  // [TILE_STAGES][TM rows of A, then TN rows of W][TILE_LD]; then the sums' place
+  float* before = ring + TILE_STAGES * STAGE;    // [TM][SUM_LD]: the parts before the block's last
   int m0 = blockIdx.x * TM, m_end = M, group = 0;
   if (offsets && !find_row_tile(offsets, E, blockIdx.x, TM, group, m0, m_end)) return;  // all blocks of a cluster alike
   const float* Wg = W + (size_t)group * w_group_stride;
   const int n0 = blockIdx.y * TN;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int mt = (warp >> 1) * (4 * RM) + (lane >> 3), nt = (warp & 1) * 64 + (lane & 7);  // rows mt + 4 i, columns nt + 8 j
-  const int k_first = blockIdx.z * k_share, k_end = min(K, k_first + k_share);
-  // loader: eight threads per row, sixteen rows at a time; rows past the end read a row that is there and are not stored
-  const int lr = tid >> 3, lk = (tid & 7) * 4;
-  const float* ap[TM / 16];
-  const float* wp[TN / 16];
+  const int shares = gridDim.z, own = GEMM_PARTS / shares, part = gemm_part(K);
+  const int k_first = min(K, (int)blockIdx.z * own * part), k_end = min(K, ((int)blockIdx.z + 1) * own * part);
+  // loader: four threads per row, 32 rows at a time; rows past the end read a row that is there and are not stored
+  const int lr = tid >> 2, lk = (tid & 3) * 4;
+  const float* ap[TM / 32];
+  const float* wp[TN / 32];
 #pragma unroll
-  for (int i = 0; i < TM / 16; ++i) ap[i] = A + (size_t)min(m0 + lr + 16 * i, m_end - 1) * lda + lk;
+  for (int i = 0; i < TM / 32; ++i) ap[i] = A + (size_t)min(m0 + lr + 32 * i, m_end - 1) * lda + lk;
 #pragma unroll
-  for (int i = 0; i < TN / 16; ++i) wp[i] = Wg + (size_t)min(n0 + lr + 16 * i, N - 1) * ldw + lk;
+  for (int i = 0; i < TN / 32; ++i) wp[i] = Wg + (size_t)min(n0 + lr + 32 * i, N - 1) * ldw + lk;
   auto fetch = [&](int k0, int stage) {  // always a group of copies, maybe an empty one
     if (k0 < k_end) {
-      const bool there = k0 + lk < k_end;  // K and the cuts of it are multiples of 4
+      const bool there = k0 + lk < k_end;  // K and the parts of it are multiples of 4
       const int at = there ? k0 : -lk;     // (an address that exists, of which nothing is read)
       float* dst = ring + stage * STAGE + lr * TILE_LD + lk;
 #pragma unroll
-      for (int i = 0; i < TM / 16; ++i) copy16_or_zero(dst + 16 * i * TILE_LD, ap[i] + at, there);
+      for (int i = 0; i < TM / 32; ++i) copy16_or_zero(dst + 32 * i * TILE_LD, ap[i] + at, there);
 #pragma unroll
-      for (int i = 0; i < TN / 16; ++i) copy16_or_zero(dst + (TM + 16 * i) * TILE_LD, wp[i] + at, there);
+      for (int i = 0; i < TN / 32; ++i) copy16_or_zero(dst + (TM + 32 * i) * TILE_LD, wp[i] + at, there);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -195,13 +204,27 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
   for (int i = 0; i < RM; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
-  fetch(k_first, 0);
-  fetch(k_first + TK, 1);
-  int stage = 0;
+#pragma unroll
+  for (int g = 0; g < TILE_STAGES - 1; ++g) fetch(k_first + g * TK, g);
+  int stage = 0, part_end = k_first + part;
+  bool first = true;
   for (int k0 = k_first; k0 < k_end; k0 += TK) {
+    if (k0 == part_end) {  // (a part is whole slices) every thread keeps its own outputs' sums
+#pragma unroll
+      for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float* at = before + (mt + 4 * i) * SUM_LD + nt + 8 * j;
+          const float s = low_of(acc[i][j]) + high_of(acc[i][j]);
+          *at = first || (shares > 1 && blockIdx.z > 0) ? s : *at + s;  // (two blocks: the second has one part here)
+          acc[i][j] = 0ull;
+        }
+      first = false;
+      part_end += part;
+    }
     asm volatile("cp.async.wait_group %0;" ::"n"(TILE_STAGES - 2) : "memory");
     __syncthreads();  // this slice is there for everyone, and everyone is past the slice whose place is filled next
-    fetch(k0 + (TILE_STAGES - 1) * TK, stage + TILE_STAGES - 1 < TILE_STAGES ? stage + TILE_STAGES - 1 : stage - 1);
+    fetch(k0 + (TILE_STAGES - 1) * TK, (stage + TILE_STAGES - 1) % TILE_STAGES);
     const float* as = ring + stage * STAGE + mt * TILE_LD;
     const float* ws = ring + stage * STAGE + (TM + nt) * TILE_LD;
 #pragma unroll
@@ -218,32 +241,37 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
         for (int j = 0; j < 8; ++j) acc[i][j] = fma2(a.y, w[j].y, acc[i][j]);
       }
     }
-    stage = stage + 1 < TILE_STAGES ? stage + 1 : 0;
+    stage = (stage + 1) % TILE_STAGES;
   }
   __syncthreads();  // the ring's last slice is read: its place serves the sums (no copies are in flight any more)
-  constexpr int SUM_LD = TN + 4;
-  float* sums = ring;  // [TM][SUM_LD]
+  float* sums = ring;  // [TM][SUM_LD]: the first block of a cluster, or the only one: all its parts; the others: the last part
+  const bool second = shares == 2 && blockIdx.z == 1;
 #pragma unroll
   for (int i = 0; i < RM; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) sums[(mt + 4 * i) * SUM_LD + nt + 8 * j] = low_of(acc[i][j]) + high_of(acc[i][j]);
-  const int shares = gridDim.z;
+    for (int j = 0; j < 8; ++j) {
+      const int at = (mt + 4 * i) * SUM_LD + nt + 8 * j;
+      const float s = low_of(acc[i][j]) + high_of(acc[i][j]);
+      sums[at] = first || second ? s : before[at] + s;
+      if (second && first) before[at] = 0.f;  // K ends inside the block's first part, whose sums are in `sums`
+    }
   if (shares == 1) __syncthreads();
   else asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   const bool vec = (ldc & 3) == 0 && ((uintptr_t)C & 15) == 0;
   for (int idx = blockIdx.z * 128 + tid; idx < TM * (TN / 4); idx += shares * 128) {
     const int r = idx / (TN / 4), c = idx % (TN / 4) * 4, m = m0 + r, n = n0 + c;
-    float* mine = sums + r * SUM_LD + c;
-    float4 v = *reinterpret_cast<float4*>(mine);
-    if (shares > 1) {
-      v = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int z = 0; z < shares; ++z) {
-        uint32_t there;
-        float4 x;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(z));
-        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(there) : "memory");
-        v = make_float4(v.x + x.x, v.y + x.y, v.z + x.z, v.w + x.w);
-      }
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (shares == 1) v = *reinterpret_cast<float4*>(sums + r * SUM_LD + c);
+    auto add = [&](const float* mine, int z) {
+      uint32_t there;
+      float4 x;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(z));
+      asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(there) : "memory");
+      v = make_float4(v.x + x.x, v.y + x.y, v.z + x.z, v.w + x.w);
+    };
+    for (int z = 0; shares > 1 && z < shares; ++z) {
+      if (shares == 2 && z == 1) add(before + r * SUM_LD + c, z);
+      add(sums + r * SUM_LD + c, z);
     }
     if (m >= m_end) continue;
     float* dst = C + (size_t)m * ldc + n;
@@ -263,14 +291,13 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
 template <int RM>
 static cudaError_t launch_tile(const float* a, const float* w, float* c, int M, int N, int K, long long lda, long long ldw, long long ldc,
                                const int* offsets, int E, long long wgs, int shares, cudaStream_t stream) {
-  const int k_share = ((K + shares - 1) / shares + TK - 1) / TK * TK;
-  const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<RM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)(sizeof(float) * TILE_STAGES * (8 * RM + TN) * TILE_LD));
+  const int smem = (int)sizeof(float) * (TILE_STAGES * (8 * RM + TN) * TILE_LD + 8 * RM * SUM_LD);
+  const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<RM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((M + 8 * RM - 1) / (8 * RM) + (offsets ? E : 0)), (N + TN - 1) / TN, shares);
   cfg.blockDim = dim3(128);
-  cfg.dynamicSmemBytes = sizeof(float) * TILE_STAGES * (8 * RM + TN) * TILE_LD;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -279,70 +306,95 @@ static cudaError_t launch_tile(const float* a, const float* w, float* c, int M, 
   attr[0].val.clusterDim.z = shares;
   cfg.attrs = attr;
   cfg.numAttrs = shares > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<RM>, a, w, c, M, N, K, lda, ldw, ldc, offsets, E, wgs, k_share);
+  return cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<RM>, a, w, c, M, N, K, lda, ldw, ldc, offsets, E, wgs);
 }
 
-// MT token rows by 16 weight rows per block of 8 warps.  The warps take turns along K, 32 of it at a time: eight lanes of
-// four K each, the four groups of eight lanes on four weight rows each, pairs of neighbouring K in one packed FMA.  Then
-// the lanes' and the warps' strands are added in a fixed order.  Weights go from memory to registers once; token rows come
-// from L2.  Blocks that share weight rows follow one another, so that more than MT rows read them from L2 again.
-// Bound by the weights' bytes and the latency of a block's few steps: one row by 8192 x 2048 takes 23 us (67 MB, 10 us at
-// the copy rate), 32768 x 2048 58 us (41); the tiles of the general kernel took 156 and 365.
-#define RN 16
+// MT token rows by 32 weight rows per block of four warps, one for each part of K; a lane has a weight row.  Every warp
+// brings its own slices of 32 K into a ring of its own (a row of a slice is 144 bytes: eight lanes read eight different
+// 16-byte columns of banks), so the warps meet only once, when the parts are added.  Blocks that share weight rows follow
+// one another: more than MT token rows read them from L2 again.
+// Bound by the weights' bytes, and with few columns by how much a block's four rings keep in flight: one
+// row by 8192 x 2048 takes 25 us (67 MB, 10 us at the copy rate), 32768 x 2048 66 us (41); the tiles of the general kernel
+// took 156 and 365.
+#define RN 32
+#define ROWS_K 32
+#define ROWS_LD 36
+#define ROWS_STAGES 4
 template <int MT>
-__global__ void __launch_bounds__(256, MT <= 4 ? 2 : 1)
+__global__ void __launch_bounds__(128)
 gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K, long long lda,
                      long long ldw, long long ldc, const int* __restrict__ offsets, int E, long long w_group_stride) {
   JLX_TL(TL_GEMM_SIMT);
-  __shared__ float part[8][MT][RN];
+  constexpr int STAGE = (RN + MT) * ROWS_LD;
+  extern __shared__ __align__(16) float rings[];  // [warp][stage][weight rows, then token rows][ROWS_LD]
+  __shared__ float sums[GEMM_PARTS][MT][RN];
   int m0 = blockIdx.x * MT, m_end = M, group = 0;
   if (offsets && !find_row_tile(offsets, E, blockIdx.x, MT, group, m0, m_end)) return;
   const float* Wg = W + (size_t)group * w_group_stride;
   const int n0 = blockIdx.y * RN;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int kl = (lane & 7) * 4, g = lane >> 3;
-  const float* ap[MT];
-  const float* wp[4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = gemm_part(K);
+  const int k_first = min(K, warp * part), k_end = min(K, k_first + part);
+  float* ring = rings + warp * ROWS_STAGES * STAGE;
+  // loader: eight lanes per row, four rows at a time
+  const int lr = lane >> 3, lk = (lane & 7) * 4;
+  auto fetch = [&](int k0, int stage) {  // always a group of copies, maybe an empty one
+    if (k0 < k_end) {
+      const bool there = k0 + lk < k_end;
+      const int at = there ? k0 + lk : 0;
+      float* dst = ring + stage * STAGE + lr * ROWS_LD + lk;
 #pragma unroll
-  for (int i = 0; i < MT; ++i) ap[i] = A + (size_t)min(m0 + i, m_end - 1) * lda;
+      for (int i = 0; i < RN / 4; ++i) copy16_or_zero(dst + 4 * i * ROWS_LD, Wg + (size_t)min(n0 + lr + 4 * i, N - 1) * ldw + at, there);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) wp[i] = Wg + (size_t)min(n0 + g + 4 * i, N - 1) * ldw;
-  unsigned long long acc[MT][4];
+      for (int i = 0; i < (MT + 3) / 4; ++i)
+        if (lr + 4 * i < MT) copy16_or_zero(dst + (RN + 4 * i) * ROWS_LD, A + (size_t)min(m0 + lr + 4 * i, m_end - 1) * lda + at, there);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  unsigned long long acc[MT];
 #pragma unroll
-  for (int i = 0; i < MT; ++i)
+  for (int i = 0; i < MT; ++i) acc[i] = 0ull;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
-#pragma unroll 2
-  for (int k = warp * 32 + kl; k < K; k += 256) {
-    ulonglong2 w[4], a[MT];
+  for (int g = 0; g < ROWS_STAGES - 1; ++g) fetch(k_first + g * ROWS_K, g);
+  int stage = 0;
+  for (int k0 = k_first; k0 < k_end; k0 += ROWS_K) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(ROWS_STAGES - 2) : "memory");
+    __syncwarp();  // this slice is there for the warp, and the warp is past the slice whose place is filled next
+    fetch(k0 + (ROWS_STAGES - 1) * ROWS_K, (stage + ROWS_STAGES - 1) % ROWS_STAGES);
+    const float* ws = ring + stage * STAGE + lane * ROWS_LD;
+    const float* as = ring + stage * STAGE + RN * ROWS_LD;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(wp[j] + k);
+    for (int k = 0; k < ROWS_K; k += 4) {
+      const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(ws + k);
 #pragma unroll
-    for (int i = 0; i < MT; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(ap[i] + k);
-#pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = fma2(a[i].y, w[j].y, fma2(a[i].x, w[j].x, acc[i][j]));
+      for (int i = 0; i < MT; ++i) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(as + i * ROWS_LD + k);
+        acc[i] = fma2(a.y, w.y, fma2(a.x, w.x, acc[i]));
+      }
+    }
+    stage = (stage + 1) % ROWS_STAGES;
   }
 #pragma unroll
-  for (int i = 0; i < MT; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float s = low_of(acc[i][j]) + high_of(acc[i][j]);
-      s += __shfl_xor_sync(0xffffffffu, s, 1);
-      s += __shfl_xor_sync(0xffffffffu, s, 2);
-      s += __shfl_xor_sync(0xffffffffu, s, 4);
-      if ((lane & 7) == 0) part[warp][i][g + 4 * j] = s;
-    }
+  for (int i = 0; i < MT; ++i) sums[warp][i][lane] = low_of(acc[i]) + high_of(acc[i]);
   __syncthreads();
-  for (int idx = threadIdx.x; idx < MT * RN; idx += 256) {
+  for (int idx = threadIdx.x; idx < MT * RN; idx += 128) {
     const int i = idx / RN, n = idx % RN;
     if (m0 + i >= m_end || n0 + n >= N) continue;
-    float s = part[0][i][n];
+    float s = sums[0][i][n];
 #pragma unroll
-    for (int w = 1; w < 8; ++w) s += part[w][i][n];
+    for (int p = 1; p < GEMM_PARTS; ++p) s += sums[p][i][n];
     C[(size_t)(m0 + i) * ldc + n0 + n] = s;
   }
+}
+
+template <int MT>
+static cudaError_t launch_rows(const float* a, const float* w, float* c, int M, int N, int K, long long lda, long long ldw, long long ldc,
+                               const int* offsets, int E, long long wgs, cudaStream_t stream) {
+  const int smem = (int)sizeof(float) * GEMM_PARTS * ROWS_STAGES * (RN + MT) * ROWS_LD;
+  const cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  const dim3 grid((unsigned)((M + MT - 1) / MT + (offsets ? (E < M ? E : M) : 0)), (N + RN - 1) / RN);
+  gemm_f32_rows_kernel<MT><<<grid, 128, smem, stream>>>(a, w, c, M, N, K, lda, ldw, ldc, offsets, E, wgs);
+  return cudaGetLastError();
 }
 
 template <typename TA, typename TW, typename TC>
@@ -361,12 +413,12 @@ enum { GEMM_FORM_RULE = 0, GEMM_FORM_GENERAL = 1, GEMM_FORM_TILE = 2, GEMM_FORM_
 
 // Which kernel, by estimates of the time in microseconds on this GPU (148 multiprocessors), fitted to measurements at N x K
 // from 2048 x 2048 to 32768 x 2048 with 1 to 1024 rows, dense and in 8 groups:
-//   rows: 0.5 us per million weights for their bytes and 0.35 to 0.9 for every tile of 1 to 8 rows.
+//   rows: 0.5 us per million weights for their bytes and 0.35 to 0.65 for every tile of 1 to 8 rows.
 //   tile: a multiprocessor takes 53 ns per K and tile of 64 rows, 31 ns of 32 rows; a lone block 64 and 38; cutting K over
-//         a cluster costs 3 us, and eight blocks wait for one another longer.
-// (32768 x 2048, one row: rows 58, 32-row tiles 140; 8192 x 2048, 8 rows: rows 33, 32-row tiles 45 cut in four; 32 rows: 82
-// and 43; 64 rows: rows 149, 64-row tiles 68 cut in four; 1024 rows: 64-row tiles 752, 32-row tiles 870; 16 rows in 8
-// groups: rows 113, 32-row tiles 235.)
+//         a cluster costs 3 us.
+// (32768 x 2048, 8 rows: rows 80, 32-row tiles 141; 8192 x 2048, 16 rows: rows 41, 32-row tiles cut in four 45; 32 rows: 78 and
+// 45; 64 rows: rows 135, 64-row tiles cut in four 72; 1024 rows: rows 2034, 64-row tiles 817; 64 rows in 8 groups: rows 180,
+// 32-row tiles 238.)
 struct GemmPlan { int form, rm, shares, mt; };
 static GemmPlan gemm_plan(int M, int N, int K, int groups) {
   const int per = (M + groups - 1) / groups;  // rows that a weight matrix typically multiplies
@@ -379,13 +431,13 @@ static GemmPlan gemm_plan(int M, int N, int K, int groups) {
     return groups > 1 ? (t > used ? t : used) : (double)((M + size - 1) / size);
   };
   GemmPlan best = {GEMM_FORM_ROWS, 0, 1, mt};
-  double least = 5.0 + million * (0.5 * used + (mt == 1 ? 0.35 : (mt == 2 ? 0.4 : (mt == 4 ? 0.6 : 0.9))) * row_tiles(mt));
+  double least = 5.0 + million * (0.5 * used + (mt == 1 ? 0.35 : (mt == 2 ? 0.4 : (mt == 4 ? 0.6 : 0.65))) * row_tiles(mt));
   for (int rm = 4; rm <= 8; rm += 4)
-    for (int shares = 1; shares <= 8 && (shares == 1 || K / shares >= 256); shares *= 2) {
+    for (int shares = 1; shares <= GEMM_PARTS && (shares == 1 || K / shares >= 256); shares *= 2) {
       const double blocks = row_tiles(8 * rm) * ((N + TN - 1) / TN) * shares;
       const double rounds = blocks <= 148 ? 1.0 : (double)(long long)(blocks / 148 + 0.999);
       const double per_k = rounds <= 1.0 ? (rm == 8 ? 0.064 : 0.038) : rounds * (rm == 8 ? 0.053 : 0.031);
-      const double t = per_k * K / shares * (shares == 8 ? 1.8 : 1.0) + (shares > 1 ? 3.0 : 0.0);
+      const double t = per_k * K / shares + (shares > 1 ? 3.0 : 0.0);
       if (t < least) {
         least = t;
         best = {GEMM_FORM_TILE, rm, shares, mt};
@@ -420,14 +472,10 @@ JLX_API int jlx_gemm_simt(const void* A, int a_dtype, const void* W, int w_dtype
     return 0;
   }
   if (form == GEMM_FORM_ROWS && (N + RN - 1) / RN <= 65535) {
-    const int mt = plan.mt;
-    const dim3 grid((unsigned)((M + mt - 1) / mt + (offsets ? (groups < M ? groups : M) : 0)), (N + RN - 1) / RN);
-#define ROWS(MT) gemm_f32_rows_kernel<MT><<<grid, 256, 0, stream>>>(a, w, (float*)C, M, N, K, lda, ldw, ldc, offsets, E, w_group_stride)
-    if (mt == 1) ROWS(1);
-    else if (mt == 2) ROWS(2);
-    else if (mt == 4) ROWS(4);
-    else ROWS(8);
-#undef ROWS
+    JLX_CUDA(plan.mt == 1 ? launch_rows<1>(a, w, (float*)C, M, N, K, lda, ldw, ldc, offsets, E, w_group_stride, stream)
+             : plan.mt == 2 ? launch_rows<2>(a, w, (float*)C, M, N, K, lda, ldw, ldc, offsets, E, w_group_stride, stream)
+             : plan.mt == 4 ? launch_rows<4>(a, w, (float*)C, M, N, K, lda, ldw, ldc, offsets, E, w_group_stride, stream)
+                            : launch_rows<8>(a, w, (float*)C, M, N, K, lda, ldw, ldc, offsets, E, w_group_stride, stream));
     JLX_LAUNCH_CHECK("gemm_f32_rows");
     return 0;
   }

@@ -850,6 +850,47 @@ def attention_generic(q: torch.Tensor, pages: torch.Tensor, block_table: torch.T
          c_float(floor_scale), _ptr(sink), _ptr(slopes), c_float(softcap), _ptr(status), _stream())
 
 
+def attention_f32_supported(q: torch.Tensor) -> bool:
+    return q.dtype == torch.float32 and q.data_ptr() % 16 == 0 and bool(library("attention_generic").jlx_attention_f32_supported(c_int(q.shape[2])))
+
+
+ATTENTION_F32_RANGE = 256  # keys of a range, csrc/attention_generic.cu
+
+
+def attention_f32_plan(max_kv_len: int, chunk: int, window: int, keep: int, blocks: int) -> tuple[int, int]:
+    """(blocks that share an item's key ranges, ranges of one) for a launch of ``blocks`` blocks: about two blocks per
+    multiprocessor."""
+    seen = min(max_kv_len, window or max_kv_len, chunk or max_kv_len) + 16  # of an item's 16 tokens together
+    ranges = -(-seen // ATTENTION_F32_RANGE) + 1 + (-(-keep // ATTENTION_F32_RANGE) + 1 if window and keep else 0)  # as they lie
+    per = -(-ranges // max(1, min(2 * sm_count() // max(blocks, 1), ranges)))
+    return -(-ranges // per), per
+
+
+def attention_f32(q: torch.Tensor, pages: torch.Tensor, block_table: torch.Tensor, req_of_token: torch.Tensor, positions: torch.Tensor,
+                  out: torch.Tensor, scale: float, chunk: int, window: int, attn_scale: float, floor_scale: float, status: torch.Tensor,
+                  n_items: int, items: torch.Tensor | None = None, max_count: int = 1, rows: torch.Tensor | None = None, splits: int = 1,
+                  per_split: int = 0, part_o: torch.Tensor | None = None, part_ml: torch.Tensor | None = None,
+                  sink: torch.Tensor | None = None, slopes: torch.Tensor | None = None, softcap: float = 0.0, keep: int = 0) -> None:
+    """:func:`attention_generic` in float32 by work items: ``items`` int32 pairs (first token row, count <= 16) of one request
+    each, or single tokens (``rows``: their token rows; None: rows 0 .. n_items).  ``splits`` > 1 blocks
+    share an item's key ranges, ``per_split`` each; part_o: float32 [N * Hq * splits * per_split * dh], part_ml: the same with 2
+    for dh."""
+    _contig(q, pages, block_table, out, items, rows, part_o, part_ml)
+    N, Hq, dh = q.shape
+    _check_sink(sink, Hq)
+    _check_sink(slopes, Hq, "slopes")
+    P, _, Hkv, page_size, dh2 = pages.shape
+    if dh2 != dh or any(t.dtype != torch.float32 for t in (q, pages, out)) or out.numel() != q.numel():
+        raise KernelError("attention_f32: queries, pages and output must be float32 of one head size")
+    if splits > 1 and (part_o is None or part_ml is None or part_o.numel() < N * Hq * splits * per_split * dh
+                       or part_ml.numel() < N * Hq * splits * per_split * 2):
+        raise KernelError("attention_f32: scratch for the partial results is too small")
+    _run("attention_generic", "jlx_attention_f32", _ptr(q), _ptr(pages), _ptr(block_table), c_int(block_table.shape[1]), _ptr(req_of_token),
+         _ptr(positions), _ptr(out), c_int(Hq), c_int(Hkv), c_int(dh), c_int(page_size), c_int(P), c_float(scale), c_int(chunk), c_int(window),
+         c_int(keep), c_float(attn_scale), c_float(floor_scale), _ptr(sink), _ptr(slopes), c_float(softcap), _ptr(items), _ptr(rows),
+         c_int(n_items), c_int(max_count), c_int(splits), c_int(per_split), _ptr(part_o), _ptr(part_ml), _ptr(status), _stream())
+
+
 def _check_sink(sink: torch.Tensor | None, Hq: int, what: str = "sink") -> None:
     if sink is not None and (sink.dtype != torch.float32 or sink.numel() != Hq or not sink.is_contiguous()):
         raise KernelError(f"attention: the {what} must be float32 [{Hq}], one number per query head")

@@ -137,6 +137,20 @@ class PagedAttention(Mixer):
                            chunk, window, attn_scale, floor_scale, part_o, part_ml, splits, split_keys, ctx.status,
                            rows, n_rows, self.sink, self.slopes, self.softcap, self.keep_first, diff)
 
+    def _items_f32(self, ctx: StepContext, q, cache: LayerCache, out, attn_scale, floor_scale, n_items: int, items=None, rows=None) -> None:
+        """The 32-bit attention over portions in tiles (``items``), or over single tokens."""
+        chunk, window = self.chunk or 0, self.window or 0
+        per_item = (FLASH_TILE if items is not None else 1) * self.n_heads // self.n_kv_heads
+        splits, per_split = K.attention_f32_plan(ctx.max_kv_len, chunk, window, self.keep_first, n_items * self.n_kv_heads * -(-per_item // 64))
+        part_o = part_ml = None
+        if splits > 1:
+            n = q.shape[0] * self.n_heads * splits * per_split
+            part_o = ctx.workspace.get("attn_f32_part_o", n * self.head_dim, torch.float32)
+            part_ml = ctx.workspace.get("attn_f32_part_ml", n * 2, torch.float32)
+        K.attention_f32(q, cache.pages, cache.block_table, ctx.req_of_token, ctx.positions, out, self.scale, chunk, window, attn_scale,
+                        floor_scale, ctx.status, n_items, items, FLASH_TILE if items is not None else 1, rows, splits, per_split, part_o, part_ml,
+                        self.sink, self.slopes, self.softcap, self.keep_first)
+
     def attend(self, ctx: StepContext, q, cache: LayerCache, out, attn_scale: float, floor_scale: float, diff=None) -> None:
         """Tensor-core kernels where they are built (bfloat16, head size 64 or 128): split-KV for
         requests that bring one token, flash tiles for the others (tcgen05 for long portions of head size 128);
@@ -172,9 +186,17 @@ class PagedAttention(Mixer):
                                         self.softcap, self.keep_first, diff)
                 return
         maps = out if diff is None else torch.empty(q.shape, dtype=torch.float32, device=q.device)
-        K.attention_generic(q, cache.pages, cache.block_table, ctx.req_of_token, ctx.positions, maps, self.scale,
-                            self.chunk or 0, self.window or 0, attn_scale, floor_scale, ctx.status, self.sink, self.slopes, self.softcap,
-                            self.keep_first)
+        if not (K.attention_f32_supported(q) and (decode or "attn_tiles_all" in ctx.arrays)):
+            K.attention_generic(q, cache.pages, cache.block_table, ctx.req_of_token, ctx.positions, maps, self.scale,
+                                self.chunk or 0, self.window or 0, attn_scale, floor_scale, ctx.status, self.sink, self.slopes, self.softcap,
+                                self.keep_first)
+        elif decode:
+            self._items_f32(ctx, q, cache, maps, attn_scale, floor_scale, q.shape[0])
+        else:
+            n_tiles, n_single = len(ctx.host_arrays["attn_tiles_all"]), len(ctx.host_arrays["attn_single_rows"])
+            self._items_f32(ctx, q, cache, maps, attn_scale, floor_scale, n_tiles, items=ctx.arrays["attn_tiles_all"])
+            if n_single:
+                self._items_f32(ctx, q, cache, maps, attn_scale, floor_scale, n_single, rows=ctx.arrays["attn_single_rows"])
         if diff is not None:
             K.map_difference(maps, out, diff)
 

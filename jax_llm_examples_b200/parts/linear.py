@@ -11,7 +11,7 @@ Which kernel runs:
   (cuBLAS through torch), as the reference leaves its dense products to its library (XLA dot_general,
   llama4/llama4_jax/model.py:907-909, 952-954, 1146-1152, 1204).
 * anything 32-bit (the true 32-bit path; weights stored in 32-bit under bfloat16 activations; K that
-  is no multiple of 8): the 32-bit FMA kernel (``csrc/gemm_simt.cu``), so that no reduced-precision
+  is no multiple of 8): the 32-bit FMA kernels (``csrc/gemm_simt.cu``), so that no reduced-precision
   matrix mode is possible there.
 """
 

@@ -202,6 +202,45 @@ def test_attention_generic(dtype, tol, Hq, Hkv, dh, page, chunk, window, temp):
         at += n
 
 
+@pytest.mark.parametrize("Hq, Hkv, dh, page", [(8, 2, 128, 64), (5, 1, 64, 16), (20, 1, 36, 8), (3, 3, 4, 4), (34, 2, 100, 32)])
+@pytest.mark.parametrize("chunk, window, keep, splits", [(0, 0, 0, 1), (0, 0, 0, 3), (64, 0, 0, 1), (0, 70, 0, 2), (0, 33, 5, 1), (0, 100, 90, 4),
+                                                       (96, 50, 0, 2)])
+def test_attention_f32_items_against_the_general_kernel(Hq, Hkv, dh, page, chunk, window, keep, splits):
+    """Portions in tiles and single tokens, whole and in key ranges, against the kernel that serves any size; with a sink,
+    slopes, a soft cap and a temperature; pages of keys that no query sees are gone.  Both sum up to 400 products and
+    weights in float32 in different orders: 400 x 6e-8 = 2.4e-5 of the values' size at worst, 5e-6 as they come."""
+    lens, q_lens = [400, 37, 1, 130, 65], [131, 16, 1, 1, 17]
+    q, pages, bt, req, pos, ks, vs = _paged_case(torch.float32, Hq, Hkv, dh, page, lens, q_lens)
+    for r, (L, n) in enumerate(zip(lens, q_lens)):
+        first = L - n
+        low = max(first // chunk * chunk if chunk else 0, first - window + 1 if window else 0)
+        for pg in range(bt.shape[1]):
+            if (pg + 1) * page <= low and pg * page >= keep:
+                bt[r, pg] = -1
+    starts = [sum(q_lens[:r]) for r in range(len(q_lens))]
+    tiles = [(s + o, min(16, n - o)) for s, n in zip(starts, q_lens) if n > 1 for o in range(0, n, 16)]
+    items = torch.tensor(tiles, device=DEV, dtype=torch.int32)
+    singles = torch.tensor([s for s, n in zip(starts, q_lens) if n == 1], device=DEV, dtype=torch.int32)
+    per = -(-4 // splits)  # up to two ranges of 256 keys, one more for the kept keys
+    part_o = torch.full((q.numel() * splits * per,), float("nan"), device=DEV)
+    part_ml = torch.full((q.shape[0] * Hq * splits * per * 2,), float("nan"), device=DEV)
+    for sink, slopes, cap, temp in ((None, None, 0.0, 0.0), (torch.randn(Hq, device=DEV), torch.rand(Hq, device=DEV) * 0.1, 3.0, 0.1)):
+        want, got, st = torch.empty_like(q), torch.full_like(q, float("nan")), status()
+        common = (q, pages, bt, req, pos)
+        K().attention_generic(*common, want, dh ** -0.5, chunk, window, temp, 16.0, st, sink, slopes, cap, keep)
+        K().attention_f32(*common, got, dh ** -0.5, chunk, window, temp, 16.0, st, len(tiles), items, 16, None, splits, per, part_o, part_ml,
+                          sink, slopes, cap, keep)
+        K().attention_f32(*common, got, dh ** -0.5, chunk, window, temp, 16.0, st, len(singles), None, 1, singles, splits, per, part_o,
+                          part_ml, sink, slopes, cap, keep)
+        assert int(st) == 0
+        close(got, want, 5e-6)
+        if splits > 1:  # merged by another kernel, the same numbers
+            whole = torch.full_like(q, float("nan"))
+            K().attention_f32(*common, whole, dh ** -0.5, chunk, window, temp, 16.0, st, q.shape[0], None, 1, None, 1, 0, None, None, sink, slopes,
+                              cap, keep)
+            assert torch.equal(whole, got)
+
+
 def test_attention_finds_one_far_key_among_hundreds():
     """Random keys would hide a key that is skipped or read from the wrong page: here one key far back
     matches the query strongly, so almost all of the output is that key's value."""
@@ -247,6 +286,9 @@ def test_gemm_f32_forms_at_the_edges_of_their_tiles(form, M, N, Kd):
     K().gemm_simt(a, w, out, form=form)
     ref, size = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
     assert bool(((out.double() - ref).abs() <= Kd * 2.0 ** -24 * size).all())
+    one = torch.empty(1, N, device=DEV)
+    K().gemm_simt(a[M - 1:], w, one, form="rows")  # the order of a sum follows from Kd alone
+    assert torch.equal(one[0], out[M - 1])
 
 
 @pytest.mark.parametrize("form", ["rule", "tile", "rows"])
