@@ -182,7 +182,7 @@ template <int NR, int G, bool READ_AFTER>
 __global__ void decay_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ d,
                                   const float* __restrict__ v, const float* __restrict__ u, float* __restrict__ state,
                                   const int* __restrict__ cu_q, const int* __restrict__ slot_ids, float* __restrict__ o,
-                                  int H, int dk, int dv) {
+                                  int H, int dk, int dv, int skip_from) {
   JLX_TL(TL_OTHER);
   pdl_launch_dependents_if_small();
   constexpr int CW = 32 / G, RL = NR / G;
@@ -214,7 +214,7 @@ __global__ void decay_scan_kernel(const float* __restrict__ q, const float* __re
   }
   pdl_wait();
   const int n0 = cu_q[r], n1 = cu_q[r + 1];
-  if (n1 <= n0) return;
+  if (n1 <= n0 || (skip_from > 0 && n1 - n0 >= skip_from)) return;  // long portions may be walked by other kernels
   float* S = state + ((size_t)slot_ids[r] * H + hd) * dk * dv;
   float s[RL];
 #pragma unroll
@@ -316,13 +316,13 @@ __global__ void decay_scan_kernel(const float* __restrict__ q, const float* __re
 
 template <int NR, int G, bool READ_AFTER>
 static int launch_decay_scan(const float* q, const float* k, const float* d, const float* v, const float* u, float* state,
-                             const int* cu_q, const int* slot_ids, float* o, int R, int H, int dk, int dv, cudaStream_t stream) {
+                             const int* cu_q, const int* slot_ids, float* o, int R, int H, int dk, int dv, int skip_from, cudaStream_t stream) {
   const int W = (dk + NR - 1) / NR, CW = 32 / G;
   const size_t smem = sizeof(float) * (2 * ((size_t)3 * SCAN_TB * W * NR + SCAN_TB * 32) + (size_t)SCAN_TB * W * CW);
   if (smem > 48 * 1024)
     JLX_CUDA(cudaFuncSetAttribute(decay_scan_kernel<NR, G, READ_AFTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   JLX_CUDA(jlx_launch_pdl(decay_scan_kernel<NR, G, READ_AFTER>, dim3(R, H, (dv + CW - 1) / CW), dim3(W * 32), smem, stream, q, k, d, v,
-                          u, state, cu_q, slot_ids, o, H, dk, dv));
+                          u, state, cu_q, slot_ids, o, H, dk, dv, skip_from));
   JLX_LAUNCH_CHECK("decay_scan");
   return 0;
 }
@@ -336,15 +336,16 @@ static int scan_row_groups(int H, int dv, int nr) {
 }
 
 // q, k, d: float32 [N, H, dk]; v: [N, H, dv]; u: [H, dk] or null (only read before the update); state: [slots, H, dk, dv];
-// o: [N, H, dv].  read_after: 1 = o_t = S_t^T q_t;  0 = o_t = (S_(t-1) + diag(u) k_t v_t^T)^T q_t.
+// o: [N, H, dv].  read_after: 1 = o_t = S_t^T q_t;  0 = o_t = (S_(t-1) + diag(u) k_t v_t^T)^T q_t.  skip_from > 0: requests of
+// at least so many tokens are left alone.
 JLX_API int jlx_decay_scan(const float* q, const float* k, const float* d, const float* v, const float* u, float* state,
                            const int* cu_q, const int* slot_ids, float* o, int R, int H, int dk, int dv, int read_after,
-                           cudaStream_t stream) {
+                           int skip_from, cudaStream_t stream) {
   JLX_REQUIRE(R >= 0 && H > 0 && dk > 0 && dv > 0, "decay_scan: bad sizes R=%d H=%d dk=%d dv=%d", R, H, dk, dv);
   JLX_REQUIRE(dk <= 512, "decay_scan: %d key channels per head; up to 512 are supported", dk);
   JLX_REQUIRE(H <= 65535 && (dv + 7) / 8 <= 65535, "decay_scan: too many heads or value columns");
   if (R == 0) return 0;
-#define JLX_SCAN_ARGS q, k, d, v, u, state, cu_q, slot_ids, o, R, H, dk, dv, stream
+#define JLX_SCAN_ARGS q, k, d, v, u, state, cu_q, slot_ids, o, R, H, dk, dv, skip_from, stream
 #define JLX_SCAN(NR, G) return read_after ? launch_decay_scan<NR, G, true>(JLX_SCAN_ARGS) : launch_decay_scan<NR, G, false>(JLX_SCAN_ARGS)
 #define JLX_SCAN_G(NR)                        \
   {                                           \

@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(512)
 hgrn2_scan_kernel(const float* __restrict__ g, float* __restrict__ state, const int* __restrict__ cu_q,
                   const int* __restrict__ slot_ids, float* __restrict__ o32, int H, int dk, int dv, int DVB,
                   const int* __restrict__ segs, float* __restrict__ seg_state, float* __restrict__ seg_decay,
-                  float* __restrict__ qd) {
+                  float* __restrict__ qd, int skip_from) {
   JLX_TL(TL_OTHER);
   pdl_launch_dependents_if_small();
   pdl_wait();
@@ -146,6 +146,7 @@ hgrn2_scan_kernel(const float* __restrict__ g, float* __restrict__ state, const 
   const int i0 = s * REC_RT, jl = live ? c * REC_CT : 0, j0 = col0 + jl;
   const int r = SEG ? segs[4 * blockIdx.x] : blockIdx.x;
   const int n0 = SEG ? segs[4 * blockIdx.x + 1] : cu_q[r], n1 = SEG ? segs[4 * blockIdx.x + 2] : cu_q[r + 1];
+  if (!SEG && skip_from > 0 && n1 - n0 >= skip_from) return;  // walked by other kernels
   const int flags = SEG ? segs[4 * blockIdx.x + 3] : 1;
   const bool from_state = flags & 1, to_scratch = flags & 2;
   const int HK = H * dk;
@@ -365,11 +366,14 @@ __global__ void head_rms_norm_kernel(const float* __restrict__ o32, const float*
   for (int j = lane; j < dv; j += 32) out[(size_t)row * dv + j] = from_f32<TO>(p[j] / rms * (w ? w[j] : 1.f));
 }
 
+// stages: which of the launches (a caller may walk the long portions, of at least skip_from tokens, by other kernels between
+// the gates and the norm; skip_from 0: none).
+enum { HGRN2_GATES = 1, HGRN2_SCAN = 2, HGRN2_NORM = 4 };
 JLX_API int jlx_hgrn2_scan(const float* qfv, int splits, long long split_stride, const float* f_bias, const float* lower,
                            float* state, const int* cu_q, const int* slot_ids, const float* norm_w, float eps, float* gates,
                            float* o32, void* out, int out_dtype, int N, int R, int H, int dk, int dv, int sm_count,
-                           const int* segs, int n_seg, int seg_tokens, float* seg_state, float* seg_decay, float* qd,
-                           cudaStream_t stream) {
+                           const int* segs, int n_seg, int seg_tokens, float* seg_state, float* seg_decay, float* qd, int stages,
+                           int skip_from, cudaStream_t stream) {
   JLX_REQUIRE(R >= 0 && N >= 0 && H > 0 && dk > 0 && dv > 0 && splits >= 1, "hgrn2_scan: bad sizes R=%d H=%d dk=%d dv=%d", R, H, dk, dv);
   JLX_REQUIRE(dk <= 32 * REC_RT, "hgrn2_scan: %d state rows per head are above the supported maximum %d", dk, 32 * REC_RT);
   JLX_REQUIRE(eps > 0.f, "hgrn2_scan: eps must be positive");
@@ -377,52 +381,55 @@ JLX_API int jlx_hgrn2_scan(const float* qfv, int splits, long long split_stride,
   JLX_REQUIRE(!segs || (n_seg >= R && seg_tokens >= COR_TOK && seg_state && seg_decay && qd), "hgrn2_scan: segments need their scratch");
   if (R == 0 || N == 0) return 0;
   const int nb = segs ? n_seg : R;  // blocks along x: segments, or requests
-  JLX_CUDA(jlx_launch_pdl(hgrn2_gates_kernel, dim3(N), dim3(256), 0, stream, qfv, splits, split_stride, f_bias, lower, gates, H * dk, H * dv));
+  if (stages & HGRN2_GATES) JLX_CUDA(jlx_launch_pdl(hgrn2_gates_kernel, dim3(N), dim3(256), 0, stream, qfv, splits, split_stride, f_bias, lower, gates, H * dk, H * dv));
   JLX_LAUNCH_CHECK("hgrn2_gates");
-  int NSP = 1;
-  while (NSP * REC_RT < dk) NSP *= 2;
-  // value columns per block: as many as a block of 512 threads takes, fewer while the grid would not fill the GPU
-  int DVB = 4;
-  while (DVB < dv && DVB < 64 && (DVB * 2 / REC_CT) * NSP <= 512) DVB *= 2;
-  while (DVB > 16 && (long long)nb * H * ((dv + DVB - 1) / DVB) < 2 * sm_count) DVB /= 2;  // every slice reads the head's f and q again
-  const int zb = (dv + DVB - 1) / DVB;
-  JLX_REQUIRE(H <= 65535 && zb <= 65535, "hgrn2_scan: too many heads or column slices");
-  const int threads = ((DVB / REC_CT) * NSP + 31) / 32 * 32;
-  const int dkp = NSP * REC_RT;
-  const size_t smem = sizeof(float) * (2 * (size_t)REC_TCH * (2 * dkp + DVB));
+  if (stages & HGRN2_SCAN) {
+    int NSP = 1;
+    while (NSP * REC_RT < dk) NSP *= 2;
+    // value columns per block: as many as a block of 512 threads takes, fewer while the grid would not fill the GPU
+    int DVB = 4;
+    while (DVB < dv && DVB < 64 && (DVB * 2 / REC_CT) * NSP <= 512) DVB *= 2;
+    while (DVB > 16 && (long long)nb * H * ((dv + DVB - 1) / DVB) < 2 * sm_count) DVB /= 2;  // every slice reads the head's f and q again
+    const int zb = (dv + DVB - 1) / DVB;
+    JLX_REQUIRE(H <= 65535 && zb <= 65535, "hgrn2_scan: too many heads or column slices");
+    const int threads = ((DVB / REC_CT) * NSP + 31) / 32 * 32;
+    const int dkp = NSP * REC_RT;
+    const size_t smem = sizeof(float) * (2 * (size_t)REC_TCH * (2 * dkp + DVB));
 #define REC_GO(NSP_)                                                                                                        \
-  case NSP_:                                                                                                                \
-    if (segs) {                                                                                                             \
-      if (smem > 48 * 1024)                                                                                                 \
-        JLX_CUDA(cudaFuncSetAttribute(hgrn2_scan_kernel<NSP_, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-      JLX_CUDA(jlx_launch_pdl(hgrn2_scan_kernel<NSP_, true>, dim3(nb, H, zb), dim3(threads), smem, stream, (const float*)gates, \
-                              state, cu_q, slot_ids, o32, H, dk, dv, DVB, segs, seg_state, seg_decay, qd));                  \
-    } else {                                                                                                                \
-      if (smem > 48 * 1024)                                                                                                 \
-        JLX_CUDA(cudaFuncSetAttribute(hgrn2_scan_kernel<NSP_, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-      JLX_CUDA(jlx_launch_pdl(hgrn2_scan_kernel<NSP_, false>, dim3(nb, H, zb), dim3(threads), smem, stream, (const float*)gates, \
-                              state, cu_q, slot_ids, o32, H, dk, dv, DVB, segs, seg_state, seg_decay, qd));                  \
-    }                                                                                                                       \
-    break
-  switch (NSP) {
-    REC_GO(1);
-    REC_GO(2);
-    REC_GO(4);
-    REC_GO(8);
-    REC_GO(16);
-    REC_GO(32);
-  }
+    case NSP_:                                                                                                                \
+      if (segs) {                                                                                                             \
+        if (smem > 48 * 1024)                                                                                                 \
+          JLX_CUDA(cudaFuncSetAttribute(hgrn2_scan_kernel<NSP_, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        JLX_CUDA(jlx_launch_pdl(hgrn2_scan_kernel<NSP_, true>, dim3(nb, H, zb), dim3(threads), smem, stream, (const float*)gates, \
+                                state, cu_q, slot_ids, o32, H, dk, dv, DVB, segs, seg_state, seg_decay, qd, skip_from));                  \
+      } else {                                                                                                                \
+        if (smem > 48 * 1024)                                                                                                 \
+          JLX_CUDA(cudaFuncSetAttribute(hgrn2_scan_kernel<NSP_, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        JLX_CUDA(jlx_launch_pdl(hgrn2_scan_kernel<NSP_, false>, dim3(nb, H, zb), dim3(threads), smem, stream, (const float*)gates, \
+                                state, cu_q, slot_ids, o32, H, dk, dv, DVB, segs, seg_state, seg_decay, qd, skip_from));                  \
+      }                                                                                                                       \
+      break
+    switch (NSP) {
+      REC_GO(1);
+      REC_GO(2);
+      REC_GO(4);
+      REC_GO(8);
+      REC_GO(16);
+      REC_GO(32);
+    }
 #undef REC_GO
-  JLX_LAUNCH_CHECK("hgrn2_scan");
-  if (segs) {
-    hgrn2_chain_kernel<<<dim3(n_seg, H, (dk * dv + 255) / 256), 256, 0, stream>>>(segs, n_seg, seg_state, seg_decay, state, slot_ids, H, dk, dv);
-    JLX_LAUNCH_CHECK("hgrn2_chain");
-    const int tiles = (seg_tokens + COR_TOK - 1) / COR_TOK;
-    const size_t csm = sizeof(float) * ((size_t)dk * COR_COL + (size_t)COR_TOK * (dk + 1));
-    if (csm > 48 * 1024) JLX_CUDA(cudaFuncSetAttribute(hgrn2_correct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
-    hgrn2_correct_kernel<<<dim3(n_seg * tiles, H, (dv + COR_COL - 1) / COR_COL), 128, csm, stream>>>(segs, seg_state, qd, o32, H, dk, dv, tiles);
-    JLX_LAUNCH_CHECK("hgrn2_correct");
+    JLX_LAUNCH_CHECK("hgrn2_scan");
+    if (segs) {
+      hgrn2_chain_kernel<<<dim3(n_seg, H, (dk * dv + 255) / 256), 256, 0, stream>>>(segs, n_seg, seg_state, seg_decay, state, slot_ids, H, dk, dv);
+      JLX_LAUNCH_CHECK("hgrn2_chain");
+      const int tiles = (seg_tokens + COR_TOK - 1) / COR_TOK;
+      const size_t csm = sizeof(float) * ((size_t)dk * COR_COL + (size_t)COR_TOK * (dk + 1));
+      if (csm > 48 * 1024) JLX_CUDA(cudaFuncSetAttribute(hgrn2_correct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
+      hgrn2_correct_kernel<<<dim3(n_seg * tiles, H, (dv + COR_COL - 1) / COR_COL), 128, csm, stream>>>(segs, seg_state, qd, o32, H, dk, dv, tiles);
+      JLX_LAUNCH_CHECK("hgrn2_correct");
+    }
   }
+  if (!(stages & HGRN2_NORM)) return 0;
   const int rows = N * H, wpb = 8;
   JLX_DISPATCH_DTYPE(out_dtype, TO, {
     JLX_CUDA(jlx_launch_pdl(head_rms_norm_kernel<TO>, dim3((rows + wpb - 1) / wpb), dim3(wpb * 32), 0, stream, (const float*)o32, norm_w,

@@ -5,6 +5,7 @@ raises.  Every launch through this module is counted (``launch_count``)."""
 from __future__ import annotations
 
 import ctypes
+import dataclasses
 from ctypes import c_float, c_int, c_longlong, c_ulonglong, c_void_p
 
 import torch
@@ -387,7 +388,7 @@ def hgrn2_scan_scratch(n_tokens: int, heads: int, dk: int, dv: int, n_segments: 
 def hgrn2_scan(qfv: torch.Tensor, splits: int, f_bias: torch.Tensor, lower: torch.Tensor, state: torch.Tensor,
                cu_q: torch.Tensor, slot_ids: torch.Tensor, norm_weight: torch.Tensor | None, eps: float, out: torch.Tensor,
                heads: int, dk: int, dv: int, scratch: torch.Tensor | None = None, segments: torch.Tensor | None = None,
-               n_segments: int = 0, segment_tokens: int = 0) -> None:
+               n_segments: int = 0, segment_tokens: int = 0, chunks: "Chunks | None" = None, chunk_scratch: torch.Tensor | None = None) -> None:
     """The gated recurrence S = diag(f) S + (1 - f) v^T, o = S^T silu(q) over each request's tokens, then the per-head
     RMS norm of o (three launches: gates, scan, norm).  qfv: float32 [N, 2 H dk + H dv] = [q | f | v] before their
     activations (or ``splits`` partials); state: float32 [slots, H, dk, dv]; out: [N, H dv]; scratch: float32 of
@@ -395,7 +396,8 @@ def hgrn2_scan(qfv: torch.Tensor, splits: int, f_bias: torch.Tensor, lower: torc
     ``segments`` (int32 [n_segments, 4] = request, first row, end row, flags; at most ``segment_tokens`` rows each, every
     token in exactly one, a request's segments in order): long portions are scanned as several segments at once, each but
     a request's first from a zero state; two more kernels chain the segments' states and correct their outputs.  flags:
-    1 = the request's first segment, 2 = the request has several."""
+    1 = the request's first segment, 2 = the request has several.
+    ``chunks`` (instead of segments, with ``chunk_scratch``): the long portions go through :func:`chunk_scan`."""
     _contig(qfv, f_bias, lower, state, norm_weight, out, scratch, segments)
     if any(t.dtype != torch.float32 for t in (qfv, f_bias, lower, state)) or (norm_weight is not None and norm_weight.dtype != torch.float32):
         raise KernelError("hgrn2_scan: projections, gate constants, state and norm weight must be float32")
@@ -425,12 +427,26 @@ def hgrn2_scan(qfv: torch.Tensor, splits: int, f_bias: torch.Tensor, lower: torc
         seg_state, seg_decay, qd = cut(n_segments * heads * dk * dv), cut(n_segments * heads * dk), cut(N * heads * dk)
     sp, stride = _splits(qfv, splits)
     global _launches
-    _run("recurrent", "jlx_hgrn2_scan", _ptr(qfv), c_int(sp), c_longlong(stride), _ptr(f_bias), _ptr(lower), _ptr(state),
-         _ptr(cu_q), _ptr(slot_ids), _ptr(norm_weight), c_float(eps), _ptr(gates), _ptr(o32), _ptr(out), c_int(code(out.dtype)),
-         c_int(N), c_int(slot_ids.numel()), c_int(heads), c_int(dk), c_int(dv), c_int(sm_count()),
-         _ptr(segments) if n_segments else None, c_int(n_segments), c_int(segment_tokens), _ptr(seg_state), _ptr(seg_decay),
-         _ptr(qd), _stream())
-    _launches += 2 + (2 if n_segments else 0)  # gates, scan, (chain, correction,) norm
+
+    def run(do: int, skip_from: int = 0) -> None:
+        _run("recurrent", "jlx_hgrn2_scan", _ptr(qfv), c_int(sp), c_longlong(stride), _ptr(f_bias), _ptr(lower), _ptr(state),
+             _ptr(cu_q), _ptr(slot_ids), _ptr(norm_weight), c_float(eps), _ptr(gates), _ptr(o32), _ptr(out), c_int(code(out.dtype)),
+             c_int(N), c_int(slot_ids.numel()), c_int(heads), c_int(dk), c_int(dv), c_int(sm_count()),
+             _ptr(segments) if n_segments else None, c_int(n_segments), c_int(segment_tokens), _ptr(seg_state), _ptr(seg_decay),
+             _ptr(qd), c_int(do), c_int(skip_from), _stream())
+
+    GATES, SCAN, NORM = 1, 2, 4  # csrc/recurrent.cu
+    if chunks is None or n_segments:
+        run(GATES | SCAN | NORM)
+        _launches += 2 + (2 if n_segments else 0)  # gates, scan, (chain, correction,) norm
+        return
+    run(GATES | (SCAN if chunks.others else 0), chunks.long_from)
+    _launches += int(chunks.others)
+    F = heads * dk
+    rows = gates[:N * (2 * F + heads * dv)].view(N, -1)
+    chunk_scan(rows[:, F:2 * F].unflatten(1, (heads, dk)), None, rows[:, :F].unflatten(1, (heads, dk)), rows[:, 2 * F:].unflatten(1, (heads, dv)),
+               None, state, slot_ids, o32[:N * heads * dv].view(N, heads, dv), True, chunks, chunk_scratch)
+    run(NORM)
 
 
 # -------------------------------------------------------------------------- latent attention
@@ -616,10 +632,10 @@ def decay_prep(q: _RowsView, k: _RowsView, v: _RowsView, z: _RowsView | None, z_
 
 
 def decay_scan(q: torch.Tensor, k: torch.Tensor, d: torch.Tensor, v: torch.Tensor, bonus: torch.Tensor | None, state: torch.Tensor,
-               cu_q: torch.Tensor, slot_ids: torch.Tensor, o: torch.Tensor, read_after_update: bool) -> None:
+               cu_q: torch.Tensor, slot_ids: torch.Tensor, o: torch.Tensor, read_after_update: bool, skip_from: int = 0) -> None:
     """S <- diag(d_t) S + k_t v_t^T over each request's tokens, in order.  ``read_after_update``: o_t = S_t^T q_t; else
     o_t = (S_(t-1) + diag(bonus) k_t v_t^T)^T q_t.  q, k, d: float32 [N, H, dk]; v, o: [N, H, dv]; bonus: [H, dk];
-    state: float32 [slots, H, dk, dv]."""
+    state: float32 [slots, H, dk, dv].  ``skip_from`` > 0: requests of at least so many tokens are left to ``chunk_scan``."""
     _contig(q, k, d, v, bonus, state, o)
     N, H, dk = q.shape
     dv = v.shape[2]
@@ -628,7 +644,56 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, d: torch.Tensor, v: torch.Tenso
     if tuple(state.shape[1:]) != (H, dk, dv) or tuple(o.shape) != (N, H, dv) or (bonus is not None and bonus.numel() != H * dk):
         raise KernelError(f"decay_scan: shapes do not fit: q {tuple(q.shape)}, v {tuple(v.shape)}, state {tuple(state.shape)}")
     _run("decay_scan", "jlx_decay_scan", _ptr(q), _ptr(k), _ptr(d), _ptr(v), _ptr(bonus), _ptr(state), _ptr(cu_q), _ptr(slot_ids),
-         _ptr(o), c_int(slot_ids.numel()), c_int(H), c_int(dk), c_int(dv), c_int(int(read_after_update)), _stream())
+         _ptr(o), c_int(slot_ids.numel()), c_int(H), c_int(dk), c_int(dv), c_int(int(read_after_update)), c_int(skip_from), _stream())
+
+
+CHUNK_TOKENS = 64  # csrc/chunk_scan.cu
+
+
+@dataclasses.dataclass
+class Chunks:
+    """Long portions cut into chunks of up to CHUNK_TOKENS tokens: ``chunks`` int32 [n, 3] (request, first token row, end row),
+    ``requests`` int32 [m, 3] (request, its first chunk, its chunks), which hold at least ``long_from`` tokens each;
+    ``others``: whether the step has requests that are not among them."""
+
+    chunks: torch.Tensor
+    requests: torch.Tensor
+    n: int
+    m: int
+    long_from: int
+    others: bool
+
+
+def chunk_scan_supported(dk: int, dv: int) -> bool:
+    """Heads that fill most of the 128 channels and columns the kernels work on."""
+    return 64 < dk <= 128 and 64 < dv <= 128
+
+
+def chunk_scan_scratch(n: int, heads: int, dk: int, dv: int) -> int:
+    """float32 elements that ``chunk_scan`` needs for n chunks: their states and decays."""
+    return n * heads * dk * (dv + 1)
+
+
+def chunk_scan(q: torch.Tensor, k: torch.Tensor | None, d: torch.Tensor, v: torch.Tensor, bonus: torch.Tensor | None, state: torch.Tensor,
+               slot_ids: torch.Tensor, o: torch.Tensor, read_after_update: bool, chunks: Chunks, scratch: torch.Tensor) -> None:
+    """:func:`decay_scan` for the requests of ``chunks`` (three launches).  q, k, d, v: float32 [N, H, size] whose rows may be
+    wider than H * size; k None: k = 1 - d.  scratch: float32 of ``chunk_scan_scratch`` elements."""
+    global _launches
+    _contig(bonus, state, o, scratch)
+    N, H, dk = q.shape
+    dv = v.shape[2]
+    for t, size in ((q, dk), (k, dk), (d, dk), (v, dv)):
+        if t is not None and (t.dtype != torch.float32 or tuple(t.shape) != (N, H, size) or t.stride(2) != 1 or t.stride(1) != size):
+            raise KernelError("chunk_scan: operands are float32 [N, H, size] with heads side by side in a row")
+    if any(t.dtype != torch.float32 for t in (state, o, scratch)) or (bonus is not None and (bonus.dtype != torch.float32 or bonus.numel() != H * dk)):
+        raise KernelError("chunk_scan: everything is float32")
+    if tuple(state.shape[1:]) != (H, dk, dv) or tuple(o.shape) != (N, H, dv) or scratch.numel() < chunk_scan_scratch(chunks.n, H, dk, dv):
+        raise KernelError(f"chunk_scan: shapes do not fit: q {tuple(q.shape)}, v {tuple(v.shape)}, state {tuple(state.shape)}")
+    ld = lambda t: c_longlong(t.stride(0) if t is not None else 0)  # noqa: E731
+    _run("chunk_scan", "jlx_chunk_scan", _ptr(q), ld(q), _ptr(k), ld(k), _ptr(d), ld(d), _ptr(v), ld(v), _ptr(bonus), _ptr(state), _ptr(slot_ids),
+         _ptr(o), _ptr(chunks.chunks), c_int(chunks.n), _ptr(chunks.requests), c_int(chunks.m), c_int(H), c_int(dk), c_int(dv),
+         c_int(int(read_after_update)), _ptr(scratch), _stream())
+    _launches += 2
 
 
 def head_norm_gate(o: torch.Tensor, weight: torch.Tensor | None, per_head: bool, gate: _RowsView | None, eps: float, mult: float,

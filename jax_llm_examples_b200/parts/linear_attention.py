@@ -14,6 +14,7 @@ from ..kernels import api as K
 from ..tracing import scope
 from .base import LayerCache, Mixer, ProjectedMixer, Rows, StateNeed, StepContext, as_rows, register_part
 from .linear import grouped_linear, linear
+from .recurrent import plan_scan_chunks, scan_chunks
 
 
 def _scan(ctx: StepContext, q, k, v, z, z_bias, form: str, tau: float, q_scale: float, bonus, state, heads: int, dk: int, dv: int,
@@ -35,7 +36,11 @@ def _scan(ctx: StepContext, q, k, v, z, z_bias, form: str, tau: float, q_scale: 
 
     qo, ko, do, vo, o = cut(n, heads, dk), cut(n, heads, dk), cut(n, heads, dk), cut(n, heads, dv), cut(n, heads, dv)
     K.decay_prep(q, k, v, z, z_bias, form, tau, q_scale, qo, ko, do, vo, heads, dk, dv, **prep)
-    K.decay_scan(qo, ko, do, vo, bonus, state, ctx.cu_q, ctx.slot_ids, o, read_after_update)
+    chunks, scratch = scan_chunks(ctx, heads, dk, dv)
+    if chunks is None or chunks.others:
+        K.decay_scan(qo, ko, do, vo, bonus, state, ctx.cu_q, ctx.slot_ids, o, read_after_update, 0 if chunks is None else chunks.long_from)
+    if chunks is not None:
+        K.chunk_scan(qo, ko, do, vo, bonus, state, ctx.slot_ids, o, read_after_update, chunks, scratch)
     return o
 
 
@@ -47,7 +52,7 @@ class GatedLinearAttention(ProjectedMixer):
     ``w_in``: [2 H dk + 2 H dv, D] = the q, k, v and gate projections stacked in that order; ``w_a1``: [rank, D];
     ``w_a2``: [H dk, rank]; ``a_bias``: [H dk].  State: float32 [H, dk, dv] per request."""
 
-    kernel_libraries = ("decay_scan", "gemm_simt", "group_norm")
+    kernel_libraries = ("decay_scan", "chunk_scan", "gemm_simt", "group_norm")
     kernel_libraries_bf16 = ("gemm_stream",)
 
     def __init__(self, w_in: torch.Tensor, w_a1: torch.Tensor, w_a2: torch.Tensor, a_bias: torch.Tensor, norm_weight: torch.Tensor,
@@ -64,6 +69,9 @@ class GatedLinearAttention(ProjectedMixer):
 
     def state_need(self):
         return StateNeed((self.heads, self.dim, self.vdim), torch.float32)
+
+    def step_planners(self):
+        return (plan_scan_chunks,)
 
     def core(self, ctx: StepContext, h, proj: Rows, col: int, cache: LayerCache, out: torch.Tensor, mult: float) -> None:
         H, dk, dv = self.heads, self.dim, self.vdim
@@ -90,7 +98,7 @@ class TimeMixWKV(Mixer):
     ``mu``: [5, D] in the order r, k, v, g, w.  ``w_rkvg``: [4, H dk, D].  ``w_w1``: [rank, D]; ``w_w2``: [H dk, rank];
     ``w0``: [H dk]; ``bonus``: [H, dk].  State: the previous input, float32 [D], and S, float32 [H, dk, dk]."""
 
-    kernel_libraries = ("decay_scan", "gemm_simt", "group_norm")
+    kernel_libraries = ("decay_scan", "chunk_scan", "gemm_simt", "group_norm")
     kernel_libraries_bf16 = ("gemm_stream",)
     needs_f32_input = True
     OVERLAP_MAX_ROWS = 256
@@ -109,6 +117,9 @@ class TimeMixWKV(Mixer):
 
     def state_needs(self):
         return (StateNeed((self.width,), torch.float32), StateNeed((self.heads, self.dim, self.dim), torch.float32))
+
+    def step_planners(self):
+        return (plan_scan_chunks,)
 
     def forward(self, ctx: StepContext, h, cache: LayerCache, h32: torch.Tensor | None = None):
         n, D = h32.shape
@@ -163,7 +174,7 @@ class RetentionMixer(ProjectedMixer):
     (0, 1].  State: float32 [H, dk, dv] per request, zero at the start.  The recurrence is the decay-scan kernel's with
     a decay that is the same for every key channel of a head and every token."""
 
-    kernel_libraries = ("decay_scan", "gemm_simt")
+    kernel_libraries = ("decay_scan", "chunk_scan", "gemm_simt")
     kernel_libraries_bf16 = ("gemm_stream",)
 
     def __init__(self, w_in: torch.Tensor, w_o: torch.Tensor, decay: torch.Tensor, heads: int, dim: int, vdim: int, eps: float,
@@ -181,6 +192,9 @@ class RetentionMixer(ProjectedMixer):
 
     def state_need(self):
         return StateNeed((self.heads, self.dim, self.vdim), torch.float32)
+
+    def step_planners(self):
+        return (plan_scan_chunks,)
 
     def core(self, ctx: StepContext, h, proj: Rows, col: int, cache: LayerCache, out: torch.Tensor, mult: float) -> None:
         H, dk, dv = self.heads, self.dim, self.vdim

@@ -62,6 +62,40 @@ def plan_scan_segments(shape: StepShape) -> dict:
     return {"scan_segments": np.array(segs, dtype=np.int32).reshape(-1, 4)}
 
 
+# Portions of at least so many tokens go through the chunk kernels (three launches of 50 to 60 us together at 16 heads, then
+# 80 ns per token; the walk: 145 ns per token and no start).  Measured, us, walk and chunks: 16 heads 256 tokens 45 and 56,
+# 512 tokens 82 and 58, 2048 tokens 297 and 161; 32 heads 512 tokens 107 and 91; 8 requests of 256 tokens, 32 heads, 288 and 319.
+CHUNK_FROM_TOKENS = 384
+
+
+def plan_scan_chunks(shape: StepShape) -> dict:
+    """The step planner of the decayed recurrences: when a request brings a long portion, its tokens in chunks of
+    ``K.CHUNK_TOKENS``: ``scan_chunks`` int32 [n, 3] = (request, first row, end row) and ``scan_chunk_requests`` [m, 3] =
+    (request, its first chunk, its chunks).  Shorter portions and single tokens are walked in order."""
+    if max(shape.q_lens) < CHUNK_FROM_TOKENS:
+        return {}
+    chunks, requests, n0 = [], [], 0
+    for r, T in enumerate(shape.q_lens):
+        if T >= CHUNK_FROM_TOKENS:
+            requests.append((r, len(chunks), -(-T // K.CHUNK_TOKENS)))
+            chunks += [(r, n0 + c, n0 + min(T, c + K.CHUNK_TOKENS)) for c in range(0, T, K.CHUNK_TOKENS)]
+        n0 += T
+    return {"scan_chunks": np.array(chunks, dtype=np.int32).reshape(-1, 3), "scan_chunk_requests": np.array(requests, dtype=np.int32).reshape(-1, 3)}
+
+
+def scan_chunks(ctx: StepContext, heads: int, dk: int, dv: int) -> "tuple[K.Chunks | None, torch.Tensor | None]":
+    """The step's chunks and the scratch of their states, if it has long portions of heads that the chunk kernels take."""
+    chunks = ctx.arrays.get("scan_chunks")
+    if chunks is None or not K.chunk_scan_supported(dk, dv):
+        return None, None
+    requests = ctx.arrays["scan_chunk_requests"]
+    n, m = chunks.numel() // 3, requests.numel() // 3
+    need = K.chunk_scan_scratch(n, heads, dk, dv)
+    scratch = ctx.workspace.get("chunk_scan", need, torch.float32) if ctx.workspace is not None else \
+        torch.empty(need, dtype=torch.float32, device=chunks.device)
+    return K.Chunks(chunks, requests, n, m, CHUNK_FROM_TOKENS, m < ctx.n_requests), scratch
+
+
 class HGRN2(InputConvMixer):
     """Gated linear recurrence with a matrix state per head, whose forget gate f doubles as the write gate 1 - f
     (keys do not exist in this form):  q = silu(W_q h), v = W_v h, f = lower + (1 - lower) * sigmoid(W_f h + b_f);
@@ -70,7 +104,7 @@ class HGRN2(InputConvMixer):
 
     ``w_qfv``: [2 H dk + H dv, D], the q, f and v projections stacked in that order."""
 
-    kernel_libraries = ("recurrent", "gemm_simt")
+    kernel_libraries = ("recurrent", "chunk_scan", "gemm_simt")
     kernel_libraries_bf16 = ("gemm_stream",)
 
     def __init__(self, w_qfv: torch.Tensor, f_bias: torch.Tensor, lower: torch.Tensor, norm_weight: torch.Tensor,
@@ -88,7 +122,7 @@ class HGRN2(InputConvMixer):
         return (StateNeed((self.heads, self.dim, self.vdim), torch.float32),)
 
     def step_planners(self):
-        return (plan_scan_segments,)
+        return (plan_scan_chunks,) if K.chunk_scan_supported(self.dim, self.vdim) else (plan_scan_segments,)
 
     def forward(self, ctx: StepContext, h, cache: LayerCache, h32: torch.Tensor | None = None):
         a, (state,) = self.read_input(ctx, h32, cache)
@@ -96,12 +130,13 @@ class HGRN2(InputConvMixer):
             qfv = as_rows(linear(ctx, a, self.w_qfv, torch.float32, partials=True))
         o = torch.empty((a.shape[0], self.heads * self.vdim), dtype=ctx.runtime.dtype, device=a.device)
         with scope("attention"):
-            segs = ctx.arrays.get("scan_segments")
+            chunks, chunk_scratch = scan_chunks(ctx, self.heads, self.dim, self.vdim)
+            segs = ctx.arrays.get("scan_segments") if chunks is None else None
             n_seg = 0 if segs is None else segs.numel() // 4
             need = K.hgrn2_scan_scratch(a.shape[0], self.heads, self.dim, self.vdim, n_seg)
             scratch = ctx.workspace.get("hgrn2_scan", need, torch.float32) if ctx.workspace else None
             K.hgrn2_scan(qfv.data, qfv.splits, self.f_bias, self.lower, state, ctx.cu_q, ctx.slot_ids, self.norm_weight,
-                         self.eps, o, self.heads, self.dim, self.vdim, scratch, segs if n_seg else None, n_seg, SEGMENT_TOKENS)
+                         self.eps, o, self.heads, self.dim, self.vdim, scratch, segs if n_seg else None, n_seg, SEGMENT_TOKENS, chunks, chunk_scratch)
         with scope("projection"):
             return linear(ctx, o, self.w_o, torch.float32, partials=True)
 

@@ -197,6 +197,53 @@ def test_decay_scan_sizes_and_a_batch_of_unequal_requests(dk, dv):
         at += n
 
 
+@pytest.mark.parametrize("dk, dv, H_", [(128, 128, 3), (68, 100, 2), (70, 127, 1)])
+@pytest.mark.parametrize("form", ["after", "before", "one minus"])
+def test_chunk_scan_sizes_strides_and_vanishing_decays(form, dk, dv, H_):
+    """The recurrence by chunks against float64, token by token: portions that end inside, at and behind a chunk's and a
+    piece's edge, heads smaller than 128 whose rows are no 16-byte pieces, operands inside wider rows, decays from 1 to
+    below 1e-30, a state to start from; slots in another order.  A sum over at most 3 x 128 products in float32, decays
+    multiplied up to 64 times: 5e-6 of the largest value."""
+    from jax_llm_examples_b200.kernels import api as K
+
+    torch.manual_seed(dk)
+    i32 = lambda x: torch.tensor(x, device=DEV, dtype=torch.int32)  # noqa: E731
+    lens, slots = [1, 64, 130, 15, 197, 65], [4, 0, 6, 2, 1, 3]
+    N = sum(lens)
+    wide = torch.randn(N, 3 * H_ * dk + H_ * dv + 8, device=DEV)
+    q, k, d = (wide[:, i * H_ * dk:(i + 1) * H_ * dk].unflatten(1, (H_, dk)) for i in range(3))
+    v = wide[:, 3 * H_ * dk:3 * H_ * dk + H_ * dv].unflatten(1, (H_, dv))
+    d.copy_(torch.sigmoid(2 * d + 2))
+    d[:, :, 1::7] = 1e-32
+    d[:, :, 2::7] = 1.0
+    d[:, :, 3::7] = 0.0
+    k.mul_(dk ** -0.5)
+    u = torch.randn(H_, dk, device=DEV) if form == "before" else None
+    state = torch.randn(7, H_, dk, dv, device=DEV)
+    before, o = state.clone(), torch.full((N, H_, dv), float("nan"), device=DEV)
+    chunks, requests, at = [], [], 0
+    for r, n in enumerate(lens):
+        requests.append((r, len(chunks), -(-n // 64)))
+        chunks += [(r, at + c, at + min(n, c + 64)) for c in range(0, n, 64)]
+        at += n
+    ch = K.Chunks(i32(chunks), i32(requests), len(chunks), len(requests), 1, False)
+    scratch = torch.empty(K.chunk_scan_scratch(ch.n, H_, dk, dv), device=DEV)
+    K.chunk_scan(q, None if form == "one minus" else k, d, v, u, state, i32(slots), o, form != "before", ch, scratch)
+    at = 0
+    for n, slot in zip(lens, slots):
+        S, want = before[slot].double(), []
+        for t in range(at, at + n):
+            dd, kk = d[t].double(), (1.0 - d[t].double()) if form == "one minus" else k[t].double()
+            kv = kk[:, :, None] * v[t].double()[:, None, :]
+            read = S + u.double()[:, :, None] * kv if form == "before" else dd[:, :, None] * S + kv
+            want.append(torch.einsum("hkv,hk->hv", read, q[t].double()))
+            S = dd[:, :, None] * S + kv
+        _close(o[at:at + n], torch.stack(want), 5e-6, f"outputs of {n} tokens")
+        _close(state[slot], S, 5e-6, f"state after {n} tokens")
+        at += n
+    assert torch.equal(state[5], before[5])
+
+
 def test_decay_forms():
     """exp(-exp(z + b)) and sigmoid(z + b)^(1 / tau) in 32-bit, also far out in both tails; q is scaled, k and v pass."""
     from jax_llm_examples_b200.kernels import api as K
