@@ -435,16 +435,18 @@ def hgrn2_scan(qfv: torch.Tensor, splits: int, f_bias: torch.Tensor, lower: torc
              _ptr(segments) if n_segments else None, c_int(n_segments), c_int(segment_tokens), _ptr(seg_state), _ptr(seg_decay),
              _ptr(qd), c_int(do), c_int(skip_from), _stream())
 
-    GATES, SCAN, NORM = 1, 2, 4  # csrc/recurrent.cu
+    GATES, SCAN, NORM, V_STAYS = 1, 2, 4, 8  # csrc/recurrent.cu
     if chunks is None or n_segments:
         run(GATES | SCAN | NORM)
         _launches += 2 + (2 if n_segments else 0)  # gates, scan, (chain, correction,) norm
         return
-    run(GATES | (SCAN if chunks.others else 0), chunks.long_from)
-    _launches += int(chunks.others)
     F = heads * dk
     rows = gates[:N * (2 * F + heads * dv)].view(N, -1)
-    chunk_scan(rows[:, F:2 * F].unflatten(1, (heads, dk)), None, rows[:, :F].unflatten(1, (heads, dk)), rows[:, 2 * F:].unflatten(1, (heads, dv)),
+    # v is read where it was projected, unless it is still in parts or the walk of the other requests needs it beside f and q
+    v = (rows if chunks.others or sp > 1 else qfv.view(N, -1))[:, 2 * F:].unflatten(1, (heads, dv))
+    run(GATES | (SCAN if chunks.others else 0) | (V_STAYS if not chunks.others and sp == 1 else 0), chunks.long_from)
+    _launches += int(chunks.others)
+    chunk_scan(rows[:, F:2 * F].unflatten(1, (heads, dk)), None, rows[:, :F].unflatten(1, (heads, dk)), v,
                None, state, slot_ids, o32[:N * heads * dv].view(N, heads, dv), True, chunks, chunk_scratch)
     run(NORM)
 
@@ -609,17 +611,17 @@ DECAY_FORMS = {"double_exp": 0, "sigmoid_power": 1, "head_constant": 2}  # csrc/
 
 
 def decay_prep(q: _RowsView, k: _RowsView, v: _RowsView, z: _RowsView | None, z_bias: torch.Tensor | None, form: str, tau: float,
-               q_scale: float, qo: torch.Tensor, ko: torch.Tensor, do: torch.Tensor, vo: torch.Tensor, heads: int, dk: int,
+               q_scale: float, qo: torch.Tensor | None, ko: torch.Tensor | None, do: torch.Tensor, vo: torch.Tensor | None, heads: int, dk: int,
                dv: int, head_decay: torch.Tensor | None = None, k_scale: float = 1.0, inv_freq: torch.Tensor | None = None,
                rot_dims: int = 0, positions: torch.Tensor | None = None) -> None:
     """qo = q_scale * q, ko = k_scale * k, vo = v, do = the decay of every key channel: exp(-exp(z + bias)) ("double_exp"),
     sigmoid(z + bias)^(1 / tau) ("sigmoid_power") or ``head_decay[h]`` ("head_constant": float32 [H], no z), all float32
     [N, H, dk] ([N, H, dv] for vo), from projected rows.  With ``rot_dims`` > 0, q and k are first turned on their first
-    rot_dims entries (entry i with i + rot_dims / 2) by the angle positions[n] * inv_freq[i]."""
+    rot_dims entries (entry i with i + rot_dims / 2) by the angle positions[n] * inv_freq[i].  qo, ko, vo None: not wanted
+    (only where ``decay_prep_selective``)."""
     _contig(z_bias, qo, ko, do, vo, head_decay, inv_freq, positions)
-    N = qo.shape[0]
-    if any(t.dtype != torch.float32 for t in (qo, ko, do, vo)) or any(
-            t is not None and t.dtype != torch.float32 for t in (z_bias, head_decay, inv_freq)):
+    N = do.shape[0]
+    if any(t is not None and t.dtype != torch.float32 for t in (qo, ko, do, vo, z_bias, head_decay, inv_freq)):
         raise KernelError("decay_prep: float32 outputs, bias, decays and frequencies are needed")
     if form == "head_constant" and (head_decay is None or head_decay.numel() != heads):
         raise KernelError(f"decay_prep: a constant decay per head needs {heads} numbers")
@@ -629,6 +631,20 @@ def decay_prep(q: _RowsView, k: _RowsView, v: _RowsView, z: _RowsView | None, z_
          _ptr(z_bias), c_int(DECAY_FORMS[form]), c_float(tau), c_float(q_scale), _ptr(qo), _ptr(ko), _ptr(do), _ptr(vo), c_int(N),
          c_int(heads), c_int(dk), c_int(dv), _ptr(head_decay), c_float(k_scale), _ptr(inv_freq), c_int(rot_dims), _ptr(positions),
          _stream())
+
+
+def decay_prep_selective(q: _RowsView, k: _RowsView, v: _RowsView, z: _RowsView | None, dk: int, dv: int, rot_dims: int) -> bool:
+    """Whether ``decay_prep`` can leave outputs out for these rows."""
+    return bool(library("decay_scan").jlx_decay_prep_selective(ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(z) if z is not None else None,
+                                                              c_int(dk), c_int(dv), c_int(rot_dims)))
+
+
+def view_rows(v: _RowsView, n: int, heads: int, size: int) -> torch.Tensor:
+    """The rows behind a view of whole projected rows (not split-K partials), as [n, heads, size]."""
+    if v.splits > 1:
+        raise KernelError("split-K partials are no rows yet")
+    flat = v.keep.view(-1)
+    return flat.as_strided((n, heads, size), (v.ld, size, 1), flat.storage_offset() + (v.p - flat.data_ptr()) // 4)
 
 
 def decay_scan(q: torch.Tensor, k: torch.Tensor, d: torch.Tensor, v: torch.Tensor, bonus: torch.Tensor | None, state: torch.Tensor,
