@@ -318,6 +318,35 @@ def test_prompt_softmax_stops_at_the_causal_edge_and_counts_the_sink_once(T, L, 
     assert torch.allclose(p0.sum(-1), torch.ones(H_, T, device=DEV), atol=1e-5)
 
 
+@pytest.mark.parametrize("L", [4, 1020, 1024, 1028, 2048, 2052, 4096, 4100, 1022])
+@pytest.mark.parametrize("window", [0, 70])
+def test_prompt_softmax_rows_in_registers_and_at_the_edges_of_their_lengths(L, window):
+    """Rows that a block holds in its registers (multiples of four up to 4096, in three lengths) and the ones behind: all
+    queries' edges and a window that leave out most keys, masked positions that hold infinities and NaN, lowest scores.
+    Weights of 32-bit sums of up to 4100 exponentials: 2e-6; rounded to bfloat16: 2^-8."""
+    from jax_llm_examples_b200.kernels import api as K
+
+    torch.manual_seed(L)
+    H_, T, scale = 2, 5, 0.7
+    start = max(0, L - T - 3)
+    s = torch.randn(H_, T, L, device=DEV) * 4
+    s[0, :, : L // 2] = torch.finfo(torch.float32).min
+    seen = torch.arange(L, device=DEV)[None] <= start + torch.arange(T, device=DEV)[:, None]
+    if window:
+        seen &= torch.arange(L, device=DEV)[None] > start + torch.arange(T, device=DEV)[:, None] - window
+    s[:, ~seen] = torch.tensor([float("nan"), float("inf")], device=DEV).repeat(int((~seen).sum()) // 2 + 1)[: int((~seen).sum())]
+    z = (s.double() * scale).masked_fill(~seen[None], -float("inf"))
+    sink = torch.tensor([0.5, -1.0], device=DEV)
+    for sk in (None, sink):
+        cat = z if sk is None else torch.cat([z, sk.double()[:, None, None].expand(H_, T, 1)], -1)
+        want = torch.softmax(cat, -1)[..., :L]
+        for out_dtype, tol in ((torch.float32, 2e-6), (torch.bfloat16, 2.0 ** -8)):
+            p = torch.full((H_, T, L), 7.0, device=DEV, dtype=out_dtype)
+            K.causal_sink_softmax(s, sk, scale, start, p, 0, window)
+            assert float((p.double() - want).abs().max()) < tol
+            assert not bool(p[:, ~seen].any())
+
+
 @pytest.mark.parametrize("name, dtype, tol", DTYPES)
 @pytest.mark.parametrize("D, F", [(40, 72), (38, 70)])  # four values per access, and one
 def test_biased_mlp_and_reinjection_block(name, dtype, tol, D, F):
