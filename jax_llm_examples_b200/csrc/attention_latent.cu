@@ -343,19 +343,25 @@ __global__ void attention_latent_kernel(const float* __restrict__ q_lat, const f
 }
 
 // ---- the same on the tensor cores (mma.sync), for a bfloat16 cache: the decoded tokens of a step
-// One block of four warps serves one query token, up to 16 heads (the M rows of the products) and one range of keys.
-// Tiles of 32 keys come by cp.async, found row by row through the block table, two in flight; a key's row [c | k_rot] in
-// shared memory is padded by 16 bytes so that ldmatrix meets no bank twice.
-//   scores   warp w takes keys [8 w, 8 w + 8) of the tile: the whole row against all 16 queries (bfloat16, 32-bit sums)
-//   softmax  the scores meet in shared memory; every warp keeps the same running maximum and sum per head (32-bit)
-//   values   warp w takes the latent's 16-column pieces w, w + 4, ...: P (bfloat16) times the tile's rows
+// One block of eight warps serves one query token, up to 16 heads (the M rows of the products) and one range of keys.
+// Tiles of 32 keys come by cp.async, two in flight, found through the block table: once per tile where pages are multiples of
+// the tile, else row by row; a key's row [c | k_rot] in shared memory is padded by 16 bytes so that ldmatrix meets no bank
+// twice.
+//   scores   warp w takes keys [8 (w % 4), + 8) of the tile and one half of the row against all 16 queries (bfloat16,
+//            32-bit sums); the halves meet in shared memory
+//   softmax  warp w takes heads 2 w and 2 w + 1, a key per lane: running maximum and sum (32-bit), the weights in bfloat16
+//   values   warp w takes the latent's 16-column pieces w, w + 8, ...: the weights times the tile's rows
+// Bound by the latency of a tile's chain and its instructions: with two blocks of 37 KB tiles an SM, eight warps that each
+// did the softmax of all heads took 6 us a tile.  32 requests of 4096 keys, 16 heads: 56 us (81).
 // When every served token is its request's only one of the step (`single`), everything but its own row is older than the
 // step: tiles that end below it are asked for before the wait for the predecessor.  Rows outside [lo, t_end] are zeros in shared memory and masked.
 #define LATM_KEYS LAT_TILE
-#define LATM_THREADS 128
+#define LATM_WARPS 8
+#define LATM_THREADS (LATM_WARPS * 32)
+#define LATM_LDP 40  // row of the weights in shared memory
 
 template <typename TO, int PIECES>
-__global__ void __launch_bounds__(LATM_THREADS)
+__global__ void __launch_bounds__(LATM_THREADS, 2)
 attention_latent_mma_kernel(const bf16* __restrict__ q_lat, const bf16* __restrict__ q_rot, const bf16* __restrict__ pages,
                             const int* __restrict__ block_table, int bt_stride, const int* __restrict__ req_of_token,
                             const int* __restrict__ positions, const float* __restrict__ sink, TO* __restrict__ out_lat, int N,
@@ -364,7 +370,9 @@ attention_latent_mma_kernel(const bf16* __restrict__ q_lat, const bf16* __restri
                             int window, int single, int* status) {
   JLX_TL(TL_ATTN_GENERIC);
   extern __shared__ __align__(16) uint8_t smem_bytes[];
-  __shared__ float sc[2][16][LATM_KEYS + 1];
+  __shared__ float sc[2][16][LATM_KEYS + 2];         // the halves' scores
+  __shared__ __align__(16) bf16 pw[16][LATM_LDP];    // the weights
+  __shared__ float corr_of[16], m_of[16], l_of[16];
   const int dk = rank + dr, dkp = (dk + 15) & ~15;  // products take 16 columns at a time: the rest of a row is zero
   bf16* qs = reinterpret_cast<bf16*>(smem_bytes);   // [16][ldk]
   bf16* ks = qs + 16 * ldk;                          // [2][LATM_KEYS][ldk]
@@ -382,13 +390,25 @@ attention_latent_mma_kernel(const bf16* __restrict__ q_lat, const bf16* __restri
   const int* table = block_table + (size_t)r * bt_stride;
   const int chunks = dk >> 3;  // 16-byte pieces of a row
   bool bad_page = false;
+  const bool whole_tiles = page_size % LATM_KEYS == 0;  // a tile lies in one page
   auto load = [&](int t) {  // a warp copies a row with neighbouring lanes
     bf16* dst = ks + (size_t)(t & 1) * LATM_KEYS * ldk;
-    for (int j = warp; j < LATM_KEYS; j += LATM_THREADS / 32) {
-      const int pos = t_begin + t * LATM_KEYS + j;
+    const int pos0 = t_begin + t * LATM_KEYS;
+    const bf16* first = nullptr;
+    if (whole_tiles) {
+      const int page = table[pos0 / page_size];
+      if (page < 0 || page >= num_pages) bad_page = true;
+      else first = pages + ((size_t)page * page_size + pos0 % page_size) * dk;
+    }
+#pragma unroll
+    for (int u = 0; u < LATM_KEYS / LATM_WARPS; ++u) {
+      const int j = warp + u * LATM_WARPS, pos = pos0 + j;
       bool valid = pos >= lo && pos <= t_end;
       const bf16* src = pages;
-      if (valid) {
+      if (whole_tiles) {
+        if (first) src = first + (size_t)j * dk;
+        else valid = false;
+      } else if (valid) {
         const int page = table[pos / page_size];
         if (page < 0 || page >= num_pages) { bad_page = true; valid = false; }
         else src = pages + ((size_t)page * page_size + pos % page_size) * dk;
@@ -405,7 +425,7 @@ attention_latent_mma_kernel(const bf16* __restrict__ q_lat, const bf16* __restri
   if (early1) { load(1); cp_async_commit(); }
   pdl_launch_dependents_if_small();
   pdl_wait();
-  for (int u = warp; u < 16; u += LATM_THREADS / 32) {  // heads beyond H get a zero query: they run along and write nothing
+  for (int u = warp; u < 16; u += LATM_WARPS) {  // heads beyond H get a zero query: they run along and write nothing
     const int h = h0 + u;
     const bool valid = h < H;
     const bf16* a = q_lat + ((size_t)(valid ? h : 0) * N + blockIdx.x) * rank;
@@ -422,10 +442,10 @@ attention_latent_mma_kernel(const bf16* __restrict__ q_lat, const bf16* __restri
   const int g0 = lane >> 2, g1 = g0 + 8;  // this thread's two heads
   const float sc2 = scale * 1.4426950408889634f;
   const bool has_sink = sink != nullptr && z == 0;
-  float m[2], l[2];  // base-2 running maximum and sum
+  float m[2], l[2];  // base-2 running maximum and sum of heads 2 warp and 2 warp + 1
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
-    const int h = h0 + (u ? g1 : g0);
+    const int h = h0 + 2 * warp + u;
     m[u] = has_sink && h < H ? sink[h] * 1.4426950408889634f : -INFINITY;
     l[u] = has_sink ? 1.f : 0.f;
   }
@@ -444,12 +464,14 @@ attention_latent_mma_kernel(const bf16* __restrict__ q_lat, const bf16* __restri
       cp_async_commit();
     }
     const bf16* kt = ks + (size_t)(t & 1) * LATM_KEYS * ldk;
-    // scores of this warp's 8 keys; two chains of sums
+    // scores of this warp's 8 keys over its half of the row (whole 32 columns); two chains of sums
     float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+    const int kw = warp & 3, half = warp >> 2, mid = (dkp / 2 + 31) & ~31, d_end = half ? dkp : min(mid, dkp);
     const uint32_t qa = smem_u32(qs + (size_t)(lane & 15) * ldk + (lane >> 4) * 8);
-    const uint32_t ka = smem_u32(kt + (size_t)(warp * 8 + (lane & 7)) * ldk + (lane >> 3) * 8);
-    int d = 0;
-    for (; d + 32 <= dkp; d += 32) {
+    const uint32_t ka = smem_u32(kt + (size_t)(kw * 8 + (lane & 7)) * ldk + (lane >> 3) * 8);
+    int d = half ? mid : 0;
+#pragma unroll 3
+    for (; d + 32 <= d_end; d += 32) {
       uint32_t a[4], b[4], c[4];
       ldmatrix_x4(qa + d * 2, a[0], a[1], a[2], a[3]);
       ldmatrix_x4(qa + d * 2 + 32, c[0], c[1], c[2], c[3]);
@@ -457,69 +479,40 @@ attention_latent_mma_kernel(const bf16* __restrict__ q_lat, const bf16* __restri
       mma_bf16(s0, a, b[0], b[1]);
       mma_bf16(s1, c, b[2], b[3]);
     }
-    if (d < dkp) {  // 16 columns are left (lanes 16.. read columns that are in the row's padding or the next row: unused)
+    if (d < d_end) {  // 16 columns are left (lanes 16.. read columns that are in the row's padding or the next row: unused)
       uint32_t a[4], b[4];
       ldmatrix_x4(qa + d * 2, a[0], a[1], a[2], a[3]);
-      ldmatrix_x4(smem_u32(kt + (size_t)(warp * 8 + (lane & 7)) * ldk + ((lane >> 3) & 1) * 8) + d * 2, b[0], b[1], b[2], b[3]);
+      ldmatrix_x4(smem_u32(kt + (size_t)(kw * 8 + (lane & 7)) * ldk + ((lane >> 3) & 1) * 8) + d * 2, b[0], b[1], b[2], b[3]);
       mma_bf16(s0, a, b[0], b[1]);
     }
     {
-      float* w0 = &sc[t & 1][g0][warp * 8 + (lane & 3) * 2];
-      float* w1 = &sc[t & 1][g1][warp * 8 + (lane & 3) * 2];
-      w0[0] = s0[0] + s1[0]; w0[1] = s0[1] + s1[1];
-      w1[0] = s0[2] + s1[2]; w1[1] = s0[3] + s1[3];
+      float* w0 = &sc[half][g0][kw * 8 + (lane & 3) * 2];
+      float* w1 = &sc[half][g1][kw * 8 + (lane & 3) * 2];
+      *reinterpret_cast<float2*>(w0) = make_float2(s0[0] + s1[0], s0[1] + s1[1]);
+      *reinterpret_cast<float2*>(w1) = make_float2(s0[2] + s1[2], s0[3] + s1[3]);
     }
     __syncthreads();
-    // every warp: the 32 keys' weights of its lanes' two heads, in the layout of the product's A operand
-    float pv[2][2][4];  // [16-key step][head][columns 2 (lane & 3) + {0, 1, 8, 9}]
-    float mx[2] = {m[0], m[1]};
-    const int tile_key = t_begin + t * LATM_KEYS;
-#pragma unroll
-    for (int st = 0; st < 2; ++st)
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int j = st * 16 + (lane & 3) * 2 + (e & 1) + (e >> 1) * 8;
-          const bool seen = tile_key + j >= lo && tile_key + j <= t_end;
-          const float s = seen ? sc[t & 1][u ? g1 : g0][j] * sc2 : -INFINITY;
-          pv[st][u][e] = s;
-          mx[u] = fmaxf(mx[u], s);
-        }
-    float corr[2], rs[2] = {0.f, 0.f};
+    const int key = t_begin + t * LATM_KEYS + lane;
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      mx[u] = fmaxf(mx[u], __shfl_xor_sync(0xffffffffu, mx[u], 1));
-      mx[u] = fmaxf(mx[u], __shfl_xor_sync(0xffffffffu, mx[u], 2));  // a tile has a visible key: never -infinity
-      corr[u] = exp2f(m[u] - mx[u]);
+      const int hd = 2 * warp + u;
+      const float s = key >= lo && key <= t_end ? (sc[0][hd][lane] + sc[1][hd][lane]) * sc2 : -INFINITY;
+      const float mx = fmaxf(m[u], warp_max(s));  // a tile has a visible key: never -infinity
+      const float corr = exp2f(m[u] - mx), w = exp2f(s - mx);
+      l[u] = l[u] * corr + warp_sum(w);
+      m[u] = mx;
+      pw[hd][lane] = __float2bfloat16_rn(w);
+      if (lane == 0) corr_of[hd] = corr;
     }
-#pragma unroll
-    for (int st = 0; st < 2; ++st)
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          pv[st][u][e] = exp2f(pv[st][u][e] - mx[u]);
-          rs[u] += pv[st][u][e];
-        }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      rs[u] += __shfl_xor_sync(0xffffffffu, rs[u], 1);
-      rs[u] += __shfl_xor_sync(0xffffffffu, rs[u], 2);
-      l[u] = l[u] * corr[u] + rs[u];
-      m[u] = mx[u];
-    }
+    __syncthreads();
+    const float corr[2] = {corr_of[g0], corr_of[g1]};
     uint32_t pa[2][4];
 #pragma unroll
-    for (int st = 0; st < 2; ++st) {
-      pa[st][0] = pack_bf16(pv[st][0][0], pv[st][0][1]);
-      pa[st][1] = pack_bf16(pv[st][1][0], pv[st][1][1]);
-      pa[st][2] = pack_bf16(pv[st][0][2], pv[st][0][3]);
-      pa[st][3] = pack_bf16(pv[st][1][2], pv[st][1][3]);
-    }
+    for (int st = 0; st < 2; ++st)
+      ldmatrix_x4(smem_u32(&pw[lane & 15][st * 16 + (lane >> 4) * 8]), pa[st][0], pa[st][1], pa[st][2], pa[st][3]);
 #pragma unroll
     for (int i = 0; i < PIECES; ++i) {
-      const int col = (warp + i * 4) * 16;
+      const int col = (warp + i * LATM_WARPS) * 16;
       if (col >= rank) break;
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
@@ -536,23 +529,28 @@ attention_latent_mma_kernel(const bf16* __restrict__ q_lat, const bf16* __restri
   }
   cp_async_wait<0>();
   if (bad_page) atomicOr(status, JLX_STATUS_BAD_PAGE);
+  if (lane < 2) {
+    m_of[2 * warp + lane] = lane ? m[1] : m[0];
+    l_of[2 * warp + lane] = lane ? l[1] : l[0];
+  }
+  __syncthreads();
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     const int h = h0 + (u ? g1 : g0);
     if (h >= H) continue;
     const size_t slot = ((size_t)blockIdx.x * H + h) * splits + z;
     if (splits > 1 && warp == 0 && (lane & 3) == 0) {
-      part_ml[2 * slot] = m[u] * 0.6931471805599453f;  // the combine kernel works with natural exponentials
-      part_ml[2 * slot + 1] = l[u];
+      part_ml[2 * slot] = m_of[u ? g1 : g0] * 0.6931471805599453f;  // the combine kernel works with natural exponentials
+      part_ml[2 * slot + 1] = l_of[u ? g1 : g0];
     }
-    const float inv = 1.f / l[u];
+    const float inv = 1.f / l_of[u ? g1 : g0];
 #pragma unroll
     for (int i = 0; i < PIECES; ++i)
 #pragma unroll
       for (int q = 0; q < 2; ++q)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const int c = (warp + i * 4) * 16 + q * 8 + (lane & 3) * 2 + e;
+          const int c = (warp + i * LATM_WARPS) * 16 + q * 8 + (lane & 3) * 2 + e;
           if (c >= rank) continue;
           if (splits > 1) part_acc[slot * rank + c] = o[i][q][u * 2 + e];
           else out_lat[((size_t)h * N + blockIdx.x) * rank + c] = from_f32<TO>(o[i][q][u * 2 + e] * inv);
@@ -645,9 +643,9 @@ JLX_API int jlx_attention_latent(const void* q_lat, const void* q_rot, const voi
                             dr, page_size, num_pages, scale, rows, splits, split_keys, part_acc, part_ml, ldm, window, single, status)); \
   } while (0)
     JLX_DISPATCH_DTYPE(out_dtype, TO, {
-      if (rank <= 128) LATM_GO(2);
-      else if (rank <= 512) LATM_GO(8);
-      else LATM_GO(16);
+      if (rank <= 128) LATM_GO(1);
+      else if (rank <= 512) LATM_GO(4);
+      else LATM_GO(8);
     });
 #undef LATM_GO
     JLX_LAUNCH_CHECK("attention_latent_mma");
@@ -791,6 +789,8 @@ __global__ void causal_sink_softmax_kernel(const float* __restrict__ s, const fl
   for (int j = first + threadIdx.x; j < visible; j += blockDim.x) l += expf(row[j] * scale - m);
   l = block_sum(l, scratch) + (sink ? expf(sink[h] - m) : 0.f);
   for (int j = threadIdx.x; j < L; j += blockDim.x) out[j] = from_f32<TO>(j >= first && j < visible ? expf(row[j] * scale - m) / l : 0.f);
+}
+
 // Rows of up to 1024 NV scores on 16-byte boundaries: the visible scores stay in a thread's registers, so every score is read
 // once, exponentiated once and written once, with two meetings of the block.  16 heads, 512 query rows, 3048 keys (100 MB of
 // scores, 50 MB of weights): the four query tiles of a 2048-token portion 113 us, 202 by the general kernel.
@@ -847,10 +847,10 @@ causal_sink_softmax_x4_kernel(const float* __restrict__ s, const float* __restri
   }
 }
 
-}
-
 JLX_API int jlx_causal_sink_softmax(const float* s, const float* sink, float scale, int q_start, int k_start, int window, void* p,
                                     int dtype, int H, int T, int L, cudaStream_t stream) {
+  JLX_REQUIRE(H > 0 && T >= 0 && L > 0 && q_start >= 0 && k_start >= 0 && k_start <= q_start && window >= 0 && H <= 65535, "causal_sink_softmax: bad sizes");
+  if (T == 0) return 0;
   if ((L & 3) == 0 && L <= 4096 && (((uintptr_t)s | (uintptr_t)p) & 15) == 0) {
     JLX_DISPATCH_DTYPE(dtype, TO, {
       const auto kernel = L <= 1024 ? causal_sink_softmax_x4_kernel<TO, 1> : (L <= 2048 ? causal_sink_softmax_x4_kernel<TO, 2> : causal_sink_softmax_x4_kernel<TO, 4>);
@@ -859,8 +859,6 @@ JLX_API int jlx_causal_sink_softmax(const float* s, const float* sink, float sca
     JLX_LAUNCH_CHECK("causal_sink_softmax");
     return 0;
   }
-  JLX_REQUIRE(H > 0 && T >= 0 && L > 0 && q_start >= 0 && k_start >= 0 && k_start <= q_start && window >= 0 && H <= 65535, "causal_sink_softmax: bad sizes");
-  if (T == 0) return 0;
   const int staged = (size_t)L * 4 <= 160 * 1024;
   const size_t smem = staged ? (size_t)(L + 4) * 4 : 0;
   JLX_DISPATCH_DTYPE(dtype, TO, {

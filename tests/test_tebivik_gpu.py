@@ -347,6 +347,39 @@ def test_prompt_softmax_rows_in_registers_and_at_the_edges_of_their_lengths(L, w
             assert not bool(p[:, ~seen].any())
 
 
+@pytest.mark.parametrize("page", [16, 24, 32, 64])
+@pytest.mark.parametrize("rank, dr, H_", [(32, 8, 3), (128, 64, 16), (136, 0, 17), (512, 64, 16), (520, 16, 5), (768, 64, 2)])
+def test_latent_decode_on_the_tensor_cores_at_the_edges_of_its_pieces(rank, dr, H_, page):
+    """The kernel for bfloat16 queries: latents of one, a few and many 16-column pieces per warp, more heads than a block's, pages
+    that hold whole tiles of 32 keys and that do not, contexts at a tile's and a page's edges, one range and several, with and
+    without a window.  Weights rounded to bfloat16: 2^-8 of the largest value and the sums' own rounding."""
+    from jax_llm_examples_b200.kernels import api as K
+
+    torch.manual_seed(rank + page)
+    lens = [1, 31, 32, 33, 64, 65, 97, 200]
+    R, most = len(lens), -(-max(lens) // page)
+    table = torch.randperm(R * most, device=DEV).to(torch.int32).reshape(R, most)
+    pages = torch.randn(R * most, 1, 1, page, rank + dr, device=DEV).bfloat16()
+    q_lat, q_rot = torch.randn(H_, R, rank, device=DEV).bfloat16(), torch.randn(R, H_, dr, device=DEV).bfloat16()
+    sink, scale = torch.randn(H_, device=DEV), (rank + dr) ** -0.5
+    i32 = lambda v: torch.tensor(v, device=DEV, dtype=torch.int32)  # noqa: E731
+    status = torch.zeros(1, device=DEV, dtype=torch.int32)
+    for window in (0, 40):
+        for split_keys in (256, 64):
+            splits = -(-max(lens) // split_keys)
+            out = torch.full((H_, R, rank), float("nan"), device=DEV, dtype=torch.bfloat16)
+            acc, ml = torch.empty(R * H_ * splits * rank, device=DEV), torch.empty(R * H_ * splits * 2, device=DEV)
+            K.attention_latent(q_lat, q_rot, pages, table, i32(list(range(R))), i32([n - 1 for n in lens]), sink, out, scale, status,
+                               None, 0, splits, split_keys, acc, ml, window, single_tokens=True)
+            assert int(status) == 0
+            for r, n in enumerate(lens):
+                keys = pages[table[r].long()].reshape(-1, rank + dr)[max(0, n - window) if window else 0:n].double()
+                z = scale * torch.cat([q_lat[:, r], q_rot[r]], -1).double() @ keys.T
+                w = torch.softmax(torch.cat([z, sink.double()[:, None]], -1), -1)[:, :-1]
+                want = w @ keys[:, :rank]
+                assert float((out[:, r].double() - want).abs().max()) < 2.0 ** -7 * float(keys.abs().max()), (n, window, split_keys)
+
+
 @pytest.mark.parametrize("name, dtype, tol", DTYPES)
 @pytest.mark.parametrize("D, F", [(40, 72), (38, 70)])  # four values per access, and one
 def test_biased_mlp_and_reinjection_block(name, dtype, tol, D, F):
