@@ -19,7 +19,7 @@
 // elsewhere moves the last bits of a result, no more.
 // Bound by 32-bit FMAs (2 x 128 x 128 per token and head for the two products, and about half as many for A) and, in
 // chunk_outputs, by the shared-memory reads and shuffles of A's diagonal.  One request of 2048 tokens, 16 heads of 128 x 128:
-// states 37 us, chain 16, outputs 98 (the token-by-token walk: 297); 32 heads: 294 (397).
+// states 36 us, chain 16, outputs 84, together 144 (the token-by-token walk: 297); 32 heads: 263 (398).
 #include "common.cuh"
 
 #define CHUNK 64
@@ -51,6 +51,13 @@ __device__ __forceinline__ unsigned long long ch_fma2(unsigned long long a, unsi
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
+typedef unsigned long long u64;
+__device__ __forceinline__ u64 ch_mul2(u64 a, u64 b) {
+  u64 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ u64 ch_pair(float x, float y) { return (u64)__float_as_uint(x) | ((u64)__float_as_uint(y) << 32); }
 __device__ __forceinline__ unsigned long long ch_twice(float x) {
   return (unsigned long long)__float_as_uint(x) | ((unsigned long long)__float_as_uint(x) << 32);
 }
@@ -257,49 +264,66 @@ __global__ void __launch_bounds__(CH_THREADS, 2) chunk_outputs_kernel(const __gr
     ch_one_minus(K, D);
     __syncthreads();
   }
-  // A on the diagonal: thread (s, group of eight channels 4 g .., 64 + 4 g ..) decays k_s from token to token
+  // A on the diagonal: a thread decays k_s and k_(s + 8), eight channels (4 g .., 64 + 4 g ..) of each, from token to token;
+  // half of the block takes the even pieces, half the odd ones
   {
-    const int g = tid & 15, sl = tid >> 4;
-    float u[8];
+    const int g = tid & 15, sl = (tid >> 4) & 7;
+    u64 u[4];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const int c = (e < 4 ? 0 : 64) + 4 * g + (e & 3);
-      u[e] = !READ_AFTER && P.bonus && c < P.dk ? P.bonus[head * P.dk + c] : 0.f;
+    for (int e = 0; e < 4; ++e) {
+      const int c = (e < 2 ? 0 : 64) + 4 * g + 2 * (e & 1);
+      auto bonus = [&](int i) { return !READ_AFTER && P.bonus && i < P.dk ? P.bonus[head * P.dk + i] : 0.f; };
+      u[e] = ch_pair(bonus(c), bonus(c + 1));
     }
+    auto eight = [&](const float* row, u64 (&x)[4]) {
+      const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(row + 4 * g), hi = *reinterpret_cast<const ulonglong2*>(row + 64 + 4 * g);
+      x[0] = lo.x; x[1] = lo.y; x[2] = hi.x; x[3] = hi.y;
+    };
 #pragma unroll 1
-    for (int p = 0; p < CHUNK / PIECE; ++p) {
-      if (p * PIECE >= cnt) {  // no tokens: A is not read there beyond what is set to zero below
-        for (int t = 0; t < PIECE; ++t)
-          if (g == 0) A[(p * (p + 3) / 2 * PIECE + t) * PIECE + sl] = 0.f;
-        continue;
-      }
-      const int s = p * PIECE + sl;
-      float w[8];
-      {
-        const float4 a = *reinterpret_cast<const float4*>(K + s * CH_LD + 4 * g), b = *reinterpret_cast<const float4*>(K + s * CH_LD + 64 + 4 * g);
-        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
-        w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
-      }
-#pragma unroll 4
-      for (int tl = 0; tl < PIECE; ++tl) {
-        const int t = p * PIECE + tl;
-        const float4 q0 = *reinterpret_cast<const float4*>(Q + t * CH_LD + 4 * g), q1 = *reinterpret_cast<const float4*>(Q + t * CH_LD + 64 + 4 * g);
-        const float4 d0 = *reinterpret_cast<const float4*>(D + t * CH_LD + 4 * g), d1 = *reinterpret_cast<const float4*>(D + t * CH_LD + 64 + 4 * g);
-        const float q[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w}, d[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-        float sum = 0.f;
+    for (int p = tid >> 7; p < CHUNK / PIECE; p += 2) {
+      float* out = A + p * (p + 3) / 2 * PIECE * PIECE;
+      u64 w[2][4];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          if (READ_AFTER) {
-            if (tl > sl) w[e] *= d[e];
-            sum = fmaf(q[e], w[e], sum);
-          } else {
-            sum = fmaf(q[e], tl == sl ? u[e] * w[e] : w[e], sum);
-            if (tl > sl) w[e] *= d[e];
+      for (int x = 0; x < 2; ++x) eight(K + (p * PIECE + sl + 8 * x) * CH_LD, w[x]);
+#pragma unroll 2
+      for (int t0 = 0; t0 < PIECE; t0 += 2) {
+        float v[2][2];  // [token][s]
+#pragma unroll
+        for (int tt = 0; tt < 2; ++tt) {
+          const int tl = t0 + tt;
+          u64 q[4], d[4];
+          eight(Q + (p * PIECE + tl) * CH_LD, q);
+          eight(D + (p * PIECE + tl) * CH_LD, d);
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const int s = sl + 8 * x;
+            u64 sum = 0ull;
+            if (READ_AFTER && tl > s)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) w[x][e] = ch_mul2(w[x][e], d[e]);
+            if (!READ_AFTER && tl == s) {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) sum = ch_fma2(q[e], ch_mul2(u[e], w[x][e]), sum);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) sum = ch_fma2(q[e], w[x][e], sum);
+            }
+            if (!READ_AFTER && tl > s)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) w[x][e] = ch_mul2(w[x][e], d[e]);
+            v[tt][x] = ch_low(sum) + ch_high(sum);
           }
         }
+        // sixteen lanes add four numbers in five exchanges: each step halves the numbers a lane still carries
+        const bool up8 = g & 8, up4 = g & 4;
+        float y[2];
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (g == 0) A[(p * (p + 3) / 2 * PIECE + tl) * PIECE + sl] = tl >= sl ? sum : 0.f;
+        for (int x = 0; x < 2; ++x) y[x] = (up8 ? v[1][x] : v[0][x]) + __shfl_xor_sync(0xffffffffu, up8 ? v[0][x] : v[1][x], 8);
+        float z = (up4 ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, up4 ? y[0] : y[1], 4);
+        z += __shfl_xor_sync(0xffffffffu, z, 2);
+        z += __shfl_xor_sync(0xffffffffu, z, 1);
+        const int t = t0 + (up8 ? 1 : 0), s = sl + (up4 ? 8 : 0);
+        if ((g & 3) == 0) out[t * PIECE + s] = t >= s ? z : 0.f;
       }
     }
   }
@@ -340,7 +364,12 @@ __global__ void __launch_bounds__(CH_THREADS, 2) chunk_outputs_kernel(const __gr
   for (int p = 1; p < CHUNK / PIECE; ++p) {
     const int sl = tid & 15, tl = tid >> 4;
     if (p > 1) {  // the pieces before the last one are decayed over it
-      for (int idx = tid; idx < (p - 1) * PIECE * CH_D; idx += CH_THREADS) K[idx / CH_D * CH_LD + idx % CH_D] *= tot[(p - 1) * CH_D + idx % CH_D];
+      const int c = 4 * (tid & 31);
+      const ulonglong2 by = *reinterpret_cast<const ulonglong2*>(tot + (p - 1) * CH_D + c);
+      for (int t = tid >> 5; t < (p - 1) * PIECE; t += CH_THREADS / 32) {
+        ulonglong2* k = reinterpret_cast<ulonglong2*>(K + t * CH_LD + c);
+        *k = make_ulonglong2(ch_mul2(k->x, by.x), ch_mul2(k->y, by.y));
+      }
       __syncthreads();
     }
     unsigned long long sum[3] = {0ull, 0ull, 0ull};
@@ -363,12 +392,20 @@ __global__ void __launch_bounds__(CH_THREADS, 2) chunk_outputs_kernel(const __gr
   load_quarter(0);  // the keys are read: their place serves the start state
   load_quarter(1);
   // rows of q decayed from the chunk's start
-  for (int idx = tid; idx < (CHUNK - PIECE) * CH_D; idx += CH_THREADS) {
-    const int t = PIECE + idx / CH_D, c = idx % CH_D;
-    float before = tot[c];
-    if (t >= 2 * PIECE) before *= tot[CH_D + c];
-    if (t >= 3 * PIECE) before *= tot[2 * CH_D + c];
-    Q[t * CH_LD + c] *= before;
+  {
+    const int c = 4 * (tid & 31);
+    ulonglong2 before = *reinterpret_cast<const ulonglong2*>(tot + c);
+#pragma unroll
+    for (int p = 1; p < CHUNK / PIECE; ++p) {
+      for (int t = p * PIECE + (tid >> 5); t < (p + 1) * PIECE; t += CH_THREADS / 32) {
+        ulonglong2* q = reinterpret_cast<ulonglong2*>(Q + t * CH_LD + c);
+        *q = make_ulonglong2(ch_mul2(q->x, before.x), ch_mul2(q->y, before.y));
+      }
+      if (p + 1 < CHUNK / PIECE) {
+        const ulonglong2 by = *reinterpret_cast<const ulonglong2*>(tot + p * CH_D + c);
+        before = make_ulonglong2(ch_mul2(before.x, by.x), ch_mul2(before.y, by.y));
+      }
+    }
   }
   const int tx = tid & 15, ty = tid >> 4;
   unsigned long long acc[4][4];

@@ -62,9 +62,9 @@ def plan_scan_segments(shape: StepShape) -> dict:
     return {"scan_segments": np.array(segs, dtype=np.int32).reshape(-1, 4)}
 
 
-# Portions of at least so many tokens go through the chunk kernels (three launches of 50 to 60 us together at 16 heads, then
-# 80 ns per token; the walk: 145 ns per token and no start).  Measured, us, walk and chunks: 16 heads 256 tokens 45 and 56,
-# 512 tokens 82 and 58, 2048 tokens 297 and 161; 32 heads 512 tokens 107 and 91; 8 requests of 256 tokens, 32 heads, 288 and 319.
+# Portions of at least so many tokens go through the chunk kernels (three launches of 50 us together at 16 heads, then
+# 65 ns per token; the walk: 145 ns per token and no start).  Measured, us, walk and chunks: 16 heads 256 tokens 46 and 50,
+# 512 tokens 81 and 52, 2048 tokens 297 and 144; 32 heads 512 tokens 108 and 81; 8 requests of 256 tokens, 32 heads, 288 and 290.
 CHUNK_FROM_TOKENS = 384
 
 
