@@ -408,12 +408,13 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // One warp per (token, key head).
 __global__ void __launch_bounds__(256) delta_gram_kernel(const float* __restrict__ q, const float* __restrict__ k,
                                                          const int* __restrict__ cu_q, const int* __restrict__ req_of_token,
-                                                         float* __restrict__ gram, int G, int dk) {
+                                                         float* __restrict__ gram, int G, int dk, int skip_from) {
   JLX_TL(TL_OTHER);
   pdl_launch_dependents_if_small();
   pdl_wait();
-  const int n = blockIdx.x, lane = threadIdx.x & 31;
-  const int t = (n - cu_q[req_of_token[n]]) % DELTA_TB;
+  const int n = blockIdx.x, lane = threadIdx.x & 31, r = req_of_token[n];
+  if (skip_from > 0 && cu_q[r + 1] - cu_q[r] >= skip_from) return;
+  const int t = (n - cu_q[r]) % DELTA_TB;
   for (int kh = threadIdx.x >> 5; kh < G; kh += blockDim.x >> 5) {
     const float* qn = q + ((size_t)n * G + kh) * dk;
     const float* kn = k + ((size_t)n * G + kh) * dk;
@@ -441,7 +442,7 @@ __global__ void __launch_bounds__(DELTA_W * 32) delta_scan_kernel(const float* _
                                                          const float* __restrict__ decay, float* __restrict__ state,
                                                          const int* __restrict__ cu_q, const int* __restrict__ slot_ids,
                                                          const float* __restrict__ gram, float* __restrict__ o, int G, int H,
-                                                         int dk, int dv) {
+                                                         int dk, int dv, int skip_from) {
   JLX_TL(TL_OTHER);
   pdl_launch_dependents_if_small();
   constexpr int T = DELTA_TB;
@@ -464,7 +465,7 @@ __global__ void __launch_bounds__(DELTA_W * 32) delta_scan_kernel(const float* _
   }
   pdl_wait();
   const int n0 = cu_q[r], n1 = cu_q[r + 1];
-  if (n1 <= n0) return;
+  if (n1 <= n0 || (skip_from > 0 && n1 - n0 >= skip_from)) return;  // long portions may be walked by other kernels
   float* S = state + ((size_t)slot_ids[r] * H + hd) * dk * dv;
   float s[NR];
 #pragma unroll
@@ -639,22 +640,23 @@ __global__ void __launch_bounds__(DELTA_W * 32) delta_scan_kernel(const float* _
 template <int NR>
 static int launch_delta_scan(const float* q, const float* k, const float* v, const float* beta, const float* decay, float* state,
                              const int* cu_q, const int* slot_ids, const float* gram, float* o, int R, int G, int H, int dk, int dv,
-                             cudaStream_t stream) {
+                             int skip_from, cudaStream_t stream) {
   constexpr int W = DELTA_W;
   constexpr size_t smem = sizeof(float) * (2 * ((size_t)2 * DELTA_TB * W * NR + DELTA_TB * 32 + 2 * DELTA_TB + 2 * DELTA_TB * DELTA_TB) +
                                            (size_t)2 * DELTA_TB * W * 32 + 2 * DELTA_TB * 32);
   if (smem > 48 * 1024) JLX_CUDA(cudaFuncSetAttribute(delta_scan_kernel<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   JLX_CUDA(jlx_launch_pdl(delta_scan_kernel<NR>, dim3((dv + 31) / 32, H, R), dim3(W * 32), smem, stream, q, k, v, beta, decay, state, cu_q,
-                          slot_ids, gram, o, G, H, dk, dv));
+                          slot_ids, gram, o, G, H, dk, dv, skip_from));
   JLX_LAUNCH_CHECK("delta_scan");
   return 0;
 }
 
 // q, k: float32 [N, G, dk]; v, o: [N, H, dv]; beta, decay: [N, H]; state: float32 [slots, H, dk, dv]; gram: scratch
 // float32 [N, G, 2, DELTA_TB] on a 16-byte boundary, or null (every block then makes the products of its groups itself).
+// skip_from > 0: requests of at least so many tokens are left alone.
 JLX_API int jlx_delta_scan(const float* q, const float* k, const float* v, const float* beta, const float* decay, float* state,
                            const int* cu_q, const int* slot_ids, const int* req_of_token, float* gram, float* o, int N, int R, int G,
-                           int H, int dk, int dv, cudaStream_t stream) {
+                           int H, int dk, int dv, int skip_from, cudaStream_t stream) {
   JLX_REQUIRE(N >= 0 && R >= 0 && G > 0 && H > 0 && dk > 0 && dv > 0 && H % G == 0, "delta_scan: bad sizes N=%d R=%d G=%d H=%d dk=%d dv=%d", N,
               R, G, H, dk, dv);
   JLX_REQUIRE(dk <= 512, "delta_scan: key size %d is above the supported maximum 512", dk);
@@ -664,10 +666,10 @@ JLX_API int jlx_delta_scan(const float* q, const float* k, const float* v, const
   if (N <= R) gram = nullptr;  // single tokens: one product per block, not worth a launch
   if (gram) {
     const int warps = G < 8 ? G : 8;
-    JLX_CUDA(jlx_launch_pdl(delta_gram_kernel, dim3(N), dim3(warps * 32), 0, stream, q, k, cu_q, req_of_token, gram, G, dk));
+    JLX_CUDA(jlx_launch_pdl(delta_gram_kernel, dim3(N), dim3(warps * 32), 0, stream, q, k, cu_q, req_of_token, gram, G, dk, skip_from));
     JLX_LAUNCH_CHECK("delta_gram");
   }
-#define DELTA_ARGS q, k, v, beta, decay, state, cu_q, slot_ids, gram, o, R, G, H, dk, dv, stream
+#define DELTA_ARGS q, k, v, beta, decay, state, cu_q, slot_ids, gram, o, R, G, H, dk, dv, skip_from, stream
   const int nr = (dk + DELTA_W - 1) / DELTA_W;  // rows per warp
   if (nr <= 4) return launch_delta_scan<4>(DELTA_ARGS);
   if (nr <= 8) return launch_delta_scan<8>(DELTA_ARGS);

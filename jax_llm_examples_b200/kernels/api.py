@@ -763,11 +763,12 @@ DELTA_GROUP = 8  # tokens that delta_scan walks together (csrc/delta_rule.cu)
 
 def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, state: torch.Tensor,
                cu_q: torch.Tensor, slot_ids: torch.Tensor, o: torch.Tensor, req_of_token: torch.Tensor | None = None,
-               scratch: torch.Tensor | None = None) -> None:
+               scratch: torch.Tensor | None = None, skip_from: int = 0) -> None:
     """Over each request's tokens, in order:  S <- g S;  u = beta (v - S^T k);  S <- S + k u^T;  o = S^T q.
     q, k: float32 [N, G, dk] (head h reads key head h // (H / G)); v, o: [N, H, dv]; beta, decay: [N, H];
     state: float32 [slots, H, dk, dv].  With `req_of_token` [N] and `scratch` (float32, N * G * 2 * DELTA_GROUP elements) a
-    step that holds prompts makes the products between a group's keys and queries once per key head, ahead of the scan."""
+    step that holds prompts makes the products between a group's keys and queries once per key head, ahead of the scan.
+    ``skip_from`` > 0: requests of at least so many tokens are left to ``delta_chunk``."""
     _contig(q, k, v, beta, decay, state, o)
     N, G, dk = q.shape
     _, H, dv = v.shape
@@ -780,7 +781,35 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
         raise KernelError(f"delta_scan: the scratch holds {scratch.numel()} elements; {N * G * 2 * DELTA_GROUP} float32 are needed")
     _run("delta_rule", "jlx_delta_scan", _ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(decay), _ptr(state), _ptr(cu_q), _ptr(slot_ids),
          _ptr(req_of_token) if ahead else None, _ptr(scratch) if ahead else None, _ptr(o), c_int(N), c_int(slot_ids.numel()), c_int(G),
-         c_int(H), c_int(dk), c_int(dv), _stream())
+         c_int(H), c_int(dk), c_int(dv), c_int(skip_from), _stream())
+
+
+def delta_chunk_supported(dk: int, dv: int) -> bool:
+    """Heads that fill most of the 128 channels and columns the kernels work on, in whole 16-byte pieces."""
+    return bool(library("delta_chunk").jlx_delta_chunk_supported(c_int(dk), c_int(dv)))
+
+
+def delta_chunk_scratch(n: int, heads: int, dk: int, dv: int) -> int:
+    """float32 elements that ``delta_chunk`` needs for n chunks."""
+    return n * heads * (CHUNK_TOKENS * (dk + dv + 1) + dk * dv + 1)
+
+
+def delta_chunk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, state: torch.Tensor,
+                slot_ids: torch.Tensor, o: torch.Tensor, chunks: Chunks, scratch: torch.Tensor) -> None:
+    """:func:`delta_scan` for the requests of ``chunks`` (three launches); scratch: float32 of ``delta_chunk_scratch`` elements."""
+    global _launches
+    _contig(q, k, v, beta, decay, state, o, scratch)
+    N, G, dk = q.shape
+    _, H, dv = v.shape
+    if any(t.dtype != torch.float32 for t in (q, k, v, beta, decay, state, o, scratch)):
+        raise KernelError("delta_chunk: everything is float32")
+    if tuple(state.shape[1:]) != (H, dk, dv) or tuple(o.shape) != (N, H, dv) or tuple(k.shape) != (N, G, dk) or H % G \
+            or scratch.numel() < delta_chunk_scratch(chunks.n, H, dk, dv):
+        raise KernelError(f"delta_chunk: shapes do not fit: q {tuple(q.shape)}, v {tuple(v.shape)}, state {tuple(state.shape)}")
+    _run("delta_chunk", "jlx_delta_chunk", _ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(decay), _ptr(state), _ptr(slot_ids), _ptr(o),
+         _ptr(chunks.chunks), c_int(chunks.n), _ptr(chunks.requests), c_int(chunks.m), c_int(G), c_int(H), c_int(dk), c_int(dv), _ptr(scratch),
+         _stream())
+    _launches += 2
 
 
 # ---------------------------------- weighted q/k norm + rotate-half rotation + page write; gated attention heads

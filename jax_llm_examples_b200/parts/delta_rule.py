@@ -17,6 +17,16 @@ import torch
 from ..kernels import api as K
 from ..tracing import scope
 from .base import LayerCache, ProjectedMixer, Rows, StateNeed, StepContext, register_part
+from .recurrent import CHUNK_FROM_TOKENS, plan_scan_chunks, step_chunks
+
+
+def chunks_pay(lens, heads: int) -> bool:
+    """Whether a step's long portions go through the chunk kernels: they take about 7 ns per token and head however the tokens are
+    spread; the walk takes 6.5 ns where many chains fill the GPU, but never less than 265 ns per token of the longest.  Measured, us,
+    walk and chunks: 16 heads 384 tokens 153 and 75, 2048 tokens 538 and 259, requests of 777, 500 and 600 tokens 280 and 249; 32
+    heads 2048 tokens 550 and 419, but 777, 500 and 600 tokens 398 and 421; 16 heads 8 requests of 256 tokens 210 and 224."""
+    long = [n for n in lens if n >= CHUNK_FROM_TOKENS]
+    return bool(long) and heads * sum(long) <= 48 * max(long)
 
 
 class GatedDeltaRule(ProjectedMixer):
@@ -31,7 +41,7 @@ class GatedDeltaRule(ProjectedMixer):
     State per request: the convolution's last taps - 1 inputs, float32 [taps - 1, 2 G dk + H dv] (if taps > 1), and S,
     float32 [H, dk, dv]."""
 
-    kernel_libraries = ("delta_rule", "decay_scan", "gemm_simt")
+    kernel_libraries = ("delta_rule", "delta_chunk", "decay_scan", "gemm_simt")
     kernel_libraries_bf16 = ("gemm_stream",)
 
     def __init__(self, w_in: torch.Tensor, conv_weight: torch.Tensor, rate_log: torch.Tensor, a_bias: torch.Tensor,
@@ -57,6 +67,9 @@ class GatedDeltaRule(ProjectedMixer):
     def state_needs(self):
         conv = (StateNeed((self.taps - 1, self.channels), torch.float32),) if self.taps > 1 else ()
         return conv + (StateNeed((self.heads, self.dim, self.vdim), torch.float32),)
+
+    def step_planners(self):
+        return (plan_scan_chunks,)
 
     def core(self, ctx: StepContext, h, proj: Rows, col: int, cache: LayerCache, out: torch.Tensor, mult: float) -> None:
         H, G, dk, dv, C = self.heads, self.key_heads, self.dim, self.vdim, self.channels
@@ -84,7 +97,14 @@ class GatedDeltaRule(ProjectedMixer):
             K.conv_unit_prep(K.rows_view(proj.data, proj.splits, col), C + H * dv, C + H * dv + H, self.conv_weight, conv_state,
                              self.rate_log, self.a_bias, ctx.cu_q, ctx.q_start, ctx.slot_ids, ctx.req_of_token, ctx.positions,
                              q, k, v, beta, decay, self.activation, self.unit_eps, self.q_scale)
-            K.delta_scan(q, k, v, beta, decay, S, ctx.cu_q, ctx.slot_ids, o, ctx.req_of_token, products)
+            chunks = step_chunks(ctx) if K.delta_chunk_supported(dk, dv) and chunks_pay(ctx.host_q_lens, H) else None
+            if chunks is None or chunks.others:
+                K.delta_scan(q, k, v, beta, decay, S, ctx.cu_q, ctx.slot_ids, o, ctx.req_of_token, products, 0 if chunks is None else chunks.long_from)
+            if chunks is not None:
+                need = K.delta_chunk_scratch(chunks.n, H, dk, dv)
+                scratch = ctx.workspace.get("delta_chunk", need, torch.float32) if ctx.workspace is not None else \
+                    torch.empty(need, dtype=torch.float32, device=dev)
+                K.delta_chunk(q, k, v, beta, decay, S, ctx.slot_ids, o, chunks, scratch)
             K.head_norm_gate(o, self.norm_weight, False, K.rows_view(proj.data, proj.splits, gate_col), self.eps, mult, out)
 
 

@@ -83,17 +83,24 @@ def plan_scan_chunks(shape: StepShape) -> dict:
     return {"scan_chunks": np.array(chunks, dtype=np.int32).reshape(-1, 3), "scan_chunk_requests": np.array(requests, dtype=np.int32).reshape(-1, 3)}
 
 
+def step_chunks(ctx: StepContext) -> "K.Chunks | None":
+    """The step's long portions in chunks, if it has any (and was planned with ``plan_scan_chunks``)."""
+    chunks = ctx.arrays.get("scan_chunks")
+    if chunks is None:
+        return None
+    requests = ctx.arrays["scan_chunk_requests"]
+    m = requests.numel() // 3
+    return K.Chunks(chunks, requests, chunks.numel() // 3, m, CHUNK_FROM_TOKENS, m < ctx.n_requests)
+
+
 def scan_chunks(ctx: StepContext, heads: int, dk: int, dv: int) -> "tuple[K.Chunks | None, torch.Tensor | None]":
     """The step's chunks and the scratch of their states, if it has long portions of heads that the chunk kernels take."""
-    chunks = ctx.arrays.get("scan_chunks")
+    chunks = step_chunks(ctx)
     if chunks is None or not K.chunk_scan_supported(dk, dv):
         return None, None
-    requests = ctx.arrays["scan_chunk_requests"]
-    n, m = chunks.numel() // 3, requests.numel() // 3
-    need = K.chunk_scan_scratch(n, heads, dk, dv)
-    scratch = ctx.workspace.get("chunk_scan", need, torch.float32) if ctx.workspace is not None else \
-        torch.empty(need, dtype=torch.float32, device=chunks.device)
-    return K.Chunks(chunks, requests, n, m, CHUNK_FROM_TOKENS, m < ctx.n_requests), scratch
+    need = K.chunk_scan_scratch(chunks.n, heads, dk, dv)
+    return chunks, ctx.workspace.get("chunk_scan", need, torch.float32) if ctx.workspace is not None else \
+        torch.empty(need, dtype=torch.float32, device=chunks.chunks.device)
 
 
 class HGRN2(InputConvMixer):

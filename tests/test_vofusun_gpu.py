@@ -61,6 +61,46 @@ def test_delta_scan_sizes_and_a_batch_of_unequal_requests(dk, dv, Hh, G, ahead):
         at += n
 
 
+@pytest.mark.parametrize("dk, dv, Hh, G", [(128, 128, 4, 2), (68, 124, 2, 1), (100, 72, 3, 3), (128, 96, 40, 8)])
+def test_delta_rule_by_chunks_against_the_walk_and_the_plain_recurrence(dk, dv, Hh, G):
+    """Portions that end inside, at and behind a chunk's and a piece's edge, heads smaller than the kernels' 128, both widths of
+    the chain's slices, keys that are written again, decays from one to zero, full and vanishing steps, states to start from in
+    slots of another order: float64 token by token, and the walk over the same requests.  Sums of at most 192 products in
+    float32 and a solution whose rows build on one another: 5e-6 of the largest value."""
+    from jax_llm_examples_b200.kernels import api as K
+
+    torch.manual_seed(dk)
+    lens, slots = [1, 64, 130, 15, 197, 65], [4, 0, 6, 2, 1, 3]
+    N = sum(lens)
+    q, k = torch.randn(N, G, dk, device=DEV) * dk ** -0.5, torch.randn(N, G, dk, device=DEV)
+    k[1::3] = 0.9 * k[0::3][:k[1::3].shape[0]] + 0.1 * k[1::3]
+    k = torch.nn.functional.normalize(k, dim=-1)
+    v, beta, decay = torch.randn(N, Hh, dv, device=DEV), torch.rand(N, Hh, device=DEV), torch.rand(N, Hh, device=DEV) * 0.5 + 0.5
+    beta[::5], beta[1::7] = 1.0, 0.0
+    decay[::4], decay[3::31], decay[5::31] = 1.0, 0.0, 1e-32
+    state = torch.randn(7, Hh, dk, dv, device=DEV) * 0.3
+    before, walked = state.clone(), state.clone()
+    o, o_walk = torch.full((N, Hh, dv), float("nan"), device=DEV), torch.empty(N, Hh, dv, device=DEV)
+    chunks, requests, at = [], [], 0
+    for r, n in enumerate(lens):
+        requests.append((r, len(chunks), -(-n // 64)))
+        chunks += [(r, at + c, at + min(n, c + 64)) for c in range(0, n, 64)]
+        at += n
+    ch = K.Chunks(_i32(chunks), _i32(requests), len(chunks), len(requests), 1, False)
+    K.delta_chunk(q, k, v, beta, decay, state, _i32(slots), o, ch, torch.empty(K.delta_chunk_scratch(ch.n, Hh, dk, dv), device=DEV))
+    K.delta_scan(q, k, v, beta, decay, walked, _i32([sum(lens[:i]) for i in range(len(lens) + 1)]), _i32(slots), o_walk)
+    c = lambda t: t.double().cpu()  # noqa: E731
+    at = 0
+    for r, n in enumerate(lens):
+        sl = slice(at, at + n)
+        want, S = plain.delta_recurrence(c(q[sl]), c(k[sl]), c(v[sl]), c(beta[sl]), c(decay[sl]), c(before[slots[r]]))
+        for name, got, got_state in (("chunks", o, state), ("walk", o_walk, walked)):
+            _close(got[sl], want, 5e-6, f"{name}: request {r}")
+            _close(got_state[slots[r]], S, 5e-6, f"{name}: state of request {r}")
+        at += n
+    assert torch.equal(state[5], before[5])
+
+
 def test_delta_scan_keeps_a_far_token_and_corrects_a_key_that_is_written_again():
     """Made so that a fault shows.  Head 1 never decays.  Along key direction e0 it is written ONCE with a full step, at
     token 3; 700 tokens later a query along e0 must read that value exactly, through portions of many sizes and a state
