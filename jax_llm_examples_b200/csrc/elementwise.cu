@@ -679,6 +679,33 @@ __global__ void silu_mul_bf16x8_kernel(const bf16* __restrict__ gu, bf16* __rest
   }
 }
 
+// float32 rows on 16-byte boundaries: four outputs per thread and access, a row cut over several blocks so that few rows fill
+// the GPU too.  The partials of an output are added in the general kernel's order.  1024 rows of 2 x 8192 (100 MB): 30 us (65 by
+// single entries); 37 rows 7 (32).
+template <typename TO>
+__global__ void __launch_bounds__(256)
+silu_mul_f32x4_kernel(const float* __restrict__ gu, int splits, long long split_stride, TO* __restrict__ out, int F, int interleaved, GluForm form) {
+  JLX_TL(TL_SILU_MUL);
+  const size_t i = blockIdx.x;
+  const float* g = gu + i * 2 * F;
+  for (int f0 = (blockIdx.y * 256 + threadIdx.x) * 4; f0 < F; f0 += gridDim.y * 256 * 4) {
+    const int gi = interleaved ? ((f0 >> 4) << 5) + (f0 & 15) : f0;
+    const int ui = interleaved ? gi + 16 : F + f0;
+    float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int z = 0; z < splits; ++z) {
+      const float4 x = *reinterpret_cast<const float4*>(g + (size_t)z * split_stride + gi), y = *reinterpret_cast<const float4*>(g + (size_t)z * split_stride + ui);
+      a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w;
+      b[0] += y.x; b[1] += y.y; b[2] += y.z; b[3] += y.w;
+    }
+    alignas(16) TO o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = from_f32<TO>(glu_act(a[j], b[j], form));
+    if (sizeof(TO) == 4) *reinterpret_cast<uint4*>(out + i * F + f0) = *reinterpret_cast<const uint4*>(o);
+    else *reinterpret_cast<uint2*>(out + i * F + f0) = *reinterpret_cast<const uint2*>(o);
+  }
+}
+
 JLX_API int jlx_silu_mul(const void* gu, int in_dtype, int splits, long long split_stride, void* out, int out_dtype,
                          int rows, int F, int interleaved, float alpha, float limit, float shift, cudaStream_t stream) {
   JLX_REQUIRE(rows >= 0 && F > 0 && splits >= 1, "silu_mul: bad sizes rows=%d F=%d splits=%d", rows, F, splits);
@@ -689,6 +716,14 @@ JLX_API int jlx_silu_mul(const void* gu, int in_dtype, int splits, long long spl
   if (in_dtype == JLX_BF16 && out_dtype == JLX_BF16 && splits == 1 && F % 16 == 0 && ((uintptr_t)gu & 15) == 0 &&
       ((uintptr_t)out & 15) == 0) {
     silu_mul_bf16x8_kernel<<<rows, 256, 0, stream>>>((const bf16*)gu, (bf16*)out, F, interleaved, form);
+    JLX_LAUNCH_CHECK("silu_mul");
+    return 0;
+  }
+  if (in_dtype == JLX_F32 && F % 4 == 0 && split_stride % 4 == 0 && (((uintptr_t)gu | (uintptr_t)out) & 15) == 0) {
+    const int pieces = (F + 1023) / 1024, ysplit = rows >= 2048 ? 1 : (pieces < 2048 / rows + 1 ? pieces : 2048 / rows + 1);
+    JLX_DISPATCH_DTYPE(out_dtype, TO, {
+      silu_mul_f32x4_kernel<TO><<<dim3(rows, ysplit), 256, 0, stream>>>((const float*)gu, splits, split_stride, (TO*)out, F, interleaved, form);
+    });
     JLX_LAUNCH_CHECK("silu_mul");
     return 0;
   }

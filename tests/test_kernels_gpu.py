@@ -61,6 +61,23 @@ def test_add_rmsnorm(out_dtype, tol, N, D, eps):
     assert torch.equal(xc2, x)  # gathered rows are not written back
 
 
+@pytest.mark.parametrize("rows", [1, 37, 2100])
+@pytest.mark.parametrize("F, interleaved", [(4, False), (48, True), (1020, False), (1024, True), (1028, False), (4096, True)])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_silu_mul_of_float32_rows_in_pieces_is_the_general_kernel(rows, F, interleaved, splits):
+    """Rows on 16-byte boundaries go four entries at a time, a row over several blocks; the same rows one entry further, and a
+    width that is no multiple of four, go entry by entry: the same bits, in both output types."""
+    if rows * F * splits > 3e7:
+        pytest.skip("more of the same")
+    for dtype in (torch.float32, torch.bfloat16):
+        gu = torch.randn(splits, rows, 2 * F, device=DEV)
+        moved = torch.empty(gu.numel() + 1, device=DEV)[1:].view_as(gu).copy_(gu)
+        out, want = torch.empty(rows, F, device=DEV, dtype=dtype), torch.empty(rows, F, device=DEV, dtype=dtype)
+        K().silu_mul(gu, out, splits=splits, interleaved=interleaved)
+        K().silu_mul(moved, want, splits=splits, interleaved=interleaved)
+        assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("dtype, tol", [(torch.float32, 1e-6), (torch.bfloat16, 1e-2)])
 def test_silu_mul(dtype, tol):
     gu = torch.randn(9, 2 * 200, device=DEV).to(dtype)
