@@ -63,7 +63,7 @@ struct PrepParams {
   int N, R, G, H, dk, dv, taps, act;
   float unit_eps, q_scale;
   int vec;                  // 16-byte accesses are possible (prep_group4)
-  int pad_;
+  int wide_taps;            // the convolution weights start on a 16-byte boundary
 };
 
 // The convolved and activated value of channel c at token row n.  `first` = the row of the request's first token in
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(256) conv_unit_prep_kernel(const PrepParams P)
 // tokens, so that a channel's weights are read once for them and every row once and not once per tap.  Blocks [0, tiles):
 // tokens whose taps lie in this step, by slices of eight groups; behind them a block per request and slice for its first
 // tokens and its state (a channel's state is read and written by one lane).  The same operations per value.
-// 2048 tokens, 16 heads of 128, 8 key heads, four taps: 49 us (120 by tokens).
+// 2048 tokens, 16 heads of 128, 8 key heads, four taps: 42 us (49 with a token looked up at its turn, 120 by tokens).
 #define PREP_TILE 8
 template <int TAPS>
 __global__ void __launch_bounds__(256) conv_unit_prep_tile_kernel(const PrepParams P, int tiles) {
@@ -251,18 +251,26 @@ __global__ void __launch_bounds__(256) conv_unit_prep_tile_kernel(const PrepPara
 #pragma unroll
   for (int j = 0; j < TAPS; ++j) {
     const float* w = P.conv_w + (size_t)c * TAPS + j;
-    tap[j] = in ? make_float4(w[0], w[TAPS], w[2 * TAPS], w[3 * TAPS]) : zero;
+    tap[j] = in && !(TAPS == 4 && P.wide_taps) ? make_float4(w[0], w[TAPS], w[2 * TAPS], w[3 * TAPS]) : zero;
+  }
+  if (TAPS == 4 && P.wide_taps && in) {  // four taps on 16-byte boundaries: a channel's weights in one access
+    const float4* w = reinterpret_cast<const float4*>(P.conv_w) + c;
+    const float4 a = w[0], b = w[1], d = w[2], e = w[3];
+    tap[0] = make_float4(a.x, b.x, d.x, e.x);
+    tap[1 % TAPS] = make_float4(a.y, b.y, d.y, e.y);
+    tap[2 % TAPS] = make_float4(a.z, b.z, d.z, e.z);
+    tap[3 % TAPS] = make_float4(a.w, b.w, d.w, e.w);
   }
   pdl_wait();
   const bool tile = (int)blockIdx.x < tiles;
   const int r0 = blockIdx.x - tiles;
   const int n0 = tile ? blockIdx.x * PREP_TILE : P.cu_q[r0], qlen = tile ? 0 : P.cu_q[r0 + 1] - n0;
-  // whether token n0 + i is this block's: its taps lie in this step, or it is one of its request's first
-  auto mine = [&](int i) {
-    if (!tile) return i < TAPS - 1 && i < qlen;
-    const int n = n0 + i;
-    return i < PREP_TILE && n < P.N && P.positions[n] - P.q_start[P.req_of_token[n]] >= TAPS - 1;
-  };
+  // bit i: token n0 + i is this block's: its taps lie in this step, or it is one of its request's first.  Lane i looks token i
+  // up: one chain of loads for all of them
+  bool mine_i = lane < TAPS - 1 && lane < qlen;
+  if (tile && lane < PREP_TILE && n0 + lane < P.N) mine_i = P.positions[n0 + lane] - P.q_start[P.req_of_token[n0 + lane]] >= TAPS - 1;
+  const unsigned mask = __ballot_sync(0xffffffffu, mine_i);
+  auto mine = [&](int i) { return (mask >> i & 1) != 0; };
   if (blockIdx.y == 0)
     for (int idx = threadIdx.x; idx < PREP_TILE * P.H; idx += 256) {
       const int i = idx / P.H, h = idx % P.H;
@@ -352,7 +360,7 @@ JLX_API int jlx_conv_unit_prep(const RowsView* proj, int b_col, int a_col, const
   const auto al16 = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
   P.vec = dk % 4 == 0 && dv % 4 == 0 && dk <= 256 && dv <= 256 && proj->ld % 4 == 0 && (proj->splits == 1 || proj->split_stride % 4 == 0) &&
           al16(proj->p) && al16(qo) && al16(ko) && al16(vo) && (!conv_state || al16(conv_state));
-  P.pad_ = 0;
+  P.wide_taps = al16(conv_w);
   const int groups = 2 * G + H;
   if (P.vec && taps >= 2 && taps <= 4 && dk <= 128 && dv <= 128 && groups <= 8 * 65535) {
     const int tiles = (N + PREP_TILE - 1) / PREP_TILE;
