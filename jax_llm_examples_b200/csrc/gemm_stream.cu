@@ -228,6 +228,19 @@ __device__ __forceinline__ void stream_epilogue(const StreamArgs& args, int warp
   }
 }
 
+// The blocks of a group of several token tiles in another order than the grid's: all token tiles of one weight tile, then the
+// next weight tile, so that the group's weights (more than L2 holds) come from memory once and not once per token tile.  x:
+// the weight tile of `xs`; row_lo: the first row of the token tile; both are replaced.  16 groups of 512 rows, 16384 x 5120:
+// 1040 us (1085); of 100 to 924 rows 1200 (1271); a prompt of 2048 tokens over 4 experts 2.80 ms (2.84).
+template <int BT>
+__device__ __forceinline__ void weight_tile_first(int& x, int xs, int group_lo, int& row_lo, int row_hi) {
+  const int tiles = (row_hi - group_lo + BT - 1) / BT;
+  if (tiles < 2) return;
+  const int place = (row_lo - group_lo) / BT * xs + x;
+  x = place / tiles;
+  row_lo = group_lo + (place - x * tiles) * BT;
+}
+
 // WT: weight tiles of 128 rows per block.  With many token rows per group the token tile is the larger part of
 // a stage; two weight tiles (two accumulators in tensor memory) per token tile halve its traffic.
 // SW, SA: stages of the weight ring and of the token ring.  Weights come from HBM and need many bytes in
@@ -259,7 +272,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
   // ---- which tile.  The group offsets are written by an earlier kernel of the stream: wait for it first, unless
   // they are known to be settled (then they are read past L1, which may hold lines of an earlier step).
-  int row_lo, row_hi, group = 0;
+  int row_lo, row_hi, group = 0, group_lo = 0, x = blockIdx.x;
   const bool settled = args.offsets && args.offsets_settled;
   if (args.offsets) {
     if (!settled) {
@@ -271,16 +284,18 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       if (t >= __ldcg(args.n_tiles)) return;
       group = __ldcg(args.tile_list + 2 * t);
       row_lo = __ldcg(args.tile_list + 2 * t + 1);
+      group_lo = __ldcg(args.offsets + group);
       row_hi = __ldcg(args.offsets + group + 1);
       found = 1;
     }
     for (int e = 0; !found && e < args.E; ++e) {
       const int lo = __ldcg(args.offsets + e), hi = __ldcg(args.offsets + e + 1);
       const int tiles = (hi - lo + BT - 1) / BT;
-      if (t < tiles) { row_lo = lo + t * BT; row_hi = hi; group = e; found = 1; break; }
+      if (t < tiles) { row_lo = lo + t * BT; group_lo = lo; row_hi = hi; group = e; found = 1; break; }
       t -= tiles;
     }
     if (!found) return;
+    weight_tile_first<BT>(x, gridDim.x, group_lo, row_lo, row_hi);
   } else if (args.uniform) {
     const int per_group = (args.uniform + BT - 1) / BT;
     group = blockIdx.y / per_group;
@@ -291,7 +306,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     row_hi = args.rows;
     if (row_lo >= row_hi) return;
   }
-  const int n0 = blockIdx.x * (WN * WT);
+  const int n0 = x * (WN * WT);
   const int k_begin = blockIdx.z * args.k_per_split;
   const int k_end = min(args.K, k_begin + args.k_per_split);
   const int k_iters = (k_end - k_begin + BK - 1) / BK;
@@ -420,7 +435,7 @@ gemm_stream_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
   }
 
   // ---- which tile (both blocks of a pair have the same blockIdx.y and decide alike)
-  int row_lo, row_hi, group = 0;
+  int row_lo, row_hi, group = 0, group_lo = 0, x = blockIdx.x >> 1;
   if (args.offsets) {
     pdl_wait();
     pdl_launch_dependents();
@@ -429,16 +444,18 @@ gemm_stream_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
       if (t >= args.n_tiles[0]) return;
       group = args.tile_list[2 * t];
       row_lo = args.tile_list[2 * t + 1];
+      group_lo = args.offsets[group];
       row_hi = args.offsets[group + 1];
       found = 1;
     }
     for (int e = 0; !found && e < args.E; ++e) {
       const int lo = args.offsets[e], hi = args.offsets[e + 1];
       const int tiles = (hi - lo + BT - 1) / BT;
-      if (t < tiles) { row_lo = lo + t * BT; row_hi = hi; group = e; found = 1; break; }
+      if (t < tiles) { row_lo = lo + t * BT; group_lo = lo; row_hi = hi; group = e; found = 1; break; }
       t -= tiles;
     }
     if (!found) return;
+    weight_tile_first<BT>(x, gridDim.x >> 1, group_lo, row_lo, row_hi);
   } else if (args.uniform) {
     const int per_group = (args.uniform + BT - 1) / BT;
     group = blockIdx.y / per_group;
@@ -449,7 +466,7 @@ gemm_stream_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     row_hi = args.rows;
     if (row_lo >= row_hi) return;
   }
-  const int n0 = blockIdx.x * WN;  // this block's weight rows
+  const int n0 = (2 * x + (int)rank) * WN;  // this block's weight rows
   const int k_begin = blockIdx.z * args.k_per_split;
   const int k_end = min(args.K, k_begin + args.k_per_split);
   const int k_iters = (k_end - k_begin + BK - 1) / BK;

@@ -5,6 +5,7 @@ import math
 import random
 
 import pytest
+import numpy as np
 import torch
 
 pytestmark = pytest.mark.gpu
@@ -987,3 +988,28 @@ def test_add_rmsnorm_adds_a_sum_of_terms_with_gathered_rows(out_dtype, tol, N, D
     scores = want @ w_router.T
     chosen = torch.gather(scores, 1, ti.long())
     assert float((scores.max(-1, keepdim=True).values - chosen).max()) < 1e-3 * float(scores.abs().max())
+
+
+@pytest.mark.parametrize("N", [384, 512])  # one block per weight tile, and a pair where the token tile is wide
+@pytest.mark.parametrize("hint", [16, 100])
+@pytest.mark.parametrize("listed", [False, True])
+def test_grouped_product_whose_groups_have_several_token_tiles(N, hint, listed):
+    """Groups of no rows, one row, a tile's edge and up to sixteen token tiles: their blocks go through the weight tiles first, and
+    every row of every group comes out once.  32-bit sums of 320 products, rounded to bfloat16."""
+    api = K()
+    sizes, Kd = [0, 5, 16, 17, 250, 1, 33, 101, 100], 320
+    off = torch.tensor([0] + list(np.cumsum(sizes)), device=DEV, dtype=torch.int32)
+    rows, E, st = sum(sizes), len(sizes), status()
+    a, w = torch.randn(rows, Kd, device=DEV).bfloat16(), torch.randn(E, N, Kd, device=DEV).bfloat16()
+    tiles = None
+    if listed:
+        bt = api.gemm_stream_token_tile(hint)
+        found = [(e, int(off[e]) + r) for e, n in enumerate(sizes) for r in range(0, n, bt)]
+        tiles = (torch.tensor(found, device=DEV, dtype=torch.int32).reshape(-1), torch.tensor([len(found)], device=DEV, dtype=torch.int32))
+    out = torch.full((rows, N), float("nan"), device=DEV)
+    api.gemm_stream(a, w, out, st, offsets=off, rows_hint=hint, tiles=tiles)
+    assert int(st) == 0
+    for e in range(E):
+        lo, hi = int(off[e]), int(off[e + 1])
+        if hi > lo:
+            close(out[lo:hi], a[lo:hi].double() @ w[e].double().T, 1e-5)
