@@ -184,6 +184,10 @@ class Workspace:
         return t[:numel]
 
     def get(self, name: str, numel: int, dtype: torch.dtype) -> torch.Tensor:
+        """Scratch of this name for work on the current stream: what runs on the second stream has buffers of its own, so
+        that two parts that run side by side never share one."""
+        if self._side is not None and torch.cuda.current_stream(self.device) == self._side:
+            name = "side:" + name
         t = self._bufs.get(name)
         if t is None or t.numel() < numel or t.dtype != dtype:
             if t is not None:

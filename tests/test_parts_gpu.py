@@ -485,3 +485,16 @@ def test_a_state_mixer_decodes_through_replayed_graphs():
         run("host", True)
     rows, eng = run("opts_out", True)
     assert eng.graph_replays == 0 and torch.equal(rows, plain_rows)
+
+
+def test_scratch_of_the_second_stream_is_kept_apart():
+    """Two parts that run side by side (the workspace's second stream beside the step's own) ask for scratch of one name."""
+    from jax_llm_examples_b200.parts.base import Workspace
+
+    ws = Workspace(torch.device("cuda", torch.cuda.current_device()))
+    before = ws.get("scratch", 64, torch.float32)
+    with torch.cuda.stream(ws.side_stream()):
+        beside = ws.get("scratch", 64, torch.float32)
+        assert ws.get("scratch", 32, torch.float32).data_ptr() == beside.data_ptr()
+    assert beside.data_ptr() != before.data_ptr()
+    assert ws.get("scratch", 64, torch.float32).data_ptr() == before.data_ptr()
