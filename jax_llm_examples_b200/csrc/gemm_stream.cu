@@ -284,7 +284,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       if (t >= __ldcg(args.n_tiles)) return;
       group = __ldcg(args.tile_list + 2 * t);
       row_lo = __ldcg(args.tile_list + 2 * t + 1);
-      group_lo = __ldcg(args.offsets + group);
+      if (BT > 64) group_lo = __ldcg(args.offsets + group);
       row_hi = __ldcg(args.offsets + group + 1);
       found = 1;
     }
@@ -295,7 +295,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       t -= tiles;
     }
     if (!found) return;
-    weight_tile_first<BT>(x, gridDim.x, group_lo, row_lo, row_hi);
+    if (BT > 64) weight_tile_first<BT>(x, gridDim.x, group_lo, row_lo, row_hi);  // (narrow tiles: decode steps, one tile a group)
   } else if (args.uniform) {
     const int per_group = (args.uniform + BT - 1) / BT;
     group = blockIdx.y / per_group;
