@@ -97,7 +97,9 @@ class GatedDeltaRule(ProjectedMixer):
             K.conv_unit_prep(K.rows_view(proj.data, proj.splits, col), C + H * dv, C + H * dv + H, self.conv_weight, conv_state,
                              self.rate_log, self.a_bias, ctx.cu_q, ctx.q_start, ctx.slot_ids, ctx.req_of_token, ctx.positions,
                              q, k, v, beta, decay, self.activation, self.unit_eps, self.q_scale)
-            chunks = step_chunks(ctx) if K.delta_chunk_supported(dk, dv) and chunks_pay(ctx.host_q_lens, H) else None
+            chunks = step_chunks(ctx) if K.delta_chunk_supported(dk, dv) else None
+            if chunks is not None and not chunks_pay(ctx.host_q_lens, H):  # (a step with chunks is never captured in a graph)
+                chunks = None
             if chunks is None or chunks.others:
                 K.delta_scan(q, k, v, beta, decay, S, ctx.cu_q, ctx.slot_ids, o, ctx.req_of_token, products, 0 if chunks is None else chunks.long_from)
             if chunks is not None:

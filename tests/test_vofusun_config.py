@@ -219,3 +219,41 @@ def test_plain_loop_adds_the_embedding_before_every_pass_but_the_first(tmp_path)
     assert after.shape[0] == len(factor)
     for run, f in enumerate(factor):
         assert torch.allclose(after[run], f * x0)
+
+
+def test_a_delta_layer_of_wide_heads_reads_no_host_copies_in_a_decode_step(monkeypatch):
+    """While a step of single tokens is captured in a graph, the step's host copies refuse to be read: the choice between the
+    recurrence's kernels must not need them there.  A step with a long portion (never captured) chooses by its lengths."""
+    from jax_llm_examples_b200.engine.engine import _NotInAGraph
+    from jax_llm_examples_b200.kernels import api as K
+    from jax_llm_examples_b200.parts import GatedDeltaRule, LayerCache, Rows, Runtime, StepContext
+    from jax_llm_examples_b200.parts.recurrent import plan_scan_chunks
+
+    ran = []
+    monkeypatch.setattr(K, "rows_view", lambda *a, **k: None)
+    monkeypatch.setattr(K, "delta_chunk_supported", lambda dk, dv: True)
+    for name in ("conv_unit_prep", "delta_scan", "delta_chunk", "head_norm_gate"):
+        monkeypatch.setattr(K, name, lambda *a, name=name, **k: ran.append(name))
+    H, G, dk, D, taps = 2, 1, 128, 8, 2
+    C = 2 * G * dk + H * dk
+    z = lambda *s: torch.zeros(*s)  # noqa: E731
+    mixer = GatedDeltaRule(z(C + H * dk + 2 * H, D), z(C, taps), z(H), z(H), z(dk), z(D, H * dk), H, G, dk, dk, 1e-5)
+    cache = LayerCache(None, None, True, None, (z(4, taps - 1, C), z(4, H, dk, dk)))
+
+    def run(lens, captured):
+        i32 = lambda v: torch.tensor(v, dtype=torch.int32)  # noqa: E731
+        n, R = sum(lens), len(lens)
+        host = _NotInAGraph() if captured else lens
+        ctx = StepContext(Runtime(torch.bfloat16, torch.device("cpu")), n, R, i32([0] * n), i32([0] * n), i32([0] * n), i32([0] * (R + 1)), i32([0] * R),
+                          i32(lens), i32(list(range(R))), i32([]), 0, i32([0]), host_q_lens=host, host_q_start=_NotInAGraph() if captured else [0] * R,
+                          max_q_len=max(lens))
+        if not captured:
+            ctx.plan_with((plan_scan_chunks,), 16)
+        ran.clear()
+        mixer.core(ctx, None, Rows(z(n, C + H * dk + 2 * H)), 0, cache, z(n, H * dk), 1.0)
+        return tuple(ran)
+
+    assert run([1, 1, 1], True) == ("conv_unit_prep", "delta_scan", "head_norm_gate")
+    assert run([2048], False) == ("conv_unit_prep", "delta_chunk", "head_norm_gate")
+    assert run([2048, 1], False) == ("conv_unit_prep", "delta_scan", "delta_chunk", "head_norm_gate")
+    assert run([383, 1], False) == ("conv_unit_prep", "delta_scan", "head_norm_gate")

@@ -581,7 +581,7 @@ def test_logits_do_not_depend_on_the_cut_or_on_the_batch(folders, name):
         assert worst < 2e-6, f"{name}: logits moved by {worst:.2e} with the cut"
 
 
-@pytest.mark.parametrize("name", ["small", "wide", "recurrent"])
+@pytest.mark.parametrize("name", ["small", "wide", "recurrent", "heads"])
 def test_decoding_through_replayed_graphs_equals_decoding_without(folders, name):
     """bfloat16: decode-only steps are captured in CUDA graphs and replayed; states and pages are found by slot and table
     on the device, so the replayed steps must give what the same steps give launched one kernel at a time."""

@@ -77,6 +77,11 @@ CONFIGS = {
         "layers": [delta(2, 1, 16, 16, 4, dense(48)), delta(4, 4, 24, 4, 7, dense(16))],
         "loop": {"start": 1, "stop": 2, "times": 2},
     },
+    # delta heads of the presets' size, and of a smaller one that the kernels for long portions take too
+    "heads": {
+        "architecture": "Vofusun", "vocab": 40, "width": 64, "embedding": {"scale": 2.0}, "norm": {"eps": 1e-6},
+        "layers": [delta(4, 2, 128, 128, 4, dense(48)), attention(2, 1, 16, 16, 24, 0.2), delta(2, 1, 68, 100, 3, dense(32))],
+    },
 }
 
 
