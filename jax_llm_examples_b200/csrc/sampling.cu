@@ -399,6 +399,7 @@ sample_pick_kernel(const float* __restrict__ logits, int V, long long ld, int ch
   const int l2 = (int)min((long long)V, (long long)t * span), h2 = min(V, l2 + span);
   __syncthreads();
   if (tid == 0) pick = V;
+  __syncthreads();  // (a span behind the row's end is empty: the loop has no barrier then)
   for (int i0 = l2; i0 < h2; i0 += SAMPLE_SPANS) {
     const int i = i0 + tid, n = min(SAMPLE_SPANS, h2 - i0);
     const float v = i < h2 ? row[i] : 0.f;

@@ -557,6 +557,34 @@ def test_sampling_at_the_edges_of_its_chunks(rows, vocab):
             assert got in refs, (m, got, refs)
 
 
+def test_a_draw_behind_the_last_span_takes_the_last_token_with_weight():
+    """The whole vocabulary at a size whose last spans lie behind the row.  One row's sums are not numbers (an infinite logit);
+    another's prefix, added span by span, stays at 1 while the total of the same spans, added as a tree, is 1 + 2.9e-5: a draw
+    above the ratio falls into no span.  The first gives the infinite logit's token, the second the last token with weight,
+    in every call and beside rows that draw as usual."""
+    from tests.plain import llama4_plain as plain
+
+    vocab, rows, span = 202048, 12, 198
+    u_of = lambda c: plain.uniform_from_bits(plain.philox4x32((c, 0, 1, 0), (5, 0))[0])  # noqa: E731
+    counter = next(c for c in range(10 ** 6) if u_of(c) > 0.99998)
+    logits = torch.randn(rows, vocab, device=DEV)
+    logits[0::3, 100123] = float("inf")
+    logits[1::3] = float("-inf")
+    logits[1::3, 0] = 0.0
+    logits[1::3, span + 7::span] = -25 * math.log(2.0)  # a quarter of the last bit of 1
+    last = int((logits[1] > float("-inf")).nonzero().max())
+    temps, ks = torch.ones(rows, device=DEV), torch.zeros(rows, device=DEV, dtype=torch.int32)
+    streams, counters = torch.ones(rows, device=DEV, dtype=torch.int64), torch.full((rows,), counter, device=DEV, dtype=torch.int64)
+    first = None
+    for _ in range(20):
+        out = torch.empty(rows, device=DEV, dtype=torch.int32)
+        K().sample(logits, out, temps, ks, streams, counters, seed=5)
+        got = out.tolist()
+        assert got[0::3] == [100123] * 4 and got[1::3] == [last] * 4
+        first = first or got
+        assert got == first
+
+
 @pytest.mark.parametrize("Hq, Hkv, dh, page, chunk, window, temp", [
     (40, 8, 128, 64, 0, 0, False), (6, 2, 64, 16, 512, 0, False), (16, 1, 128, 32, 0, 300, True), (4, 4, 64, 128, 0, 0, True),
     (10, 2, 128, 16, 1024, 0, False)])
