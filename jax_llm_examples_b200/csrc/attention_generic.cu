@@ -19,6 +19,8 @@
 #include "attention_maps.cuh"
 #include "common.cuh"
 
+#include <type_traits>
+
 #define ATT_TILE 32
 #define ATT_MAX_WARPS 8
 #define ATT_MAX_D32 16  // head size up to 512
@@ -164,7 +166,9 @@ JLX_API int jlx_attention_generic(const void* q, const void* pages, int dtype, c
 // The same attention over float32 pages for head sizes that are multiples of 4 up to 128, for work items (first token row,
 // count) of one request each: up to 16 tokens of a prompt portion, or one decoded token.  A block serves an item and a KV
 // head: 16 RI rows, a row being a (token, query head of the group) pair, share each key tile; more rows take more blocks.
-// Scores, softmax and sums as above (32-bit FMAs, two per instruction; every row's maximum and sum over its own keys).
+// Scores, softmax and sums as above (32-bit FMAs, two per instruction; every row's maximum and sum over its own keys).  A key
+// of the tile that a row does not see has the weight -1, and its value is left out of the row's sum whatever it is (zero
+// times an infinite value would not be zero); only the tiles at the rows' edges look for such weights.
 // A thread has the rows ty + 16 i and of a key tile the keys tx + 16 j, then 8 columns of the output.  Keys and values come
 // by asynchronous copies, the values while the scores are made; the weights lie where the keys were.
 // A row's keys fall into ranges of 256 positions; each has a maximum, a sum and an output of its own, and they are merged in
@@ -256,7 +260,7 @@ __device__ __forceinline__ float a32_weights(float m_first, float m_second, floa
 }
 
 template <int DH, int RI>
-__global__ void __launch_bounds__(256) attention_f32_kernel(const __grid_constant__ A32Params P) {
+__global__ void __launch_bounds__(256, RI == 1 ? 3 : 1) attention_f32_kernel(const __grid_constant__ A32Params P) {
   JLX_TL(TL_ATTN_GENERIC);
   constexpr int ROWS = 16 * RI, LDQ = DH + 4, LDP = A32_KEYS + 4, DV = DH / 64;
   extern __shared__ __align__(16) float smem[];
@@ -270,6 +274,7 @@ __global__ void __launch_bounds__(256) attention_f32_kernel(const __grid_constan
   const int split = blockIdx.z % P.splits, row0 = blockIdx.z / P.splits * ROWS;
   if (row0 >= cnt * G) return;
   const int p_first = P.positions[n0], p_last = p_first + cnt - 1, r = P.req_of_token[n0];
+  const int start_last = a32_first_key(P, p_last);
   const A32Ranges ranges = a32_ranges(P, p_first, p_last);
   const int i_first = split * P.per_split, i_end = P.splits == 1 ? ranges.count : min(ranges.count, i_first + P.per_split);
   if (i_first >= i_end) return;
@@ -353,13 +358,15 @@ __global__ void __launch_bounds__(256) attention_f32_kernel(const __grid_constan
 #pragma unroll
       for (int i = 0; i < RI; ++i) {
         float s[4], top = -INFINITY;
+        bool seen[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int at = t0 + tx + 16 * j;
           float x = (a32_low(s2[i][j]) + a32_high(s2[i][j])) * qs[i];
           if (P.softcap > 0.f) x = P.softcap * tanhf(x / P.softcap);
           x = fmaf(-slope[i], (float)(pos[i] - at), x);
-          s[j] = at < end && at <= pos[i] && (at >= start[i] || at < P.keep) ? x : -INFINITY;
+          seen[j] = at < end && at <= pos[i] && (at >= start[i] || at < P.keep);
+          s[j] = seen[j] ? x : -INFINITY;
           top = fmaxf(top, s[j]);
         }
 #pragma unroll
@@ -371,7 +378,7 @@ __global__ void __launch_bounds__(256) attention_f32_kernel(const __grid_constan
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const float w = expf(s[j] - base);
-          Ks[(ty + 16 * i) * LDP + tx + 16 * j] = w;
+          Ks[(ty + 16 * i) * LDP + tx + 16 * j] = seen[j] ? w : -1.f;
           sum += w;
         }
 #pragma unroll
@@ -384,24 +391,31 @@ __global__ void __launch_bounds__(256) attention_f32_kernel(const __grid_constan
       }
       asm volatile("cp.async.wait_group 0;" ::: "memory");
       __syncthreads();  // weights and values are there
+      auto add_values = [&](auto all_seen) {
 #pragma unroll 2
-      for (int j = 0; j < A32_KEYS; j += 4) {
-        float4 w[RI];
+        for (int j = 0; j < A32_KEYS; j += 4) {
+          float4 w[RI];
 #pragma unroll
-        for (int i = 0; i < RI; ++i) w[i] = *reinterpret_cast<const float4*>(Ks + (ty + 16 * i) * LDP + j);
+          for (int i = 0; i < RI; ++i) w[i] = *reinterpret_cast<const float4*>(Ks + (ty + 16 * i) * LDP + j);
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj)
+          for (int jj = 0; jj < 4; ++jj)
 #pragma unroll
-          for (int h = 0; h < DV; ++h) {
-            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(Vs + (j + jj) * DH + 64 * h + 4 * tx);
+            for (int h = 0; h < DV; ++h) {
+              const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(Vs + (j + jj) * DH + 64 * h + 4 * tx);
 #pragma unroll
-            for (int i = 0; i < RI; ++i) {
-              const unsigned long long x = a32_twice(jj == 0 ? w[i].x : (jj == 1 ? w[i].y : (jj == 2 ? w[i].z : w[i].w)));
-              acc[i][2 * h] = a32_fma2(x, v.x, acc[i][2 * h]);
-              acc[i][2 * h + 1] = a32_fma2(x, v.y, acc[i][2 * h + 1]);
+              for (int i = 0; i < RI; ++i) {
+                const float wj = jj == 0 ? w[i].x : (jj == 1 ? w[i].y : (jj == 2 ? w[i].z : w[i].w));
+                if (!decltype(all_seen)::value && wj < 0.f) continue;
+                const unsigned long long x = a32_twice(wj);
+                acc[i][2 * h] = a32_fma2(x, v.x, acc[i][2 * h]);
+                acc[i][2 * h + 1] = a32_fma2(x, v.y, acc[i][2 * h + 1]);
+              }
             }
-          }
-      }
+        }
+      };
+      // (rows that are not there: whatever they add is not stored)
+      if (t0 + A32_KEYS - 1 <= p_first && (t0 >= start_last || t0 + A32_KEYS <= P.keep)) add_values(std::true_type());
+      else add_values(std::false_type());
     }
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
@@ -420,7 +434,7 @@ __global__ void __launch_bounds__(256) attention_f32_kernel(const __grid_constan
             *reinterpret_cast<float4*>(P.part_o + at * dh + d) =
                 make_float4(a32_low(acc[i][2 * h]), a32_high(acc[i][2 * h]), a32_low(acc[i][2 * h + 1]), a32_high(acc[i][2 * h + 1]));
         }
-      } else if (m[i] > -INFINITY) {  // else a range without a key that the row sees
+      } else if (l[i] != 0.f) {  // else a range without a key that the row sees
         float a, b;
         all_m[i] = a32_weights(all_m[i], m[i], a, b);
         all_l[i] = fmaf(l[i], b, all_l[i] * a);
@@ -468,7 +482,7 @@ __global__ void __launch_bounds__(128) attention_f32_combine_kernel(const __grid
   for (int s = 0; s < count; ++s) {
     const float m = P.part_ml[2 * (at + s)], l = P.part_ml[2 * (at + s) + 1];
     const float4 v = d < P.dh ? *reinterpret_cast<const float4*>(P.part_o + (at + s) * P.dh + d) : make_float4(0.f, 0.f, 0.f, 0.f);
-    if (m == -INFINITY) continue;
+    if (l == 0.f) continue;
     float a, b;
     all_m = a32_weights(all_m, m, a, b);
     all_l = fmaf(l, b, all_l * a);

@@ -259,6 +259,36 @@ def test_attention_f32_items_against_the_general_kernel(Hq, Hkv, dh, page, chunk
             assert torch.equal(whole, got)
 
 
+@pytest.mark.parametrize("Hq, Hkv, dh", [(8, 2, 128), (5, 1, 36)])
+@pytest.mark.parametrize("chunk, window, keep, splits", [(0, 0, 0, 1), (0, 0, 0, 3), (64, 0, 0, 1), (0, 70, 5, 2)])
+def test_attention_f32_items_keep_values_of_unseen_keys_out(Hq, Hkv, dh, chunk, window, keep, splits):
+    """Tokens whose keys or values are infinite or not numbers, in tiles and as single tokens, with neighbours of the same tile
+    in front of them and windows that have left them: every token's output is finite where the general kernel's is, which
+    reads only what a token sees, and not a number where that kernel's is not."""
+    lens, q_lens, page = [400, 300, 66], [131, 1, 17], 16
+    q, pages, bt, req, pos, ks, vs = _paged_case(torch.float32, Hq, Hkv, dh, page, lens, q_lens)
+    for r, at, plane, bad in ((0, 290, 1, float("inf")), (0, 350, 0, float("nan")), (0, 397, 1, float("nan")), (0, 120, 1, -float("inf")),
+                              (1, 299, 0, float("nan")), (1, 100, 1, float("inf")), (2, 60, 1, float("nan")), (2, 63, 0, float("inf"))):
+        pages[int(bt[r, at // page]), plane, :, at % page] = bad
+    starts = [sum(q_lens[:r]) for r in range(len(q_lens))]
+    tiles = [(s + o, min(16, n - o)) for s, n in zip(starts, q_lens) if n > 1 for o in range(0, n, 16)]
+    items = torch.tensor(tiles, device=DEV, dtype=torch.int32)
+    singles = torch.tensor([s for s, n in zip(starts, q_lens) if n == 1], device=DEV, dtype=torch.int32)
+    per = -(-4 // splits)
+    part_o = torch.full((2 * q.numel() * splits * per,), float("nan"), device=DEV)
+    part_ml = torch.full((2 * q.shape[0] * Hq * splits * per * 2,), float("nan"), device=DEV)
+    want, got, st = torch.empty_like(q), torch.full_like(q, 7.0), status()
+    common = (q, pages, bt, req, pos)
+    K().attention_generic(*common, want, dh ** -0.5, chunk, window, 0.0, 1.0, st, None, None, 0.0, keep)
+    K().attention_f32(*common, got, dh ** -0.5, chunk, window, 0.0, 1.0, st, len(tiles), items, 16, None, splits, per, part_o, part_ml, keep=keep)
+    K().attention_f32(*common, got, dh ** -0.5, chunk, window, 0.0, 1.0, st, len(singles), None, 1, singles, splits, per, part_o, part_ml, keep=keep)
+    assert int(st) == 0
+    sound = torch.isfinite(want)
+    assert 0 < int(sound.sum()) < sound.numel()
+    assert torch.equal(torch.isfinite(got), sound)
+    close(got[sound], want[sound], 5e-6)
+
+
 def test_attention_finds_one_far_key_among_hundreds():
     """Random keys would hide a key that is skipped or read from the wrong page: here one key far back
     matches the query strongly, so almost all of the output is that key's value."""
