@@ -228,6 +228,24 @@ __device__ __forceinline__ void ch_rows_times(const float* X, int ldx, const flo
   }
 }
 
+// The same for four rows of a diagonal piece, whose first is column n: row n + i takes the columns up to its own and leaves the rows
+// of Y behind them out, whatever they hold (zero times an infinite value would not be zero).
+__device__ __forceinline__ void ch_rows_times_to_diagonal(const float* X, const float* Y, int n, int tx, unsigned long long (&acc)[4][4]) {
+  ch_rows_times(X, PIECE, Y, n, tx, acc);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const ulonglong2 y0 = *reinterpret_cast<const ulonglong2*>(Y + (n + e) * CH_D + 4 * tx), y1 = *reinterpret_cast<const ulonglong2*>(Y + (n + e) * CH_D + 64 + 4 * tx);
+#pragma unroll
+    for (int i = e; i < 4; ++i) {
+      const unsigned long long xx = ch_twice(X[i * PIECE + n + e]);
+      acc[i][0] = ch_fma2(xx, y0.x, acc[i][0]);
+      acc[i][1] = ch_fma2(xx, y0.y, acc[i][1]);
+      acc[i][2] = ch_fma2(xx, y1.x, acc[i][2]);
+      acc[i][3] = ch_fma2(xx, y1.y, acc[i][3]);
+    }
+  }
+}
+
 template <bool READ_AFTER>
 __global__ void __launch_bounds__(CH_THREADS, 2) chunk_outputs_kernel(const __grid_constant__ ChunkParams P) {
   JLX_TL(TL_OTHER);
@@ -426,8 +444,9 @@ __global__ void __launch_bounds__(CH_THREADS, 2) chunk_outputs_kernel(const __gr
   }
   if (4 * ty >= cnt) return;
   const int p = ty / 4;
-  for (int b = 0; b <= p; ++b)
+  for (int b = 0; b < p; ++b)
     ch_rows_times(A + ((p * (p + 1) / 2 + b) * PIECE + 4 * (ty & 3)) * PIECE, PIECE, V + b * PIECE * CH_D, PIECE, tx, acc);
+  ch_rows_times_to_diagonal(A + (p * (p + 3) / 2 * PIECE + 4 * (ty & 3)) * PIECE, V + p * PIECE * CH_D, 4 * (ty & 3), tx, acc);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int t = 4 * ty + i;

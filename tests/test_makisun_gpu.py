@@ -244,6 +244,34 @@ def test_chunk_scan_sizes_strides_and_vanishing_decays(form, dk, dv, H_):
     assert torch.equal(state[5], before[5])
 
 
+@pytest.mark.parametrize("form", ["after", "before"])
+@pytest.mark.parametrize("what", ["v", "k", "d", "q"])
+def test_chunk_scan_keeps_what_is_not_finite_from_earlier_tokens(form, what):
+    """One entry of one token infinite or not a number, at the places of a piece and a chunk: the outputs that are finite are
+    those of the walk, token by token, and the same numbers; the state too."""
+    from jax_llm_examples_b200.kernels import api as K
+
+    H_, dk, dv, N = 2, 72, 68, 150
+    i32 = lambda x: torch.tensor(x, device=DEV, dtype=torch.int32)  # noqa: E731
+    for at, bad in ((5, float("inf")), (31, float("nan")), (32, -float("inf")), (63, float("inf")), (77, float("nan")), (149, float("inf"))):
+        torch.manual_seed(at)
+        t = {"q": torch.randn(N, H_, dk, device=DEV), "k": torch.randn(N, H_, dk, device=DEV) * dk ** -0.5,
+             "d": 0.9 + 0.1 * torch.rand(N, H_, dk, device=DEV), "v": torch.randn(N, H_, dv, device=DEV)}
+        t[what][at, 1, 3] = bad
+        u = torch.randn(H_, dk, device=DEV) if form == "before" else None
+        state = torch.randn(2, H_, dk, dv, device=DEV)
+        walked, o, want = state.clone(), torch.empty(N, H_, dv, device=DEV), torch.empty(N, H_, dv, device=DEV)
+        chunks = i32([(0, c, min(N, c + 64)) for c in range(0, N, 64)])
+        ch = K.Chunks(chunks, i32([(0, 0, 3)]), 3, 1, 1, False)
+        K.chunk_scan(t["q"], t["k"], t["d"], t["v"], u, state, i32([1]), o, form == "after", ch, torch.empty(K.chunk_scan_scratch(3, H_, dk, dv), device=DEV))
+        K.decay_scan(t["q"], t["k"], t["d"], t["v"], u, walked, i32([0, N]), i32([1]), want, form == "after")
+        for got, ref in ((o, want), (state, walked)):
+            sound = torch.isfinite(ref)
+            assert torch.equal(torch.isfinite(got), sound), (what, at)
+            if bool(sound.any()):
+                _close(got[sound], ref[sound], 5e-6, f"{what} of token {at}")
+
+
 def test_decay_forms():
     """exp(-exp(z + b)) and sigmoid(z + b)^(1 / tau) in 32-bit, also far out in both tails; q is scaled, k and v pass."""
     from jax_llm_examples_b200.kernels import api as K
