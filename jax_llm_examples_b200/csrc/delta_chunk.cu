@@ -377,7 +377,10 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_chain_kernel(const __grid
   }
 }
 
-// acc[i][..] += X[i][0 .. n) times Y[0 .. n)[the thread's columns 4 tx .. , 64 + 4 tx ..]; the sum over n is made by itself first
+// total[i][..] += X[i][0 .. n) times Y[0 .. n)[the thread's columns 4 tx .. , 64 + 4 tx ..]; the sum over n is made by itself first.
+// DIAGONAL: row i goes on to column n + i and leaves the rows of Y behind it out, whatever they hold (zero times an infinite value
+// would not be zero).
+template <bool DIAGONAL = false>
 __device__ __forceinline__ void dc_rows_times(const float* X, int ldx, const float* Y, int n, int tx, u64 (&total)[4][4]) {
   u64 acc[4][4];
 #pragma unroll
@@ -402,6 +405,19 @@ __device__ __forceinline__ void dc_rows_times(const float* X, int ldx, const flo
       }
     }
   }
+  if (DIAGONAL)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const ulonglong2 y0 = *reinterpret_cast<const ulonglong2*>(Y + (n + e) * DC_D + 4 * tx), y1 = *reinterpret_cast<const ulonglong2*>(Y + (n + e) * DC_D + 64 + 4 * tx);
+#pragma unroll
+      for (int i = e; i < 4; ++i) {
+        const u64 xx = dc_twice(X[i * ldx + n + e]);
+        acc[i][0] = dc_fma2(xx, y0.x, acc[i][0]);
+        acc[i][1] = dc_fma2(xx, y0.y, acc[i][1]);
+        acc[i][2] = dc_fma2(xx, y1.x, acc[i][2]);
+        acc[i][3] = dc_fma2(xx, y1.y, acc[i][3]);
+      }
+    }
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -475,7 +491,8 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_outputs_kernel(const __gr
     for (int j = 0; j < 4; ++j) asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(acc[i][j]) : "l"(acc[i][j]), "l"(x));
   }
   const int p = ty / 4;
-  for (int b = 0; b <= p; ++b) dc_rows_times(A + ((p * (p + 1) / 2 + b) * PIECE + 4 * (ty & 3)) * PIECE, PIECE, K + b * PIECE * DC_D, PIECE, tx, acc);
+  for (int b = 0; b < p; ++b) dc_rows_times(A + ((p * (p + 1) / 2 + b) * PIECE + 4 * (ty & 3)) * PIECE, PIECE, K + b * PIECE * DC_D, PIECE, tx, acc);
+  dc_rows_times<true>(A + (p * (p + 3) / 2 * PIECE + 4 * (ty & 3)) * PIECE, PIECE, K + p * PIECE * DC_D, 4 * (ty & 3), tx, acc);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int t = 4 * ty + i;

@@ -101,6 +101,31 @@ def test_delta_rule_by_chunks_against_the_walk_and_the_plain_recurrence(dk, dv, 
     assert torch.equal(state[5], before[5])
 
 
+@pytest.mark.parametrize("what", ["v", "k", "beta", "decay", "q"])
+def test_delta_rule_by_chunks_keeps_what_is_not_finite_from_earlier_tokens(what):
+    """One entry of one token infinite or not a number, at the places of a piece and a chunk: the outputs that are finite are
+    those of the walk, token by token, and the same numbers; the state too."""
+    from jax_llm_examples_b200.kernels import api as K
+
+    Hh, G, dk, dv, N = 2, 1, 72, 68, 150
+    for at, bad in ((5, float("inf")), (31, float("nan")), (32, -float("inf")), (63, float("inf")), (77, float("nan")), (149, float("inf"))):
+        torch.manual_seed(at)
+        t = {"q": torch.randn(N, G, dk, device=DEV) * dk ** -0.5, "k": torch.nn.functional.normalize(torch.randn(N, G, dk, device=DEV), dim=-1),
+             "v": torch.randn(N, Hh, dv, device=DEV), "beta": torch.rand(N, Hh, device=DEV), "decay": 0.9 + 0.1 * torch.rand(N, Hh, device=DEV)}
+        t[what][(at, 1) if t[what].dim() == 2 else (at, t[what].shape[1] - 1, 3)] = bad
+        state = torch.randn(2, Hh, dk, dv, device=DEV) * 0.3
+        walked, o, want = state.clone(), torch.empty(N, Hh, dv, device=DEV), torch.empty(N, Hh, dv, device=DEV)
+        ch = K.Chunks(_i32([(0, c, min(N, c + 64)) for c in range(0, N, 64)]), _i32([(0, 0, 3)]), 3, 1, 1, False)
+        ops = (t["q"], t["k"], t["v"], t["beta"], t["decay"])
+        K.delta_chunk(*ops, state, _i32([1]), o, ch, torch.empty(K.delta_chunk_scratch(3, Hh, dk, dv), device=DEV))
+        K.delta_scan(*ops, walked, _i32([0, N]), _i32([1]), want)
+        for got, ref in ((o, want), (state, walked)):
+            sound = torch.isfinite(ref)
+            assert torch.equal(torch.isfinite(got), sound), (what, at)
+            if bool(sound.any()):
+                _close(got[sound], ref[sound], 5e-6, f"{what} of token {at}")
+
+
 def test_delta_scan_keeps_a_far_token_and_corrects_a_key_that_is_written_again():
     """Made so that a fault shows.  Head 1 never decays.  Along key direction e0 it is written ONCE with a full step, at
     token 3; 700 tokens later a query along e0 must read that value exactly, through portions of many sizes and a state
