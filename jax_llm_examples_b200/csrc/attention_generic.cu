@@ -198,8 +198,9 @@ struct A32Params {
   const float* slopes;
   float softcap;
   int splits, per_split;  // blocks that share an item's ranges (1: one block merges them itself), and the ranges of one
-  float* part_o;          // [token row][Hq][splits * per_split][dh]
-  float* part_ml;         // [token row][Hq][splits * per_split][2]
+  int part_rows;          // rows of the partial results: 0: a token's row of the step, else item * part_rows + its place in the item
+  float* part_o;          // [row][Hq][splits * per_split][dh]
+  float* part_ml;         // [row][Hq][splits * per_split][2]
   int* status;
 };
 
@@ -422,7 +423,8 @@ __global__ void __launch_bounds__(256, RI == 1 ? 3 : 1) attention_f32_kernel(con
       const int row = row0 + ty + 16 * i;
       if (P.splits > 1) {
         if (row >= cnt * G) continue;
-        const size_t at = ((size_t)(n0 + row / G) * P.Hq + hk * G + row % G) * (P.splits * P.per_split) + ri;
+        const int part_row = P.part_rows ? blockIdx.x * P.part_rows + row / G : n0 + row / G;
+        const size_t at = ((size_t)part_row * P.Hq + hk * G + row % G) * (P.splits * P.per_split) + ri;
         if (tx == 0) {
           P.part_ml[2 * at] = m[i];
           P.part_ml[2 * at + 1] = l[i];
@@ -474,7 +476,7 @@ __global__ void __launch_bounds__(128) attention_f32_combine_kernel(const __grid
   const int t = blockIdx.x % max_count, lane = threadIdx.x & 31, h = blockIdx.y * 4 + (threadIdx.x >> 5);
   if (t >= cnt || h >= P.Hq) return;
   const int p_first = P.positions[n0], count = min(a32_ranges(P, p_first, p_first + cnt - 1).count, P.splits * P.per_split);
-  const size_t at = ((size_t)(n0 + t) * P.Hq + h) * (P.splits * P.per_split);
+  const size_t at = ((size_t)(P.part_rows ? blockIdx.x : n0 + t) * P.Hq + h) * (P.splits * P.per_split);
   float all_m = -INFINITY, all_l = 0.f;
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
   const int d = 4 * lane;
@@ -511,12 +513,12 @@ static cudaError_t launch_attention_f32(const A32Params& P, int n_items, int row
 }
 
 // n_items items of at most max_count tokens (items null: single tokens, rows[i] or i).  part_o, part_ml: for splits > 1, room for
-// every token row of the step.
+// every token row of the step, or (part_by_item) for n_items * max_count rows.
 JLX_API int jlx_attention_f32(const float* q, const float* pages, const int* block_table, int bt_stride, const int* req_of_token,
                               const int* positions, float* out, int Hq, int Hkv, int dh, int page_size, int num_pages, float scale,
                               int chunk, int window, int keep, float attn_scale, float floor_scale, const float* sink, const float* slopes,
                               float softcap, const int* items, const int* rows, int n_items, int max_count, int splits, int per_split,
-                              float* part_o, float* part_ml, int* status, cudaStream_t stream) {
+                              int part_by_item, float* part_o, float* part_ml, int* status, cudaStream_t stream) {
   JLX_REQUIRE(Hq > 0 && Hkv > 0 && page_size > 0 && num_pages > 0 && n_items >= 0, "attention_f32: bad sizes");
   JLX_REQUIRE(Hq % Hkv == 0 && Hkv <= 65535, "attention_f32: %d query heads for %d KV heads", Hq, Hkv);
   JLX_REQUIRE(jlx_attention_f32_supported(dh), "attention_f32: head size %d is no multiple of 4 up to 128", dh);
@@ -530,7 +532,8 @@ JLX_API int jlx_attention_f32(const float* q, const float* pages, const int* blo
   const int row_blocks = (rows_of_item + (few ? 15 : 63)) / (few ? 16 : 64);
   JLX_REQUIRE((long long)row_blocks * splits <= 65535, "attention_f32: too many key ranges");
   const A32Params P = {q, pages, block_table, bt_stride, req_of_token, positions, out, items, rows, Hq, Hkv, dh, page_size, num_pages, scale,
-                       chunk, window, keep, attn_scale, floor_scale, sink, slopes, softcap, splits, per_split, part_o, part_ml, status};
+                       chunk, window, keep, attn_scale, floor_scale, sink, slopes, softcap, splits, per_split, part_by_item ? max_count : 0, part_o,
+                       part_ml, status};
   if (dh <= 64) JLX_CUDA((few ? launch_attention_f32<64, 1>(P, n_items, row_blocks, stream) : launch_attention_f32<64, 4>(P, n_items, row_blocks, stream)));
   else JLX_CUDA((few ? launch_attention_f32<128, 1>(P, n_items, row_blocks, stream) : launch_attention_f32<128, 4>(P, n_items, row_blocks, stream)));
   if (splits > 1) {

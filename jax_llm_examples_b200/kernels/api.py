@@ -976,6 +976,12 @@ def attention_f32_plan(max_kv_len: int, chunk: int, window: int, keep: int, bloc
     return -(-ranges // per), per
 
 
+def attention_f32_part_rows(n_tokens: int, n_items: int, max_count: int) -> int:
+    """Rows of partial results that a launch over ``n_items`` items of up to ``max_count`` tokens keeps: its own, or the
+    step's where those are fewer."""
+    return min(n_tokens, n_items * max_count)
+
+
 def attention_f32(q: torch.Tensor, pages: torch.Tensor, block_table: torch.Tensor, req_of_token: torch.Tensor, positions: torch.Tensor,
                   out: torch.Tensor, scale: float, chunk: int, window: int, attn_scale: float, floor_scale: float, status: torch.Tensor,
                   n_items: int, items: torch.Tensor | None = None, max_count: int = 1, rows: torch.Tensor | None = None, splits: int = 1,
@@ -983,8 +989,8 @@ def attention_f32(q: torch.Tensor, pages: torch.Tensor, block_table: torch.Tenso
                   sink: torch.Tensor | None = None, slopes: torch.Tensor | None = None, softcap: float = 0.0, keep: int = 0) -> None:
     """:func:`attention_generic` in float32 by work items: ``items`` int32 pairs (first token row, count <= 16) of one request
     each, or single tokens (``rows``: their token rows; None: rows 0 .. n_items).  ``splits`` > 1 blocks
-    share an item's key ranges, ``per_split`` each; part_o: float32 [N * Hq * splits * per_split * dh], part_ml: the same with 2
-    for dh."""
+    share an item's key ranges, ``per_split`` each; part_o: float32 [rows * Hq * splits * per_split * dh] with rows =
+    ``attention_f32_part_rows``, part_ml: the same with 2 for dh."""
     _contig(q, pages, block_table, out, items, rows, part_o, part_ml)
     N, Hq, dh = q.shape
     _check_sink(sink, Hq)
@@ -992,13 +998,15 @@ def attention_f32(q: torch.Tensor, pages: torch.Tensor, block_table: torch.Tenso
     P, _, Hkv, page_size, dh2 = pages.shape
     if dh2 != dh or any(t.dtype != torch.float32 for t in (q, pages, out)) or out.numel() != q.numel():
         raise KernelError("attention_f32: queries, pages and output must be float32 of one head size")
-    if splits > 1 and (part_o is None or part_ml is None or part_o.numel() < N * Hq * splits * per_split * dh
-                       or part_ml.numel() < N * Hq * splits * per_split * 2):
+    part_rows = attention_f32_part_rows(N, n_items, max_count)
+    if splits > 1 and (part_o is None or part_ml is None or part_o.numel() < part_rows * Hq * splits * per_split * dh
+                       or part_ml.numel() < part_rows * Hq * splits * per_split * 2):
         raise KernelError("attention_f32: scratch for the partial results is too small")
     _run("attention_generic", "jlx_attention_f32", _ptr(q), _ptr(pages), _ptr(block_table), c_int(block_table.shape[1]), _ptr(req_of_token),
          _ptr(positions), _ptr(out), c_int(Hq), c_int(Hkv), c_int(dh), c_int(page_size), c_int(P), c_float(scale), c_int(chunk), c_int(window),
          c_int(keep), c_float(attn_scale), c_float(floor_scale), _ptr(sink), _ptr(slopes), c_float(softcap), _ptr(items), _ptr(rows),
-         c_int(n_items), c_int(max_count), c_int(splits), c_int(per_split), _ptr(part_o), _ptr(part_ml), _ptr(status), _stream())
+         c_int(n_items), c_int(max_count), c_int(splits), c_int(per_split), c_int(int(part_rows < N)), _ptr(part_o), _ptr(part_ml),
+         _ptr(status), _stream())
 
 
 def _check_sink(sink: torch.Tensor | None, Hq: int, what: str = "sink") -> None:

@@ -137,19 +137,46 @@ class PagedAttention(Mixer):
                            chunk, window, attn_scale, floor_scale, part_o, part_ml, splits, split_keys, ctx.status,
                            rows, n_rows, self.sink, self.slopes, self.softcap, self.keep_first, diff)
 
+    # The 32-bit attention keeps the partial results of its key ranges up to this size (float32 elements): longer work goes in
+    # passes over its items, and an item that alone keeps more is not split.
+    F32_SCRATCH = 1 << 26
+
     def _items_f32(self, ctx: StepContext, q, cache: LayerCache, out, attn_scale, floor_scale, n_items: int, items=None, rows=None) -> None:
-        """The 32-bit attention over portions in tiles (``items``), or over single tokens."""
+        """The 32-bit attention over portions in tiles (``items``), or over single tokens (the listed rows, or all)."""
         chunk, window = self.chunk or 0, self.window or 0
-        per_item = (FLASH_TILE if items is not None else 1) * self.n_heads // self.n_kv_heads
-        splits, per_split = K.attention_f32_plan(ctx.max_kv_len, chunk, window, self.keep_first, n_items * self.n_kv_heads * -(-per_item // 64))
+        tokens = FLASH_TILE if items is not None else 1  # of an item, at most
+        blocks = self.n_kv_heads * -(-tokens * self.n_heads // self.n_kv_heads // 64)
+        kept = lambda n, plan: K.attention_f32_part_rows(q.shape[0], n, tokens) * self.n_heads * plan[0] * plan[1]  # noqa: E731
+        most, plan = n_items, K.attention_f32_plan(ctx.max_kv_len, chunk, window, self.keep_first, n_items * blocks)
+        while plan[0] > 1 and kept(most, plan) * self.head_dim > self.F32_SCRATCH:
+            if most == 1:
+                most, plan = n_items, (1, 0)
+                break
+            most = -(-most // 2)
+            plan = K.attention_f32_plan(ctx.max_kv_len, chunk, window, self.keep_first, most * blocks)
         part_o = part_ml = None
-        if splits > 1:
-            n = q.shape[0] * self.n_heads * splits * per_split
-            part_o = ctx.workspace.get("attn_f32_part_o", n * self.head_dim, torch.float32)
-            part_ml = ctx.workspace.get("attn_f32_part_ml", n * 2, torch.float32)
-        K.attention_f32(q, cache.pages, cache.block_table, ctx.req_of_token, ctx.positions, out, self.scale, chunk, window, attn_scale,
-                        floor_scale, ctx.status, n_items, items, FLASH_TILE if items is not None else 1, rows, splits, per_split, part_o, part_ml,
-                        self.sink, self.slopes, self.softcap, self.keep_first)
+        if plan[0] > 1:
+            part_o = self._scratch_f32(ctx, "attn_f32_part_o", kept(most, plan) * self.head_dim, q.device)
+            part_ml = self._scratch_f32(ctx, "attn_f32_part_ml", kept(most, plan) * 2, q.device)
+        for i in range(0, n_items, most):
+            n, of_step = min(most, n_items - i), (q, out, ctx.req_of_token, ctx.positions)
+            part_items, part_rows = items, rows
+            if n < n_items:  # a pass over some of the items
+                if items is not None:
+                    part_items = items[2 * i:2 * (i + n)]
+                elif rows is not None:
+                    part_rows = rows[i:i + n]
+                else:
+                    of_step = tuple(t[i:i + n] for t in of_step)
+            q_of, out_of, req_of_token, positions = of_step
+            K.attention_f32(q_of, cache.pages, cache.block_table, req_of_token, positions, out_of, self.scale, chunk, window, attn_scale,
+                            floor_scale, ctx.status, n, part_items, tokens, part_rows, *plan, part_o, part_ml, self.sink, self.slopes,
+                            self.softcap, self.keep_first)
+
+    @staticmethod
+    def _scratch_f32(ctx: StepContext, name: str, numel: int, device) -> torch.Tensor:
+        """Scratch in powers of two: a context that grows leaves few outgrown buffers behind in the workspace."""
+        return ctx.workspace.get(name, 1 << (numel - 1).bit_length(), torch.float32)
 
     def attend(self, ctx: StepContext, q, cache: LayerCache, out, attn_scale: float, floor_scale: float, diff=None) -> None:
         """Tensor-core kernels where they are built (bfloat16, head size 64 or 128): split-KV for
