@@ -176,6 +176,8 @@ class PagedAttention(Mixer):
     @staticmethod
     def _scratch_f32(ctx: StepContext, name: str, numel: int, device) -> torch.Tensor:
         """Scratch in powers of two: a context that grows leaves few outgrown buffers behind in the workspace."""
+        if ctx.workspace is None:
+            return torch.empty(numel, dtype=torch.float32, device=device)
         return ctx.workspace.get(name, 1 << (numel - 1).bit_length(), torch.float32)
 
     def attend(self, ctx: StepContext, q, cache: LayerCache, out, attn_scale: float, floor_scale: float, diff=None) -> None:
