@@ -960,8 +960,10 @@ def attention_generic(q: torch.Tensor, pages: torch.Tensor, block_table: torch.T
          c_float(floor_scale), _ptr(sink), _ptr(slopes), c_float(softcap), _ptr(status), _stream())
 
 
-def attention_f32_supported(q: torch.Tensor) -> bool:
-    return q.dtype == torch.float32 and q.data_ptr() % 16 == 0 and bool(library("attention_generic").jlx_attention_f32_supported(c_int(q.shape[2])))
+def attention_f32_supported(q: torch.Tensor, pages: torch.Tensor, out: torch.Tensor) -> bool:
+    """float32 throughout, a head size that :func:`attention_f32` takes, and rows on 16-byte boundaries."""
+    return all(t.dtype == torch.float32 and t.data_ptr() % 16 == 0 for t in (q, pages, out)) and \
+        bool(library("attention_generic").jlx_attention_f32_supported(c_int(q.shape[2])))
 
 
 ATTENTION_F32_RANGE = 256  # keys of a range, csrc/attention_generic.cu

@@ -215,7 +215,7 @@ class PagedAttention(Mixer):
                                         self.softcap, self.keep_first, diff)
                 return
         maps = out if diff is None else torch.empty(q.shape, dtype=torch.float32, device=q.device)
-        if not (K.attention_f32_supported(q) and (decode or "attn_tiles_all" in ctx.arrays)):
+        if not (K.attention_f32_supported(q, cache.pages, maps) and (decode or "attn_tiles_all" in ctx.arrays)):
             K.attention_generic(q, cache.pages, cache.block_table, ctx.req_of_token, ctx.positions, maps, self.scale,
                                 self.chunk or 0, self.window or 0, attn_scale, floor_scale, ctx.status, self.sink, self.slopes, self.softcap,
                                 self.keep_first)

@@ -498,3 +498,25 @@ def test_scratch_of_the_second_stream_is_kept_apart():
         assert ws.get("scratch", 32, torch.float32).data_ptr() == beside.data_ptr()
     assert beside.data_ptr() != before.data_ptr()
     assert ws.get("scratch", 64, torch.float32).data_ptr() == before.data_ptr()
+
+
+@pytest.mark.parametrize("q_lens, starts", [((40, 1, 17), (30, 600, 5)), ((1, 1, 1), (30, 600, 5))])
+def test_float32_attention_over_pages_off_16_byte_boundaries(q_lens, starts):
+    """Pages or queries one entry behind a 16-byte boundary go to the kernel that serves any address: the same results as on the
+    boundary, to two orders of sums over up to 600 products in float32."""
+    import jax_llm_examples_b200 as J
+    from jax_llm_examples_b200.parts import LayerCache, PagedAttention
+
+    torch.manual_seed(1)
+    heads, kv, dh, off = 8, 2, 64, lambda t: torch.cat([t.new_zeros(1), t.reshape(-1)])[1:].view_as(t)  # noqa: E731
+    mixer = PagedAttention(torch.zeros((heads + 2 * kv) * dh, 8, device=DEV), torch.zeros(8, heads * dh, device=DEV), heads, kv, dh, None)
+    ctx, table = _ctx(J, J.parts.Runtime(torch.float32, torch.device(DEV)), q_lens, starts, n_pages=128)
+    pages, q = torch.randn(128, 2, kv, 16, dh, device=DEV), torch.randn(sum(q_lens), heads, dh, device=DEV)
+    outs = []
+    for p, x in ((pages, q), (off(pages), q), (pages, off(q))):
+        out = torch.full_like(q, float("nan"))
+        mixer.attend(ctx, x, LayerCache(p, table, True, None), out, 0.0, 1.0)
+        outs.append(out)
+    assert int(ctx.status) == 0
+    for out in outs[1:]:
+        assert float((out - outs[0]).abs().max()) < 5e-6 * float(outs[0].abs().max())
