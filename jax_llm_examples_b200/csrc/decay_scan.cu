@@ -278,9 +278,11 @@ decay_prep_x4_kernel(RowsView q, RowsView k, RowsView v, RowsView z, const float
     for (int c = 4 * threadIdx.x; c < H * dv; c += 4 * blockDim.x) *reinterpret_cast<float4*>(vo + n * H * dv + c) = rows_at4(v, n, c);
 }
 
-// Whether jlx_decay_prep can leave outputs out for these views.
-JLX_API int jlx_decay_prep_selective(const RowsView* q, const RowsView* k, const RowsView* v, const RowsView* z, int dk, int dv, int rot) {
-  return dk % 4 == 0 && dv % 4 == 0 && rot % 8 == 0 && rot <= PREP_MAX_ROT && rows_vec(*q) && rows_vec(*k) && rows_vec(*v) && (!z || rows_vec(*z));
+// Whether jlx_decay_prep can leave outputs out for these views (outputs that start on 16-byte boundaries).
+JLX_API int jlx_decay_prep_selective(const RowsView* q, const RowsView* k, const RowsView* v, const RowsView* z, const float* z_bias, int dk, int dv,
+                                     int rot) {
+  return dk % 4 == 0 && dv % 4 == 0 && rot % 8 == 0 && rot <= PREP_MAX_ROT && rows_vec(*q) && rows_vec(*k) && rows_vec(*v) && (!z || rows_vec(*z)) &&
+         on16(z_bias);
 }
 
 JLX_API int jlx_decay_prep(const RowsView* q, const RowsView* k, const RowsView* v, const RowsView* z, const float* z_bias,
@@ -295,8 +297,7 @@ JLX_API int jlx_decay_prep(const RowsView* q, const RowsView* k, const RowsView*
   if (!z) z = &none;
   if (N == 0) return 0;
   const float inv_tau = mode == DECAY_SIGMOID_POWER ? 1.f / tau : 0.f;
-  if (dk % 4 == 0 && dv % 4 == 0 && rot % 8 == 0 && rot <= PREP_MAX_ROT && rows_vec(*q) && rows_vec(*k) && rows_vec(*v) && rows_vec(*z) && on16(z_bias) &&
-      on16(qo) && on16(ko) && on16(d_out) && on16(vo)) {
+  if (jlx_decay_prep_selective(q, k, v, z, z_bias, dk, dv, rot) && on16(qo) && on16(ko) && on16(d_out) && on16(vo)) {
     JLX_CUDA(jlx_launch_pdl(decay_prep_x4_kernel, dim3(N), dim3(256), 0, stream, *q, *k, *v, *z, z_bias, mode, inv_tau, q_scale, qo, ko, d_out, vo, H,
                             dk, dv, head_decay, k_scale, inv_freq, rot, positions));
     JLX_LAUNCH_CHECK("decay_prep");

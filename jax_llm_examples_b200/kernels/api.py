@@ -633,10 +633,11 @@ def decay_prep(q: _RowsView, k: _RowsView, v: _RowsView, z: _RowsView | None, z_
          _stream())
 
 
-def decay_prep_selective(q: _RowsView, k: _RowsView, v: _RowsView, z: _RowsView | None, dk: int, dv: int, rot_dims: int) -> bool:
-    """Whether ``decay_prep`` can leave outputs out for these rows."""
+def decay_prep_selective(q: _RowsView, k: _RowsView, v: _RowsView, z: _RowsView | None, z_bias: torch.Tensor | None, dk: int, dv: int,
+                         rot_dims: int) -> bool:
+    """Whether ``decay_prep`` can leave outputs out for these rows (and outputs that start on 16-byte boundaries)."""
     return bool(library("decay_scan").jlx_decay_prep_selective(ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(z) if z is not None else None,
-                                                              c_int(dk), c_int(dv), c_int(rot_dims)))
+                                                              _ptr(z_bias), c_int(dk), c_int(dv), c_int(rot_dims)))
 
 
 def view_rows(v: _RowsView, n: int, heads: int, size: int) -> torch.Tensor:

@@ -24,7 +24,7 @@ def _scan(ctx: StepContext, q, k, v, z, z_bias, form: str, tau: float, q_scale: 
     chunks, scratch = scan_chunks(ctx, heads, dk, dv)
     walks = chunks is None or chunks.others
     # where the chunk kernels serve all requests, operands that need no arithmetic are read where they were projected
-    whole = not walks and K.decay_prep_selective(q, k, v, z, dk, dv, prep.get("rot_dims", 0))
+    whole = not walks and K.decay_prep_selective(q, k, v, z, z_bias, dk, dv, prep.get("rot_dims", 0))
     stays = {"q": whole and q.splits == 1 and q_scale == 1.0 and not prep.get("rot_dims"),
              "k": whole and k.splits == 1 and prep.get("k_scale", 1.0) == 1.0 and not prep.get("rot_dims"), "v": whole and v.splits == 1}
     need = n * heads * (3 * dk + 2 * dv)

@@ -133,3 +133,22 @@ def test_hgrn2_kernels_with_chunks_from_partial_sums(splits, dk, dv, lens):
     _close(out, want, 1e-5, "outputs")
     _close(state, walked, 1e-5, "states")
     assert torch.equal(state[0], walked[0]) and torch.equal(qfv, before)
+
+
+def _off(t):
+    """The same numbers one entry behind a 16-byte boundary."""
+    moved = torch.cat([t.new_zeros(1), t.reshape(-1)])[1:].view_as(t)
+    assert moved.data_ptr() % 16
+    return moved
+
+
+def test_a_decays_bias_off_16_byte_boundaries():
+    """Long portions of a gated linear attention take it as ever, whatever of q, k and v is left in place."""
+    torch.manual_seed(7)
+    mixer, _ = _mixer("gated", torch.float32, 2, 128, 128, 40)
+    seqs, steps, outs = [torch.randn(500, 40)], [[(0, 0, 450)], [(0, 450, 500)]], []
+    for bias in (mixer.a_bias, _off(mixer.a_bias)):
+        mixer.a_bias = bias
+        states = tuple(torch.zeros(2, *n.shape, device=DEV) for n in mixer.state_needs())
+        outs.append(_run(mixer, torch.float32, seqs, steps, [1], states, mixer.step_planners())[0])
+    _close(outs[1], outs[0], 1e-5)
