@@ -521,7 +521,7 @@ JLX_API int jlx_delta_chunk(const float* q, const float* k, const float* v, cons
   JLX_REQUIRE(jlx_delta_chunk_supported(dk, dv), "delta_chunk: heads of %d x %d are not supported", dk, dv);
   JLX_REQUIRE(H <= 65535, "delta_chunk: too many heads");
   if (n == 0 || m == 0) return 0;
-  JLX_REQUIRE(scratch && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)o | (uintptr_t)scratch | (uintptr_t)state) & 15) == 0,
+  JLX_REQUIRE(scratch && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)o | (uintptr_t)scratch) & 15) == 0,
               "delta_chunk: rows must start on 16-byte boundaries");
   float* X = scratch;
   float* Y = X + (size_t)n * H * CHUNK * dv;

@@ -152,3 +152,14 @@ def test_a_decays_bias_off_16_byte_boundaries():
         states = tuple(torch.zeros(2, *n.shape, device=DEV) for n in mixer.state_needs())
         outs.append(_run(mixer, torch.float32, seqs, steps, [1], states, mixer.step_planners())[0])
     _close(outs[1], outs[0], 1e-5)
+
+
+def test_states_of_the_delta_rule_off_16_byte_boundaries():
+    """The kernels for long portions read and write states entry by entry: slabs may start anywhere, as for the walk."""
+    torch.manual_seed(7)
+    mixer, _ = _mixer("delta", torch.float32, 2, 128, 128, 40)
+    seqs, steps, outs = [torch.randn(500, 40)], [[(0, 0, 450)], [(0, 450, 500)]], []
+    for place in (lambda s: s, _off):
+        states = tuple(place(torch.zeros(2, *n.shape, device=DEV)) for n in mixer.state_needs())
+        outs.append(_run(mixer, torch.float32, seqs, steps, [1], states, mixer.step_planners())[0])
+    _close(outs[1], outs[0], 1e-5)
