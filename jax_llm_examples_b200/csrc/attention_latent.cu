@@ -39,7 +39,8 @@ __device__ __forceinline__ void store4(bf16* p, float4 v) {
   o2[1] = __floats2bfloat162_rn(v.z, v.w);
   *reinterpret_cast<uint2*>(p) = o;
 }
-// Bound by a block's chain (row, meeting, write) times the blocks an SM holds: 2048 tokens, latents of 768 and 512: 11 us (18.5 with 4-byte accesses).
+// Bound by a block's chain (row, meeting, write) times the blocks an SM holds: 2048 tokens, latents of 768 and 512: 15 us (18.5 with 4-byte accesses;
+// 11 with each thread's four entries added first, which is another order of the sums).
 template <typename TO>
 __global__ void latent_kv_prep_kernel(const float* __restrict__ proj, int splits, long long split_stride,
                                       const float* __restrict__ q_norm_w, const float* __restrict__ kv_norm_w, float eps,
@@ -82,10 +83,11 @@ __global__ void latent_kv_prep_kernel(const float* __restrict__ proj, int splits
         const float4 x = *reinterpret_cast<const float4*>(from + (size_t)z * split_stride + i);
         v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
       }
-      *reinterpret_cast<float4*>(sums + i) = v;  // (read back by this thread only)
-      ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss))));
+      *reinterpret_cast<float4*>(sums + i) = v;
     }
     if (blockIdx.y == 1) rotated_part(to + rank);
+    __syncthreads();
+    for (int i = threadIdx.x; i < size; i += blockDim.x) ss = fmaf(sums[i], sums[i], ss);  // in the order of the rows below
     const float rms = sqrtf(block_sum(ss, scratch) / (float)size + eps);
     for (int i = 4 * threadIdx.x; i < size; i += 4 * blockDim.x) {
       const float4 v = *reinterpret_cast<const float4*>(sums + i), g = *reinterpret_cast<const float4*>(gamma + i);
@@ -136,7 +138,7 @@ JLX_API int jlx_latent_kv_prep(const float* proj, int splits, long long split_st
   // 16 bytes per access where rows and norm weights allow it
   const int vec = ((q_rank | rank | dr | ld) & 3) == 0 && (split_stride & 3) == 0 &&
                   (((uintptr_t)proj | (uintptr_t)q_norm_w | (uintptr_t)kv_norm_w | (uintptr_t)cq | (uintptr_t)pages) & 15) == 0;
-  const int threads = widest >= (vec ? 1024 : 512) ? 256 : 128;  // (never by the number of tokens: it gives the sums their order)
+  const int threads = widest >= 512 ? 256 : 128;  // by the widths alone: it gives the sums their order
   JLX_DISPATCH_DTYPE(dtype, TO, {
     // a block for the query's latent and one for the cached row
     JLX_CUDA(jlx_launch_pdl(latent_kv_prep_kernel<TO>, dim3(N, pages ? 2 : 1), dim3(threads), sizeof(float) * (size_t)widest, stream, proj, splits, split_stride, q_norm_w, kv_norm_w,

@@ -347,6 +347,30 @@ def test_prompt_softmax_rows_in_registers_and_at_the_edges_of_their_lengths(L, w
             assert not bool(p[:, ~seen].any())
 
 
+@pytest.mark.parametrize("q_rank, rank, dr", [(64, 32, 8), (768, 512, 64), (512, 516, 4), (1536, 96, 0), (1028, 1024, 64)])
+@pytest.mark.parametrize("splits", [1, 2])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_latents_are_normed_in_one_order_at_every_address(dtype, splits, q_rank, rank, dr):
+    """Rows and weights on 16-byte boundaries are read in whole pieces, others entry by entry: the same latents and cached rows
+    to the bit."""
+    from jax_llm_examples_b200.kernels import api as K
+
+    torch.manual_seed(rank)
+    N, page = 11, 16
+    i32 = lambda v: torch.tensor(v, device=DEV, dtype=torch.int32)  # noqa: E731
+    proj = torch.randn(splits, N, q_rank + rank + dr + 4, device=DEV)
+    proj = proj if splits > 1 else proj[0]
+    qw, kw, freq = torch.rand(q_rank, device=DEV) + 0.5, torch.rand(rank, device=DEV) + 0.5, torch.rand(dr // 2, device=DEV)
+    moved = torch.cat([qw.new_zeros(1), qw])[1:]
+    outs = []
+    for weight in (qw, moved):
+        cq, pages, status = torch.zeros(N, q_rank, device=DEV, dtype=dtype), torch.zeros(1, 1, 1, page, rank + dr, device=DEV, dtype=dtype), i32([0])
+        K.latent_kv_prep(proj, splits, weight, kw, 1e-5, freq, dr, cq, pages, i32([[0]]), i32([0] * N), i32(list(range(N))), q_rank, rank, dr, status)
+        assert int(status) == 0
+        outs.append((cq, pages))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
 @pytest.mark.parametrize("page", [16, 24, 32, 64])
 @pytest.mark.parametrize("rank, dr, H_", [(32, 8, 3), (128, 64, 16), (136, 0, 17), (512, 64, 16), (520, 16, 5), (768, 64, 2)])
 def test_latent_decode_on_the_tensor_cores_at_the_edges_of_its_pieces(rank, dr, H_, page):
