@@ -468,12 +468,13 @@ __global__ void attention_latent_kernel(const float* __restrict__ q_lat, const f
 // Tiles of 32 keys come by cp.async, two in flight, found through the block table: once per tile where pages are multiples of
 // the tile, else row by row; a key's row [c | k_rot] in shared memory is padded by 16 bytes so that ldmatrix meets no bank
 // twice.
-//   scores   warp w takes keys [8 (w % 4), + 8) of the tile and one half of the row against all 16 queries (bfloat16,
-//            32-bit sums); the halves meet in shared memory
-//   softmax  warp w takes heads 2 w and 2 w + 1, a key per lane: running maximum and sum (32-bit), the weights in bfloat16
+//   scores   warp w takes keys [8 (w % 4), + 8) of the tile and every second 16 columns of the row against all 16 queries
+//            (bfloat16, 32-bit sums, one strand for the even pieces and one for the odd); the strands meet in shared memory
+//   softmax  warp w takes heads 2 w and 2 w + 1, half a warp each: running maximum and sum (32-bit; eight keys one by one,
+//            then the four eights), the weights in bfloat16
 //   values   warp w takes the latent's 16-column pieces w, w + 8, ...: the weights times the tile's rows
 // Bound by the latency of a tile's chain and its instructions: with two blocks of 37 KB tiles an SM, eight warps that each
-// did the softmax of all heads took 6 us a tile.  32 requests of 4096 keys, 16 heads: 56 us (81).
+// did the softmax of all heads took 6 us a tile.  32 requests of 4096 keys, 16 heads: 54 us (81), 32 heads 109 (168).
 // When every served token is its request's only one of the step (`single`), everything but its own row is older than the
 // step: tiles that end below it are asked for before the wait for the predecessor.  Rows outside [lo, t_end] are zeros in shared memory and masked.
 #define LATM_KEYS LAT_TILE
@@ -491,7 +492,7 @@ attention_latent_mma_kernel(const bf16* __restrict__ q_lat, const bf16* __restri
                             int window, int single, int* status) {
   JLX_TL(TL_ATTN_GENERIC);
   extern __shared__ __align__(16) uint8_t smem_bytes[];
-  __shared__ float sc[2][16][LATM_KEYS + 2];         // the halves' scores
+  __shared__ __align__(8) float sc[2][16][LATM_KEYS + 2];  // the strands' scores
   __shared__ __align__(16) bf16 pw[16][LATM_LDP];    // the weights
   __shared__ float corr_of[16], m_of[16], l_of[16];
   const int dk = rank + dr, dkp = (dk + 15) & ~15;  // products take 16 columns at a time: the rest of a row is zero
@@ -563,13 +564,10 @@ attention_latent_mma_kernel(const bf16* __restrict__ q_lat, const bf16* __restri
   const int g0 = lane >> 2, g1 = g0 + 8;  // this thread's two heads
   const float sc2 = scale * 1.4426950408889634f;
   const bool has_sink = sink != nullptr && z == 0;
-  float m[2], l[2];  // base-2 running maximum and sum of heads 2 warp and 2 warp + 1
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int h = h0 + 2 * warp + u;
-    m[u] = has_sink && h < H ? sink[h] * 1.4426950408889634f : -INFINITY;
-    l[u] = has_sink ? 1.f : 0.f;
-  }
+  // the softmax: half a warp has a head, lanes 4 q + i of it the keys 2 q + 8 i and the next one
+  const int hd = 2 * warp + (lane >> 4), key2 = ((lane >> 2) & 3) * 2 + (lane & 3) * 8;
+  float m = has_sink && h0 + hd < H ? sink[h0 + hd] * 1.4426950408889634f : -INFINITY;  // base-2 running maximum and sum
+  float l = has_sink ? 1.f : 0.f;                                                        // (the sum: in the lanes 4 q + 3)
   float o[PIECES][2][4];
 #pragma unroll
   for (int i = 0; i < PIECES; ++i)
@@ -585,45 +583,57 @@ attention_latent_mma_kernel(const bf16* __restrict__ q_lat, const bf16* __restri
       cp_async_commit();
     }
     const bf16* kt = ks + (size_t)(t & 1) * LATM_KEYS * ldk;
-    // scores of this warp's 8 keys over its half of the row (whole 32 columns); two chains of sums
-    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
-    const int kw = warp & 3, half = warp >> 2, mid = (dkp / 2 + 31) & ~31, d_end = half ? dkp : min(mid, dkp);
-    const uint32_t qa = smem_u32(qs + (size_t)(lane & 15) * ldk + (lane >> 4) * 8);
-    const uint32_t ka = smem_u32(kt + (size_t)(kw * 8 + (lane & 7)) * ldk + (lane >> 3) * 8);
-    int d = half ? mid : 0;
+    // scores of this warp's 8 keys: its strand's chain of sums
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    const int kw = warp & 3, strand = warp >> 2, whole = dkp & ~31;
+    const uint32_t qa = smem_u32(qs + (size_t)(lane & 15) * ldk + strand * 16 + (lane >> 4) * 8);
+    const uint32_t ka = smem_u32(kt + (size_t)(kw * 8 + (lane & 7)) * ldk + strand * 16 + ((lane >> 3) & 1) * 8);
+    const uint32_t ka2 = ka + (lane >> 4) * 64;  // lanes 16 ..: the next 32 columns' piece
+    int d = 0;
 #pragma unroll 3
-    for (; d + 32 <= d_end; d += 32) {
+    for (; d + 64 <= whole; d += 64) {
       uint32_t a[4], b[4], c[4];
       ldmatrix_x4(qa + d * 2, a[0], a[1], a[2], a[3]);
-      ldmatrix_x4(qa + d * 2 + 32, c[0], c[1], c[2], c[3]);
-      ldmatrix_x4(ka + d * 2, b[0], b[1], b[2], b[3]);
-      mma_bf16(s0, a, b[0], b[1]);
-      mma_bf16(s1, c, b[2], b[3]);
+      ldmatrix_x4(qa + d * 2 + 64, c[0], c[1], c[2], c[3]);
+      ldmatrix_x4(ka2 + d * 2, b[0], b[1], b[2], b[3]);
+      mma_bf16(s, a, b[0], b[1]);
+      mma_bf16(s, c, b[2], b[3]);
     }
-    if (d < d_end) {  // 16 columns are left (lanes 16.. read columns that are in the row's padding or the next row: unused)
+    if (d < whole || (strand == 0 && d < dkp)) {  // 32 columns are left, or 16, which are the first strand's (or both, one after the other)
       uint32_t a[4], b[4];
       ldmatrix_x4(qa + d * 2, a[0], a[1], a[2], a[3]);
-      ldmatrix_x4(smem_u32(kt + (size_t)(kw * 8 + (lane & 7)) * ldk + ((lane >> 3) & 1) * 8) + d * 2, b[0], b[1], b[2], b[3]);
-      mma_bf16(s0, a, b[0], b[1]);
+      ldmatrix_x4(ka + d * 2, b[0], b[1], b[2], b[3]);
+      mma_bf16(s, a, b[0], b[1]);
+      if (d < whole && strand == 0 && whole < dkp) {
+        ldmatrix_x4(qa + whole * 2, a[0], a[1], a[2], a[3]);
+        ldmatrix_x4(ka + whole * 2, b[0], b[1], b[2], b[3]);
+        mma_bf16(s, a, b[0], b[1]);
+      }
     }
-    {
-      float* w0 = &sc[half][g0][kw * 8 + (lane & 3) * 2];
-      float* w1 = &sc[half][g1][kw * 8 + (lane & 3) * 2];
-      *reinterpret_cast<float2*>(w0) = make_float2(s0[0] + s1[0], s0[1] + s1[1]);
-      *reinterpret_cast<float2*>(w1) = make_float2(s0[2] + s1[2], s0[3] + s1[3]);
-    }
+    *reinterpret_cast<float2*>(&sc[strand][g0][kw * 8 + (lane & 3) * 2]) = make_float2(s[0], s[1]);
+    *reinterpret_cast<float2*>(&sc[strand][g1][kw * 8 + (lane & 3) * 2]) = make_float2(s[2], s[3]);
     __syncthreads();
-    const int key = t_begin + t * LATM_KEYS + lane;
+    {
+      const int key = t_begin + t * LATM_KEYS + key2;
+      const float2 x = *reinterpret_cast<const float2*>(&sc[0][hd][key2]), y = *reinterpret_cast<const float2*>(&sc[1][hd][key2]);
+      const float s0 = key >= lo && key <= t_end ? (x.x + y.x) * sc2 : -INFINITY;
+      const float s1 = key + 1 >= lo && key + 1 <= t_end ? (x.y + y.y) * sc2 : -INFINITY;
+      float mx = fmaxf(m, fmaxf(s0, s1));
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int hd = 2 * warp + u;
-      const float s = key >= lo && key <= t_end ? (sc[0][hd][lane] + sc[1][hd][lane]) * sc2 : -INFINITY;
-      const float mx = fmaxf(m[u], warp_max(s));  // a tile has a visible key: never -infinity
-      const float corr = exp2f(m[u] - mx), w = exp2f(s - mx);
-      l[u] = l[u] * corr + warp_sum(w);
-      m[u] = mx;
-      pw[hd][lane] = __float2bfloat16_rn(w);
-      if (lane == 0) corr_of[hd] = corr;
+      for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));  // a tile has a visible key: never -infinity
+      const float corr = exp2f(m - mx), w0 = exp2f(s0 - mx), w1 = exp2f(s1 - mx);
+      *reinterpret_cast<uint32_t*>(&pw[hd][key2]) = pack_bf16(w0, w1);
+      float rs = w0 + w1;
+#pragma unroll
+      for (int k = 1; k < 4; ++k) {
+        const float upto = __shfl_up_sync(0xffffffffu, rs, 1);
+        if ((lane & 3) == k) rs = (upto + w0) + w1;
+      }
+      rs += __shfl_xor_sync(0xffffffffu, rs, 4);
+      rs += __shfl_xor_sync(0xffffffffu, rs, 8);
+      l = l * corr + rs;
+      m = mx;
+      if ((lane & 15) == 3) corr_of[hd] = corr;
     }
     __syncthreads();
     const float corr[2] = {corr_of[g0], corr_of[g1]};
@@ -650,9 +660,9 @@ attention_latent_mma_kernel(const bf16* __restrict__ q_lat, const bf16* __restri
   }
   cp_async_wait<0>();
   if (bad_page) atomicOr(status, JLX_STATUS_BAD_PAGE);
-  if (lane < 2) {
-    m_of[2 * warp + lane] = lane ? m[1] : m[0];
-    l_of[2 * warp + lane] = lane ? l[1] : l[0];
+  if ((lane & 15) == 3) {
+    m_of[hd] = m;
+    l_of[hd] = l;
   }
   __syncthreads();
 #pragma unroll
