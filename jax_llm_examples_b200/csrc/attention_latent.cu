@@ -39,8 +39,8 @@ __device__ __forceinline__ void store4(bf16* p, float4 v) {
   o2[1] = __floats2bfloat162_rn(v.z, v.w);
   *reinterpret_cast<uint2*>(p) = o;
 }
-// Bound by a block's chain (row, meeting, write) times the blocks an SM holds: 2048 tokens, latents of 768 and 512: 15 us (18.5 with 4-byte accesses;
-// 11 with each thread's four entries added first, which is another order of the sums).
+// Bound by a block's chain (row, meetings, write) times the blocks an SM holds: 2048 tokens, latents of 768 and 512, timed with the launch:
+// 23 us (27 with 4-byte accesses; 18 with a thread's four entries added first, another order of the sums).
 template <typename TO>
 __global__ void latent_kv_prep_kernel(const float* __restrict__ proj, int splits, long long split_stride,
                                       const float* __restrict__ q_norm_w, const float* __restrict__ kv_norm_w, float eps,
@@ -474,7 +474,8 @@ __global__ void attention_latent_kernel(const float* __restrict__ q_lat, const f
 //            then the four eights), the weights in bfloat16
 //   values   warp w takes the latent's 16-column pieces w, w + 8, ...: the weights times the tile's rows
 // Bound by the latency of a tile's chain and its instructions: with two blocks of 37 KB tiles an SM, eight warps that each
-// did the softmax of all heads took 6 us a tile.  32 requests of 4096 keys, 16 heads: 54 us (81), 32 heads 109 (168).
+// did the softmax of all heads took 6 us a tile.  32 requests of 4096 keys, timed with the launch: 16 heads 69 us (91 with four
+// warps), 32 heads 116 (175).
 // When every served token is its request's only one of the step (`single`), everything but its own row is older than the
 // step: tiles that end below it are asked for before the wait for the predecessor.  Rows outside [lo, t_end] are zeros in shared memory and masked.
 #define LATM_KEYS LAT_TILE
