@@ -933,36 +933,29 @@ __global__ void causal_sink_softmax_kernel(const float* __restrict__ s, const fl
   for (int j = threadIdx.x; j < L; j += blockDim.x) out[j] = from_f32<TO>(j >= first && j < visible ? expf(row[j] * scale - m) / l : 0.f);
 }
 
-// Rows of up to 1024 NV scores on 16-byte boundaries: the visible scores stay in a thread's registers, so every score is read
-// once, exponentiated once and written once, with two meetings of the block.  16 heads, 512 query rows, 3048 keys (100 MB of
-// scores, 50 MB of weights): the four query tiles of a 2048-token portion 113 us, 202 by the general kernel.
+// Rows of up to 256 NV scores: the visible ones stay in the registers of the threads that add them in the kernel above, so every
+// score is read once and exponentiated once.  The same operations and sums per weight.  Bound by its instructions, the divisions
+// first (16 heads, 1024 query rows of 3048 keys, 41 us of bytes: 86 us, 74 with products by 1 / l, which round once more; the
+// kernel above 121).
 template <typename TO, int NV>
 __global__ void __launch_bounds__(256)
-causal_sink_softmax_x4_kernel(const float* __restrict__ s, const float* __restrict__ sink, float scale, int q_start, int k_start, int window,
-                              TO* __restrict__ p, int T, int L) {
+causal_sink_softmax_rows_kernel(const float* __restrict__ s, const float* __restrict__ sink, float scale, int q_start, int k_start, int window,
+                                TO* __restrict__ p, int T, int L) {
   JLX_TL(TL_OTHER);
   __shared__ float scratch[33];
   const int i = blockIdx.x, h = blockIdx.y;
   const float* row = s + ((size_t)h * T + i) * L;
   TO* out = p + ((size_t)h * T + i) * L;
   const int own = q_start + i - k_start, visible = min(L, own + 1), first = window > 0 ? max(0, own - window + 1) : 0;
+  const int j0 = first + threadIdx.x;  // the thread's scores: j0, j0 + 256, ..
   float m = sink ? sink[h] : -INFINITY;
-  float4 x[NV];
+  float x[NV];
+#pragma unroll
+  for (int u = 0; u < NV; ++u) x[u] = j0 + 256 * u < visible ? row[j0 + 256 * u] : 0.f;
 #pragma unroll
   for (int u = 0; u < NV; ++u) {
-    const int j = 4 * (threadIdx.x + 256 * u);
-    x[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (j < visible && j + 3 >= first) x[u] = *reinterpret_cast<const float4*>(row + j);
-  }
-#pragma unroll
-  for (int u = 0; u < NV; ++u) {
-    const int j = 4 * (threadIdx.x + 256 * u);
-    auto seen = [&](int e) { return j + e >= first && j + e < visible; };
-    x[u].x = seen(0) ? x[u].x * scale : -INFINITY;
-    x[u].y = seen(1) ? x[u].y * scale : -INFINITY;
-    x[u].z = seen(2) ? x[u].z * scale : -INFINITY;
-    x[u].w = seen(3) ? x[u].w * scale : -INFINITY;
-    m = fmaxf(m, fmaxf(fmaxf(x[u].x, x[u].y), fmaxf(x[u].z, x[u].w)));
+    x[u] = j0 + 256 * u < visible ? x[u] * scale : -INFINITY;
+    m = fmaxf(m, x[u]);
   }
   m = warp_max(m);
   if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = m;
@@ -973,29 +966,24 @@ causal_sink_softmax_x4_kernel(const float* __restrict__ s, const float* __restri
   float l = 0.f;
 #pragma unroll
   for (int u = 0; u < NV; ++u) {
-    x[u] = make_float4(expf(x[u].x - m), expf(x[u].y - m), expf(x[u].z - m), expf(x[u].w - m));  // not visible: exp(-inf) = 0
-    l += (x[u].x + x[u].y) + (x[u].z + x[u].w);
+    x[u] = expf(x[u] - m);  // not visible: exp(-inf) = 0
+    l += x[u];
   }
   l = block_sum(l, scratch) + (sink ? expf(sink[h] - m) : 0.f);
-  const float by = 1.f / l;
 #pragma unroll
-  for (int u = 0; u < NV; ++u) {
-    const int j = 4 * (threadIdx.x + 256 * u);
-    if (j < L) {
-      alignas(16) const TO v[4] = {from_f32<TO>(x[u].x * by), from_f32<TO>(x[u].y * by), from_f32<TO>(x[u].z * by), from_f32<TO>(x[u].w * by)};
-      if (sizeof(TO) == 2) *reinterpret_cast<uint2*>(out + j) = *reinterpret_cast<const uint2*>(v);
-      else *reinterpret_cast<uint4*>(out + j) = *reinterpret_cast<const uint4*>(v);
-    }
-  }
+  for (int u = 0; u < NV; ++u)
+    if (j0 + 256 * u < visible) out[j0 + 256 * u] = from_f32<TO>(x[u] / l);
+  for (int j = threadIdx.x; j < L; j += 256)
+    if (j < first || j >= visible) out[j] = from_f32<TO>(0.f);
 }
 
 JLX_API int jlx_causal_sink_softmax(const float* s, const float* sink, float scale, int q_start, int k_start, int window, void* p,
                                     int dtype, int H, int T, int L, cudaStream_t stream) {
   JLX_REQUIRE(H > 0 && T >= 0 && L > 0 && q_start >= 0 && k_start >= 0 && k_start <= q_start && window >= 0 && H <= 65535, "causal_sink_softmax: bad sizes");
   if (T == 0) return 0;
-  if ((L & 3) == 0 && L <= 4096 && (((uintptr_t)s | (uintptr_t)p) & 15) == 0) {
+  if (L <= 4096) {
     JLX_DISPATCH_DTYPE(dtype, TO, {
-      const auto kernel = L <= 1024 ? causal_sink_softmax_x4_kernel<TO, 1> : (L <= 2048 ? causal_sink_softmax_x4_kernel<TO, 2> : causal_sink_softmax_x4_kernel<TO, 4>);
+      const auto kernel = L <= 1024 ? causal_sink_softmax_rows_kernel<TO, 4> : (L <= 2048 ? causal_sink_softmax_rows_kernel<TO, 8> : causal_sink_softmax_rows_kernel<TO, 16>);
       kernel<<<dim3(T, H), 256, 0, stream>>>(s, sink, scale, q_start, k_start, window, (TO*)p, T, L);
     });
     JLX_LAUNCH_CHECK("causal_sink_softmax");

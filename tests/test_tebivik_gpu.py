@@ -347,6 +347,26 @@ def test_prompt_softmax_rows_in_registers_and_at_the_edges_of_their_lengths(L, w
             assert not bool(p[:, ~seen].any())
 
 
+@pytest.mark.parametrize("L", [4, 255, 260, 1024, 1027, 2052, 4096])
+@pytest.mark.parametrize("window", [0, 70, 700])
+def test_prompt_softmax_adds_in_one_order_in_both_its_kernels(L, window):
+    """Which kernel runs is a matter of the rows' length: the same scores in longer rows give the same weights to the bit."""
+    from jax_llm_examples_b200.kernels import api as K
+
+    torch.manual_seed(L)
+    H_, T, wide = 2, 9, 4100
+    start = max(0, L - T)
+    s = torch.randn(H_, T, wide, device=DEV) * 4
+    for sink in (None, torch.tensor([0.5, -1.0], device=DEV)):
+        for dtype in (torch.float32, torch.bfloat16):
+            p, longer = torch.empty(H_, T, L, device=DEV, dtype=dtype), torch.empty(H_, T, wide, device=DEV, dtype=dtype)
+            K.causal_sink_softmax(s[..., :L].contiguous(), sink, 0.7, start, p, 0, window)
+            K.causal_sink_softmax(s, sink, 0.7, start, longer, 0, window)
+            rows = range(T) if L >= T else range(L)  # (behind these a longer row shows more keys)
+            for i in rows:
+                assert torch.equal(p[:, i], longer[:, i, :L])
+
+
 @pytest.mark.parametrize("q_rank, rank, dr", [(64, 32, 8), (768, 512, 64), (512, 516, 4), (1536, 96, 0), (1028, 1024, 64)])
 @pytest.mark.parametrize("splits", [1, 2])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
