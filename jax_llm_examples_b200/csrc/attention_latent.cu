@@ -902,7 +902,7 @@ __global__ void causal_sink_softmax_kernel(const float* __restrict__ s, const fl
   const int first = window > 0 ? max(0, own - window + 1) : 0;
   float m = sink ? sink[h] : -INFINITY;
   if (staged) {
-    if ((L & 3) == 0) {  // rows start on 16-byte boundaries
+    if ((L & 3) == 0 && ((uintptr_t)s & 15) == 0) {  // rows start on 16-byte boundaries
       for (int j = (first & ~3) + threadIdx.x * 4; j < visible; j += blockDim.x * 4) {
         float4 v = *reinterpret_cast<const float4*>(row + j);
         v.x *= scale; v.y *= scale; v.z *= scale; v.w *= scale;

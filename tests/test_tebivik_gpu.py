@@ -367,6 +367,19 @@ def test_prompt_softmax_adds_in_one_order_in_both_its_kernels(L, window):
                 assert torch.equal(p[:, i], longer[:, i, :L])
 
 
+@pytest.mark.parametrize("L", [4100, 5000])
+def test_prompt_softmax_of_long_rows_off_16_byte_boundaries(L):
+    """Scores one entry behind a 16-byte boundary, in rows that are read in 16-byte pieces where they start on one."""
+    from jax_llm_examples_b200.kernels import api as K
+
+    torch.manual_seed(L)
+    s = torch.randn(2, 3, L, device=DEV)
+    p, moved = torch.empty_like(s), torch.empty_like(s)
+    K.causal_sink_softmax(s, None, 0.7, L - 50, p, 0, 0)
+    K.causal_sink_softmax(torch.cat([s.new_zeros(1), s.reshape(-1)])[1:].view_as(s), None, 0.7, L - 50, moved, 0, 0)
+    assert torch.equal(p, moved)
+
+
 @pytest.mark.parametrize("q_rank, rank, dr", [(64, 32, 8), (768, 512, 64), (512, 516, 4), (1536, 96, 0), (1028, 1024, 64)])
 @pytest.mark.parametrize("splits", [1, 2])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
