@@ -3,6 +3,7 @@
 from __future__ import annotations
 
 import functools
+import math
 
 import numpy as np
 import torch
@@ -104,8 +105,9 @@ class LatentAttention(InputConvMixer):
     # Scores of a prompt portion are made as one [H, T, L] float32 tensor per query tile; this bounds its size.
     SCORE_TILE_BYTES = 1 << 30
     # Query rows of a portion per score product: a tile computes the keys above its own diagonal in vain, and a tile that is too
-    # small leaves the GPU waiting for its four launches (about 40 us of the host's time).  Tiles of 2^26 scores, at least 512 rows:
-    # 16 heads, 2048 tokens at position 1000, 340 us in two tiles, 460 in four of 512.
+    # small leaves the GPU waiting for its four launches (about 40 us of the host's time).  Tiles of 2^26 scores, at least 512 rows;
+    # behind a window, where the keys in vain are as many again, of 2^25.  2048 tokens at position 1000, us, against tiles of 512:
+    # 16 heads 470 (520), with a window of 1024 414 (494); 32 heads 776 (778), with windows of 128 476 (530), of 1024 615 (615).
     QUERY_TILE, TILE_SCORES = 512, 1 << 26
     MIN_SPLIT_KEYS = 64
     SPLIT_ROUNDS = 2  # blocks per multiprocessor that the key ranges of a decode step aim at
@@ -134,6 +136,17 @@ class LatentAttention(InputConvMixer):
                            self.scale, ctx.status, rows, n_rows, splits, split_keys, part_acc, part_ml, self.window or 0,
                            single_tokens=rows is not None or ctx.max_q_len == 1)
 
+    def _query_tile(self, T: int, L: int) -> int:
+        """Query rows per score product for T tokens over L keys."""
+        H, W = self.heads, self.window
+        rows = self.TILE_SCORES // (H * L)
+        if W is not None and W < L:  # a tile of t rows sees t + W keys
+            rows = min(rows, (math.isqrt(W * W + 2 * self.TILE_SCORES // H) - W) // 2)
+        if rows <= self.QUERY_TILE:
+            return max(16, min(self.QUERY_TILE, self.SCORE_TILE_BYTES // (4 * H * L)))
+        rows = -(-T // -(-T // rows))  # of about equal sizes, in whole row tiles of the products
+        return -(-rows // 128) * 128
+
     def _portion(self, ctx: StepContext, cache: LayerCache, r: int, n0: int, T: int, start: int, q_full, rows_out, gate) -> None:
         """One request's prompt portion (rows n0 .. n0 + T, positions start ..) on the tensor cores: the request's cached
         rows gathered, every head's keys and values up-projected from them (the library's product), scores and weighted
@@ -155,8 +168,7 @@ class LatentAttention(InputConvMixer):
         v = kv_up[:, H * dn:].unflatten(1, (H, dv)).permute(1, 0, 2)  # [H, L, dv], a view
         # query tiles: each sees the keys from its first row's window to its own last row only (the rest of the causal
         # triangle is not computed)
-        tile = max(16, min(max(self.QUERY_TILE, self.TILE_SCORES // (H * L)), self.SCORE_TILE_BYTES // (4 * H * L)))
-        tile = -(-T // -(-T // tile))  # of equal sizes
+        tile = self._query_tile(T, L)
         for t0 in range(0, T, tile):
             t1 = min(T, t0 + tile)
             lo = 0 if self.window is None else max(0, start + t0 - self.window + 1 - k0) // 8 * 8

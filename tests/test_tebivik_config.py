@@ -105,3 +105,17 @@ def test_plain_implementation_is_causal_and_its_parts_reduce_as_they_should(tmp_
     r = plain.rotate_pairs(v, torch.tensor([0, 1, 2, 3]), 100.0, 6)
     assert torch.allclose(r[0], v[0]) and torch.allclose(r[..., 6:], v[..., 6:])
     assert torch.allclose(r[..., 0:2].norm(dim=-1), v[..., 0:2].norm(dim=-1))
+
+
+def test_query_tiles_of_a_latent_prompt():
+    """Few heads and keys: large tiles of about equal sizes; many, or a window that a large tile mostly computes in vain: 512 rows as
+    long as the scores' bytes allow."""
+    import types
+
+    from jax_llm_examples_b200.parts import LatentAttention as A
+
+    for heads, window, T, L, want in ((16, None, 2048, 3048, 1024), (32, None, 2048, 3048, 768), (64, None, 2048, 3048, 512), (16, 1024, 2048, 3072, 1024),
+                                      (32, 1024, 2048, 3072, 512), (32, 128, 2048, 2176, 768), (32, 4096, 2048, 3048, 768), (16, None, 20, 100000, 20),
+                                      (128, None, 2048, 18432, 113), (128, None, 64, 1 << 20, 16), (16, None, 700, 3704, 700)):
+        part = types.SimpleNamespace(heads=heads, window=window, TILE_SCORES=A.TILE_SCORES, QUERY_TILE=A.QUERY_TILE, SCORE_TILE_BYTES=A.SCORE_TILE_BYTES)
+        assert min(T, A._query_tile(part, T, L)) == want, (heads, window, T, L)
