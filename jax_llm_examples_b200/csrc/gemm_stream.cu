@@ -151,6 +151,7 @@ struct StreamArgs {
   int splits;
   int k_per_split;       // multiple of BK
   int offsets_settled;   // grouped: offsets and tile list were complete before the kernel in front of this one began its work
+  int weight_first;      // grouped: all token tiles of a weight tile before the next weight tile
   int* status;
 };
 
@@ -229,9 +230,12 @@ __device__ __forceinline__ void stream_epilogue(const StreamArgs& args, int warp
 }
 
 // The blocks of a group of several token tiles in another order than the grid's: all token tiles of one weight tile, then the
-// next weight tile, so that the group's weights (more than L2 holds) come from memory once and not once per token tile.  x:
-// the weight tile of `xs`; row_lo: the first row of the token tile; both are replaced.  16 groups of 512 rows, 16384 x 5120:
-// 1040 us (1085); of 100 to 924 rows 1200 (1271); a prompt of 2048 tokens over 4 experts 2.80 ms (2.84).
+// next weight tile, so that the group's weights come from memory once and not once per token tile.  x: the weight tile of `xs`;
+// row_lo: the first row of the token tile; both are replaced.  Only for groups whose weights are more than L2 holds (L2_BYTES):
+// smaller ones stay there from tile to tile, and the grid's order leaves its short last tiles to the end.  Times over the grid's,
+// 4 and 16 groups, 512 to 8192 rows in all: 16384 x 5120 (168 MB) 0.90 to 1.00; 14336 x 4096 (117 MB) 0.96 to 1.04; 5120 x 8192
+// (84 MB) 1.00 to 1.09; 8192 x 2048 (34 MB) 0.99 to 1.13.
+#define L2_BYTES (126ll << 20)
 template <int BT>
 __device__ __forceinline__ void weight_tile_first(int& x, int xs, int group_lo, int& row_lo, int row_hi) {
   const int tiles = (row_hi - group_lo + BT - 1) / BT;
@@ -295,7 +299,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       t -= tiles;
     }
     if (!found) return;
-    if (BT > 64) weight_tile_first<BT>(x, gridDim.x, group_lo, row_lo, row_hi);  // (narrow tiles: decode steps, one tile a group)
+    if (BT > 64 && args.weight_first) weight_tile_first<BT>(x, gridDim.x, group_lo, row_lo, row_hi);  // (narrow tiles: decode steps, one tile a group)
   } else if (args.uniform) {
     const int per_group = (args.uniform + BT - 1) / BT;
     group = blockIdx.y / per_group;
@@ -455,7 +459,7 @@ gemm_stream_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
       t -= tiles;
     }
     if (!found) return;
-    weight_tile_first<BT>(x, gridDim.x >> 1, group_lo, row_lo, row_hi);
+    if (args.weight_first) weight_tile_first<BT>(x, gridDim.x >> 1, group_lo, row_lo, row_hi);
   } else if (args.uniform) {
     const int per_group = (args.uniform + BT - 1) / BT;
     group = blockIdx.y / per_group;
@@ -700,6 +704,7 @@ JLX_API int jlx_gemm_stream(const void* A, const void* W, void* out, int out_is_
   a.out_is_f32 = out_is_f32; a.silu = mode == 2; a.glu_alpha = glu_alpha; a.glu_limit = glu_limit; a.glu_shift = glu_shift; a.splits = splits; a.k_per_split = kps; a.status = status;
   a.act = mode == 3 ? act : 0;
   a.offsets_settled = offsets && offsets_settled;
+  a.weight_first = offsets && (long long)N * K * (long long)sizeof(bf16) > L2_BYTES;
   // Row tiles to launch blocks for.  Grouped: a group of r rows has ceil(r / bt) <= r / bt + 1 tiles and only a group
   // with rows has any, so there are at most rows / bt + min(E, rows) of them.  (A looser bound costs time: a block
   // without a tile returns at once, but with the kernel's shared memory only two blocks fit an SM at a time, and with

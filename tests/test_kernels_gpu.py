@@ -1071,3 +1071,27 @@ def test_grouped_product_whose_groups_have_several_token_tiles(N, hint, listed):
         lo, hi = int(off[e]), int(off[e + 1])
         if hi > lo:
             close(out[lo:hi], a[lo:hi].double() @ w[e].double().T, 1e-5)
+
+
+@pytest.mark.parametrize("N", [33280, 33408])  # pairs of blocks, and one block per weight tile: 130 and 130.5 pairs of weight tiles
+@pytest.mark.parametrize("listed", [False, True])
+def test_grouped_product_whose_weights_outgrow_l2(N, listed):
+    """Groups of 136 MB of weights go through the weight tiles first: every row of every group, of several token tiles, one or
+    none, comes out once.  32-bit sums of 2048 products."""
+    api = K()
+    sizes, Kd, hint = [300, 0, 16, 101], 2048, 100
+    off = torch.tensor([0] + list(np.cumsum(sizes)), device=DEV, dtype=torch.int32)
+    rows, E, st = sum(sizes), len(sizes), status()
+    a, w = torch.randn(rows, Kd, device=DEV).bfloat16(), torch.randn(E, N, Kd, device=DEV).bfloat16()
+    tiles = None
+    if listed:
+        bt = api.gemm_stream_token_tile(hint)
+        found = [(e, int(off[e]) + r) for e, n in enumerate(sizes) for r in range(0, n, bt)]
+        tiles = (torch.tensor(found, device=DEV, dtype=torch.int32).reshape(-1), torch.tensor([len(found)], device=DEV, dtype=torch.int32))
+    out = torch.full((rows, N), float("nan"), device=DEV)
+    api.gemm_stream(a, w, out, st, offsets=off, rows_hint=hint, tiles=tiles)
+    assert int(st) == 0
+    for e in range(E):
+        lo, hi = int(off[e]), int(off[e + 1])
+        if hi > lo:
+            close(out[lo:hi], a[lo:hi].float() @ w[e].float().T, 1e-5)
