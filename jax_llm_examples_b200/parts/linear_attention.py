@@ -14,14 +14,14 @@ from ..kernels import api as K
 from ..tracing import scope
 from .base import LayerCache, Mixer, ProjectedMixer, Rows, StateNeed, StepContext, as_rows, register_part
 from .linear import grouped_linear, linear
-from .recurrent import plan_scan_chunks, scan_chunks
+from .recurrent import decay_chunks_pay, plan_scan_chunks, scan_chunks
 
 
 def _scan(ctx: StepContext, q, k, v, z, z_bias, form: str, tau: float, q_scale: float, bonus, state, heads: int, dk: int, dv: int,
           read_after_update: bool, **prep) -> torch.Tensor:
     """The recurrence over the step's tokens from projected rows (views); returns o float32 [N, H, dv]."""
     n, dev = ctx.n_tokens, state.device
-    chunks, scratch = scan_chunks(ctx, heads, dk, dv)
+    chunks, scratch = scan_chunks(ctx, heads, dk, dv, decay_chunks_pay)
     walks = chunks is None or chunks.others
     # where the chunk kernels serve all requests, operands that need no arithmetic are read where they were projected
     whole = not walks and K.decay_prep_selective(q, k, v, z, z_bias, dk, dv, prep.get("rot_dims", 0))

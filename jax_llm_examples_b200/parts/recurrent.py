@@ -62,10 +62,16 @@ def plan_scan_segments(shape: StepShape) -> dict:
     return {"scan_segments": np.array(segs, dtype=np.int32).reshape(-1, 4)}
 
 
-# Portions of at least so many tokens go through the chunk kernels (three launches of 50 us together at 16 heads, then
+# Portions of at least so many tokens may go through the chunk kernels (three launches of 50 us together at 16 heads, then
 # 65 ns per token; the walk: 145 ns per token and no start).  Measured, us, walk and chunks: 16 heads 256 tokens 46 and 50,
 # 512 tokens 81 and 52, 2048 tokens 297 and 144; 32 heads 512 tokens 108 and 81; 8 requests of 256 tokens, 32 heads, 288 and 290.
 CHUNK_FROM_TOKENS = 384
+# The chunk kernels work on 128 x 128 whatever a head's sizes, the decayed walk on what there is, over more heads and requests at
+# once: from heads of this area on chunks are ahead at any number of heads and requests (112 x 112, 8 to 64 heads, 1 to 16 requests of
+# 384 to 2048 tokens: 0.32 to 1.02 of the walk's time); smaller ones take them for portions from CHUNK_FROM_SMALL on that are
+# worth up to CHUNK_CHAINS heads of the longest (72 x 72 and 96 x 96, 8 to 32 heads: 0.29 to 0.98); beyond, 72 x 72 took 0.97 to
+# 1.73 of the walk's time at 2 to 16 requests of 32 to 64 heads, and 96 x 96 0.87 to 1.31.
+CHUNK_AREA, CHUNK_FROM_SMALL, CHUNK_CHAINS = 112 * 112, 512, 32
 
 
 def plan_scan_chunks(shape: StepShape) -> dict:
@@ -93,10 +99,17 @@ def step_chunks(ctx: StepContext) -> "K.Chunks | None":
     return K.Chunks(chunks, requests, chunks.numel() // 3, m, CHUNK_FROM_TOKENS, m < ctx.n_requests)
 
 
-def scan_chunks(ctx: StepContext, heads: int, dk: int, dv: int) -> "tuple[K.Chunks | None, torch.Tensor | None]":
-    """The step's chunks and the scratch of their states, if it has long portions of heads that the chunk kernels take."""
+def decay_chunks_pay(lens, heads: int, dk: int, dv: int) -> bool:
+    """Whether a step's long portions go through the chunk kernels rather than the decayed recurrences' walk (see CHUNK_AREA)."""
+    long = [n for n in lens if n >= CHUNK_FROM_TOKENS]
+    return dk * dv >= CHUNK_AREA or (max(long) >= CHUNK_FROM_SMALL and heads * sum(long) <= CHUNK_CHAINS * max(long))
+
+
+def scan_chunks(ctx: StepContext, heads: int, dk: int, dv: int, pays=None) -> "tuple[K.Chunks | None, torch.Tensor | None]":
+    """The step's chunks and the scratch of their states, if it has long portions of heads that the chunk kernels take, and if
+    ``pays(lengths, heads, dk, dv)`` says so."""
     chunks = step_chunks(ctx)
-    if chunks is None or not K.chunk_scan_supported(dk, dv):
+    if chunks is None or not K.chunk_scan_supported(dk, dv) or (pays is not None and not pays(ctx.host_q_lens, heads, dk, dv)):
         return None, None
     need = K.chunk_scan_scratch(chunks.n, heads, dk, dv)
     return chunks, ctx.workspace.get("chunk_scan", need, torch.float32) if ctx.workspace is not None else \

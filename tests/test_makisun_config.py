@@ -172,3 +172,13 @@ def test_plain_router_takes_the_softmax_over_the_chosen_only():
         wgt = torch.exp(zz) / torch.exp(zz).sum()
         ref = sum(wgt[j] * plain.expert(h[t:t + 1], P, f"m.e{int(chosen[t, j])}.")[0] for j in range(2))
         assert torch.allclose(out[t], ref)
+
+
+def test_which_long_portions_go_by_chunks():
+    """Heads near 128 x 128 always; smaller ones while the portions are worth few heads of the longest."""
+    from jax_llm_examples_b200.parts.recurrent import decay_chunks_pay
+
+    for lens, heads, dk, dv, chunks in (([384], 64, 128, 128, True), ([384] * 16, 64, 112, 112, True), ([2048, 1, 300], 16, 72, 72, True),
+                                        ([511], 8, 72, 72, False), ([512], 32, 96, 96, True), ([512], 33, 96, 96, False), ([384] * 5, 32, 72, 72, False),
+                                        ([1024] * 4, 8, 128, 72, True), ([1024] * 4, 16, 72, 128, False), ([777, 500, 600], 16, 72, 72, False)):
+        assert decay_chunks_pay(lens, heads, dk, dv) == chunks, (lens, heads, dk, dv)
