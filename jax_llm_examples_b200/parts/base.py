@@ -22,6 +22,7 @@ from __future__ import annotations
 import dataclasses
 from typing import Any, Callable
 
+import numpy as np
 import torch
 
 from ..cache.manager import Retention
@@ -240,12 +241,15 @@ class StepContext:
 
     def plan_with(self, planners, page_size: int) -> None:
         """Runs step planners for a context made by hand (a test of one part): what the engine does while it
-        packs a step, with one small copy per array instead of the descriptor's single one."""
-        shape = StepShape(tuple(self.host_q_lens), tuple(self.host_q_start), page_size, self.max_kv_len)
+        packs a step; the arrays travel in one copy, as they do there."""
+        shape, made = StepShape(tuple(self.host_q_lens), tuple(self.host_q_start), page_size, self.max_kv_len), {}
         for planner in planners:
-            for name, a in planner(shape).items():
-                self.host_arrays[name] = a
-                self.arrays[name] = torch.tensor(a.tolist(), dtype=torch.int32).reshape(-1).to(self.token_ids.device)
+            made.update(planner(shape))
+        self.host_arrays.update(made)
+        if made:
+            flat = [np.asarray(a, dtype=np.int32).reshape(-1) for a in made.values()]
+            on_device = torch.from_numpy(np.concatenate(flat)).to(self.token_ids.device)
+            self.arrays.update(zip(made, on_device.split([a.size for a in flat])))
 
 
 @dataclasses.dataclass(frozen=True)
