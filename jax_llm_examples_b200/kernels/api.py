@@ -1010,6 +1010,8 @@ def attention_f32(q: torch.Tensor, pages: torch.Tensor, block_table: torch.Tenso
          c_int(keep), c_float(attn_scale), c_float(floor_scale), _ptr(sink), _ptr(slopes), c_float(softcap), _ptr(items), _ptr(rows),
          c_int(n_items), c_int(max_count), c_int(splits), c_int(per_split), c_int(int(part_rows < N)), _ptr(part_o), _ptr(part_ml),
          _ptr(status), _stream())
+    global _launches
+    _launches += int(splits > 1)  # the combine kernel
 
 
 def _check_sink(sink: torch.Tensor | None, Hq: int, what: str = "sink") -> None:
@@ -1301,3 +1303,5 @@ def sample(logits: torch.Tensor, out: torch.Tensor, temperature: torch.Tensor | 
     scratch = torch.empty(_sample_scratch(M, V), dtype=torch.uint8, device=logits.device)
     _run("sampling", "jlx_sample", _ptr(logits), c_int(M), c_int(V), c_longlong(V), _ptr(temperature), _ptr(top_k),
          _ptr(streams), _ptr(counters), c_ulonglong(seed & 0xFFFFFFFFFFFFFFFF), _ptr(out), _ptr(scratch), _stream())
+    global _launches
+    _launches += 1 + int(temperature is not None)  # the chunks' largest, (the spans' sums,) the choice

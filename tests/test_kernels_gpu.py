@@ -1095,3 +1095,19 @@ def test_grouped_product_whose_weights_outgrow_l2(N, listed):
         lo, hi = int(off[e]), int(off[e + 1])
         if hi > lo:
             close(out[lo:hi], a[lo:hi].float() @ w[e].float().T, 1e-5)
+
+
+def test_calls_of_several_launches_count_them_all():
+    """The sampler's three kernels (two without temperatures), and the 32-bit attention's merging of key ranges."""
+    n = K().launch_count()
+    logits, out = torch.randn(3, 1000, device=DEV), torch.empty(3, device=DEV, dtype=torch.int32)
+    K().sample(logits, out)
+    assert K().launch_count() - n == 2
+    ones = torch.ones(3, device=DEV, dtype=torch.int64)
+    K().sample(logits, out, ones.float(), ones.int(), ones, ones)
+    assert K().launch_count() - n == 5
+    q, pages, bt, req, pos, _, _ = _paged_case(torch.float32, 2, 1, 64, 16, [300], [1])
+    for splits, launches in ((1, 6), (2, 8)):
+        K().attention_f32(q, pages, bt, req, pos, torch.empty_like(q), 0.125, 0, 0, 0.0, 1.0, status(), 1, splits=splits, per_split=1,
+                          part_o=torch.empty(2 * 2 * 64, device=DEV), part_ml=torch.empty(2 * 2 * 2, device=DEV))
+        assert K().launch_count() - n == launches
