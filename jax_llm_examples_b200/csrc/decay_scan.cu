@@ -226,7 +226,11 @@ __global__ void decay_prep_kernel(RowsView q, RowsView k, RowsView v, RowsView z
 // rotation's sines and cosines made once per token instead of once per head.  Outputs that are null are left out: a caller
 // that can read q, k or v where they were projected needs no copy of them.  The same operations per value.
 // 2048 tokens, 16 heads of 128, the decay alone: 10 us (all four outputs, a block per token and head: 63).
+// A block's chain is longer than the other kernel's (several pieces per thread, partial sums one after the other), so it pays once
+// the tokens fill the GPU: 16 heads, all outputs, us, here and there: 1 token 5.1 and 3.2 (from 8 partial sums 7.2 and 3.3), 64 tokens
+// 5.5 and 3.4, 256 tokens 7.5 and 7.7 (from 8 partial sums 14.3 and 10.0), 512 tokens 8.7 and 13.1.
 #define PREP_MAX_ROT 512
+#define PREP_ROWS_FROM 257
 __global__ void __launch_bounds__(256)
 decay_prep_x4_kernel(RowsView q, RowsView k, RowsView v, RowsView z, const float* __restrict__ z_bias, int mode, float inv_tau, float q_scale,
                      float* __restrict__ qo, float* __restrict__ ko, float* __restrict__ d_out, float* __restrict__ vo, int H, int dk, int dv,
@@ -297,7 +301,8 @@ JLX_API int jlx_decay_prep(const RowsView* q, const RowsView* k, const RowsView*
   if (!z) z = &none;
   if (N == 0) return 0;
   const float inv_tau = mode == DECAY_SIGMOID_POWER ? 1.f / tau : 0.f;
-  if (jlx_decay_prep_selective(q, k, v, z, z_bias, dk, dv, rot) && on16(qo) && on16(ko) && on16(d_out) && on16(vo)) {
+  if ((N >= PREP_ROWS_FROM || !qo || !ko || !vo) && jlx_decay_prep_selective(q, k, v, z, z_bias, dk, dv, rot) && on16(qo) && on16(ko) && on16(d_out) &&
+      on16(vo)) {
     JLX_CUDA(jlx_launch_pdl(decay_prep_x4_kernel, dim3(N), dim3(256), 0, stream, *q, *k, *v, *z, z_bias, mode, inv_tau, q_scale, qo, ko, d_out, vo, H,
                             dk, dv, head_decay, k_scale, inv_freq, rot, positions));
     JLX_LAUNCH_CHECK("decay_prep");
@@ -549,7 +554,10 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, const float* 
 }
 
 // Heads of up to 256 columns: one warp per (token, head), 32 columns per access, no barrier.  The squares are added as the block
-// of W warps above adds them, so the results are the same.  2048 tokens, 16 heads of 128: 22 us (28).
+// of W warps above adds them, so the results are the same.  2048 tokens, 16 heads of 128: 18 us (24).  With few of them the block's
+// shorter chain is ahead: 1 to 64 tokens of 16 heads 3.7 to 4.1 us here, 3.2 to 3.4 there; 4096 heads in all 6.2 and 5.2, 6400 5.3
+// and 6.8.
+#define NORM_WARPS_FROM 4097
 template <typename T, int W, int NV>
 __global__ void __launch_bounds__(256)
 head_norm_gate_warp_kernel(const float* __restrict__ o, const float* __restrict__ weight, int per_head, RowsView gate, float eps, float mult,
@@ -594,7 +602,7 @@ JLX_API int jlx_head_norm_gate(const float* o, const float* weight, int per_head
   if (N == 0) return 0;
   RowsView none = {nullptr, 0, 0, 1, 0};
   const int threads = dv > 128 ? 128 : (dv > 32 ? 64 : 32);
-  if (dv <= 256 && (long long)N * H < (1ll << 31)) {
+  if (dv <= 256 && (long long)N * H >= NORM_WARPS_FROM && (long long)N * H < (1ll << 31)) {
     JLX_DISPATCH_DTYPE(out_dtype, T, {
       JLX_CUDA(jlx_launch_pdl(dv <= 32 ? head_norm_gate_warp_kernel<T, 1, 1> : (dv <= 128 ? head_norm_gate_warp_kernel<T, 2, 4> : head_norm_gate_warp_kernel<T, 4, 8>),
                               dim3((N * H + 7) / 8), dim3(256), 0, stream, o, weight, per_head, gate ? *gate : none, eps, mult, (T*)out, ld_out, N * H, H, dv));

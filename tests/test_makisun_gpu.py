@@ -272,6 +272,38 @@ def test_chunk_scan_keeps_what_is_not_finite_from_earlier_tokens(form, what):
                 _close(got[sound], ref[sound], 5e-6, f"{what} of token {at}")
 
 
+@pytest.mark.parametrize("splits", [1, 3])
+@pytest.mark.parametrize("form", ["double_exp", "head_constant"])
+def test_few_rows_and_many_are_prepared_and_normed_alike(form, splits):
+    """Steps of few tokens take other kernels of the decays' preparation and of the heads' norm than steps of many: the same rows
+    give the same numbers to the bit on both sides of both borders."""
+    from jax_llm_examples_b200.kernels import api as K
+
+    torch.manual_seed(splits)
+    H_, d = 16, 64
+    N, F = 300, 4 * H_ * d
+    rows, decays = torch.randn(splits, N, F, device=DEV), torch.randn(splits, N, H_ * d, device=DEV)
+    bias, const, freq = torch.randn(H_ * d, device=DEV), torch.rand(H_, device=DEV), torch.rand(16, device=DEV)
+    o, weight = torch.randn(N, H_, d, device=DEV), torch.rand(d, device=DEV)
+
+    def run(n):
+        x, z = rows[:, :n].contiguous(), decays[:, :n].contiguous()
+        view = lambda t, c=0: K.rows_view(t if splits > 1 else t[0], splits, c)  # noqa: E731
+        q, k, dec, v = (torch.full((n, H_, d), float("nan"), device=DEV) for _ in range(4))
+        more = dict(head_decay=const, k_scale=0.3, inv_freq=freq, rot_dims=32, positions=torch.arange(n, device=DEV, dtype=torch.int32)) \
+            if form == "head_constant" else {}
+        K.decay_prep(view(x), view(x, H_ * d), view(x, 2 * H_ * d), None if more else view(z), None if more else bias, form, 1.0, 0.7, q, k, dec, v,
+                     H_, d, d, **more)
+        out = torch.empty(n, H_ * d, device=DEV)
+        K.head_norm_gate(o[:n].contiguous(), weight, False, view(x, 3 * H_ * d), 1e-5, 1.0, out)
+        return q, k, dec, v, out
+
+    many = run(N)
+    for n in (1, 7, 255, 256, 257):
+        for few, whole in zip(run(n), many):
+            assert torch.equal(few, whole[:n]), n
+
+
 def test_decay_forms():
     """exp(-exp(z + b)) and sigmoid(z + b)^(1 / tau) in 32-bit, also far out in both tails; q is scaled, k and v pass."""
     from jax_llm_examples_b200.kernels import api as K
