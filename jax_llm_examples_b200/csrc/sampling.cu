@@ -560,10 +560,12 @@ JLX_API int jlx_sample_max_top_k() { return SAMPLE_MAX_K; }
 
 // Chunks of a row for sample_top_kernel.  At most SAMPLE_STRAND values per thread (the bound of its candidate list).  8 from
 // 16 rows on: 64 rows are then 512 blocks, all resident at once (four an SM).  16 below, where blocks are few: one row of
-// 202048, top 64, takes 24 us of which three launches' latency is most.
+// 202048, top 64, takes 24 us of which three launches' latency is most.  At least four values per thread: more lists than that
+// only lengthen the merging.
 static int sample_chunk(int M, int V) {
   const int chunks = M < 16 ? 16 : 8;
-  const int size = ((V + chunks - 1) / chunks + 3) / 4 * 4;
+  int size = ((V + chunks - 1) / chunks + 3) / 4 * 4;
+  if (size < 4 * SAMPLE_THREADS) size = 4 * SAMPLE_THREADS;
   const int most = SAMPLE_THREADS * (SAMPLE_STRAND - 4);  // whole vectors, and one of the last 1..3 values, per thread
   return size < most ? size : most;
 }
