@@ -487,14 +487,13 @@ JLX_API int jlx_chunk_scan(const float* q, long long ldq, const float* k, long l
   const int smem_states = (int)sizeof(float) * (2 * CHUNK * CH_LD + CHUNK * CH_D);
   const int smem_out = (int)sizeof(float) * (3 * CHUNK * CH_LD + 10 * PIECE * PIECE + (CHUNK / PIECE - 1) * CH_D);  // two blocks an SM
   JLX_CUDA(cudaFuncSetAttribute(chunk_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_states));
-  JLX_CUDA(cudaFuncSetAttribute(chunk_outputs_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_out));
-  JLX_CUDA(cudaFuncSetAttribute(chunk_outputs_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_out));
+  const auto outputs = read_after ? chunk_outputs_kernel<true> : chunk_outputs_kernel<false>;
+  JLX_CUDA(cudaFuncSetAttribute(outputs, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_out));
   chunk_states_kernel<<<dim3(n, H), CH_THREADS, smem_states, stream>>>(P);
   JLX_LAUNCH_CHECK("chunk_states");
   chunk_chain_kernel<<<dim3((unsigned)(((size_t)H * dk * dv + 255) / 256), m), 256, 0, stream>>>(P);
   JLX_LAUNCH_CHECK("chunk_chain");
-  if (read_after) chunk_outputs_kernel<true><<<dim3(n, H), CH_THREADS, smem_out, stream>>>(P);
-  else chunk_outputs_kernel<false><<<dim3(n, H), CH_THREADS, smem_out, stream>>>(P);
+  outputs<<<dim3(n, H), CH_THREADS, smem_out, stream>>>(P);
   JLX_LAUNCH_CHECK("chunk_outputs");
   return 0;
 }

@@ -640,14 +640,6 @@ def decay_prep_selective(q: _RowsView, k: _RowsView, v: _RowsView, z: _RowsView 
                                                               _ptr(z_bias), c_int(dk), c_int(dv), c_int(rot_dims)))
 
 
-def view_rows(v: _RowsView, n: int, heads: int, size: int) -> torch.Tensor:
-    """The rows behind a view of whole projected rows (not split-K partials), as [n, heads, size]."""
-    if v.splits > 1:
-        raise KernelError("split-K partials are no rows yet")
-    flat = v.keep.view(-1)
-    return flat.as_strided((n, heads, size), (v.ld, size, 1), flat.storage_offset() + (v.p - flat.data_ptr()) // 4)
-
-
 def decay_scan(q: torch.Tensor, k: torch.Tensor, d: torch.Tensor, v: torch.Tensor, bonus: torch.Tensor | None, state: torch.Tensor,
                cu_q: torch.Tensor, slot_ids: torch.Tensor, o: torch.Tensor, read_after_update: bool, skip_from: int = 0) -> None:
     """S <- diag(d_t) S + k_t v_t^T over each request's tokens, in order.  ``read_after_update``: o_t = S_t^T q_t; else
@@ -691,25 +683,36 @@ def chunk_scan_scratch(n: int, heads: int, dk: int, dv: int) -> int:
     return n * heads * dk * (dv + 1)
 
 
-def chunk_scan(q: torch.Tensor, k: torch.Tensor | None, d: torch.Tensor, v: torch.Tensor, bonus: torch.Tensor | None, state: torch.Tensor,
-               slot_ids: torch.Tensor, o: torch.Tensor, read_after_update: bool, chunks: Chunks, scratch: torch.Tensor) -> None:
+def _chunk_rows(t: "torch.Tensor | _RowsView | None", n: int, heads: int, size: int) -> tuple:
+    """(address, row stride) of one operand of ``chunk_scan``."""
+    if t is None:
+        return None, c_longlong(0)
+    if isinstance(t, _RowsView):
+        if t.splits > 1:
+            raise KernelError("chunk_scan: split-K partials are no rows yet")
+        return c_void_p(t.p), c_longlong(t.ld)
+    if t.dtype != torch.float32 or t.shape != (n, heads, size) or t.stride()[1:] != (size, 1):
+        raise KernelError("chunk_scan: operands are float32 [N, H, size] with heads side by side in a row")
+    return _ptr(t), c_longlong(t.stride(0))
+
+
+def chunk_scan(q: "torch.Tensor | _RowsView", k: "torch.Tensor | _RowsView | None", d: "torch.Tensor | _RowsView", v: "torch.Tensor | _RowsView",
+               bonus: torch.Tensor | None, state: torch.Tensor, slot_ids: torch.Tensor, o: torch.Tensor, read_after_update: bool, chunks: Chunks,
+               scratch: torch.Tensor) -> None:
     """:func:`decay_scan` for the requests of ``chunks`` (three launches).  q, k, d, v: float32 [N, H, size] whose rows may be
-    wider than H * size; k None: k = 1 - d.  scratch: float32 of ``chunk_scan_scratch`` elements."""
+    wider than H * size, or views of projected rows (``rows_view``, no partials); k None: k = 1 - d.  scratch: float32 of
+    ``chunk_scan_scratch`` elements."""
     global _launches
     _contig(bonus, state, o, scratch)
-    N, H, dk = q.shape
-    dv = v.shape[2]
-    for t, size in ((q, dk), (k, dk), (d, dk), (v, dv)):
-        if t is not None and (t.dtype != torch.float32 or tuple(t.shape) != (N, H, size) or t.stride(2) != 1 or t.stride(1) != size):
-            raise KernelError("chunk_scan: operands are float32 [N, H, size] with heads side by side in a row")
-    if any(t.dtype != torch.float32 for t in (state, o, scratch)) or (bonus is not None and (bonus.dtype != torch.float32 or bonus.numel() != H * dk)):
+    (N, H, dv), dk = o.shape, state.shape[2]
+    if state.dtype != torch.float32 or o.dtype != torch.float32 or scratch.dtype != torch.float32 or (
+            bonus is not None and (bonus.dtype != torch.float32 or bonus.numel() != H * dk)):
         raise KernelError("chunk_scan: everything is float32")
-    if tuple(state.shape[1:]) != (H, dk, dv) or tuple(o.shape) != (N, H, dv) or scratch.numel() < chunk_scan_scratch(chunks.n, H, dk, dv):
-        raise KernelError(f"chunk_scan: shapes do not fit: q {tuple(q.shape)}, v {tuple(v.shape)}, state {tuple(state.shape)}")
-    ld = lambda t: c_longlong(t.stride(0) if t is not None else 0)  # noqa: E731
-    _run("chunk_scan", "jlx_chunk_scan", _ptr(q), ld(q), _ptr(k), ld(k), _ptr(d), ld(d), _ptr(v), ld(v), _ptr(bonus), _ptr(state), _ptr(slot_ids),
-         _ptr(o), _ptr(chunks.chunks), c_int(chunks.n), _ptr(chunks.requests), c_int(chunks.m), c_int(H), c_int(dk), c_int(dv),
-         c_int(int(read_after_update)), _ptr(scratch), _stream())
+    if state.shape[1:] != (H, dk, dv) or scratch.numel() < chunk_scan_scratch(chunks.n, H, dk, dv):
+        raise KernelError(f"chunk_scan: shapes do not fit: state {tuple(state.shape)}, o {tuple(o.shape)}")
+    _run("chunk_scan", "jlx_chunk_scan", *_chunk_rows(q, N, H, dk), *_chunk_rows(k, N, H, dk), *_chunk_rows(d, N, H, dk), *_chunk_rows(v, N, H, dv),
+         _ptr(bonus), _ptr(state), _ptr(slot_ids), _ptr(o), _ptr(chunks.chunks), c_int(chunks.n), _ptr(chunks.requests), c_int(chunks.m), c_int(H),
+         c_int(dk), c_int(dv), c_int(int(read_after_update)), _ptr(scratch), _stream())
     _launches += 2
 
 

@@ -25,8 +25,7 @@ def _scan(ctx: StepContext, q, k, v, z, z_bias, form: str, tau: float, q_scale: 
     walks = chunks is None or chunks.others
     # where the chunk kernels serve all requests, operands that need no arithmetic are read where they were projected
     whole = not walks and K.decay_prep_selective(q, k, v, z, z_bias, dk, dv, prep.get("rot_dims", 0))
-    stays = {"q": whole and q.splits == 1 and q_scale == 1.0 and not prep.get("rot_dims"),
-             "k": whole and k.splits == 1 and prep.get("k_scale", 1.0) == 1.0 and not prep.get("rot_dims"), "v": whole and v.splits == 1}
+    unturned = whole and q.splits == 1 and not prep.get("rot_dims")  # (q, k and v come from one product)
     need = n * heads * (3 * dk + 2 * dv)
     buf = ctx.workspace.get("decay_scan", need, torch.float32) if ctx.workspace is not None else torch.empty(need, dtype=torch.float32, device=dev)
     at = 0
@@ -41,13 +40,15 @@ def _scan(ctx: StepContext, q, k, v, z, z_bias, form: str, tau: float, q_scale: 
         return t
 
     o, do = cut(n, heads, dv), cut(n, heads, dk)
-    qo, ko, vo = (None if stays[x] else cut(n, heads, size) for x, size in (("q", dk), ("k", dk), ("v", dv)))
+    qo = None if unturned and q_scale == 1.0 else cut(n, heads, dk)
+    ko = None if unturned and prep.get("k_scale", 1.0) == 1.0 else cut(n, heads, dk)
+    vo = None if whole and v.splits == 1 else cut(n, heads, dv)
     K.decay_prep(q, k, v, z, z_bias, form, tau, q_scale, qo, ko, do, vo, heads, dk, dv, **prep)
-    qo, ko, vo = (K.view_rows(x, n, heads, size) if x_o is None else x_o for x, x_o, size in ((q, qo, dk), (k, ko, dk), (v, vo, dv)))
     if walks:
         K.decay_scan(qo, ko, do, vo, bonus, state, ctx.cu_q, ctx.slot_ids, o, read_after_update, 0 if chunks is None else chunks.long_from)
     if chunks is not None:
-        K.chunk_scan(qo, ko, do, vo, bonus, state, ctx.slot_ids, o, read_after_update, chunks, scratch)
+        K.chunk_scan(q if qo is None else qo, k if ko is None else ko, do, v if vo is None else vo, bonus, state, ctx.slot_ids, o, read_after_update,
+                     chunks, scratch)
     return o
 
 
