@@ -66,12 +66,19 @@ def plan_scan_segments(shape: StepShape) -> dict:
 # 65 ns per token; the walk: 145 ns per token and no start).  Measured, us, walk and chunks: 16 heads 256 tokens 46 and 50,
 # 512 tokens 81 and 52, 2048 tokens 297 and 144; 32 heads 512 tokens 108 and 81; 8 requests of 256 tokens, 32 heads, 288 and 290.
 CHUNK_FROM_TOKENS = 384
-# The chunk kernels work on 128 x 128 whatever a head's sizes, the decayed walk on what there is, over more heads and requests at
-# once: from heads of this area on chunks are ahead at any number of heads and requests (112 x 112, 8 to 64 heads, 1 to 16 requests of
-# 384 to 2048 tokens: 0.32 to 1.02 of the walk's time); smaller ones take them for portions from CHUNK_FROM_SMALL on that are
-# worth up to CHUNK_CHAINS heads of the longest (72 x 72 and 96 x 96, 8 to 32 heads: 0.29 to 0.98); beyond, 72 x 72 took 0.97 to
-# 1.73 of the walk's time at 2 to 16 requests of 32 to 64 heads, and 96 x 96 0.87 to 1.31.
-CHUNK_AREA, CHUNK_FROM_SMALL, CHUNK_CHAINS = 112 * 112, 512, 32
+# When they take the decayed recurrences' portions:
+# * Two launches more and their arguments are 20 us of the host's time, which such a layer is bound by at few tokens, and requests
+#   beside the portions are walked all the same.  So the portions must be worth CHUNK_WORK heads x tokens, or CHUNK_LEAD tokens; beside
+#   others, what the longest is ahead of them counts.  A layer's pass, us, walk and chunks: 16 heads 400 tokens (retention, gated, time
+#   mixing) 121 and 138, 153 and 164, 215 and 224; 768 tokens 167 and 140, 184 and 166, 216 and 224; 1024 tokens 216 and 141, 233 and
+#   168, 249 and 225; 640 beside 360 tokens 196 and 215, 213 and 231, 236 and 253; 32 heads 400 tokens 208 and 161, 229 and 180, 221 and 223.
+# * The chunk kernels work on 128 x 128 whatever a head's sizes, the walk on what there is, over more heads and requests at once: from
+#   heads of CHUNK_AREA on chunks are ahead at any number of them (112 x 112, 8 to 64 heads, 1 to 16 requests of 384 to 2048
+#   tokens: 0.32 to 1.02 of the walk's time); smaller ones take them for portions worth CHUNK_WORK_SMALL and up to CHUNK_CHAINS heads
+#   of the longest (72 x 72 and 96 x 96, 8 to 32 heads: 0.29 to 0.98; 32 heads, 384 tokens 1.03 to 1.07); beyond, 72 x 72 took 0.97 to
+#   1.73 of the walk's time at 2 to 16 requests of 32 to 64 heads, and 96 x 96 0.87 to 1.31.
+CHUNK_WORK, CHUNK_LEAD = 12288, 1024
+CHUNK_AREA, CHUNK_WORK_SMALL, CHUNK_CHAINS = 112 * 112, 16384, 32
 
 
 def plan_scan_chunks(shape: StepShape) -> dict:
@@ -100,9 +107,13 @@ def step_chunks(ctx: StepContext) -> "K.Chunks | None":
 
 
 def decay_chunks_pay(lens, heads: int, dk: int, dv: int) -> bool:
-    """Whether a step's long portions go through the chunk kernels rather than the decayed recurrences' walk (see CHUNK_AREA)."""
-    long = [n for n in lens if n >= CHUNK_FROM_TOKENS]
-    return dk * dv >= CHUNK_AREA or (max(long) >= CHUNK_FROM_SMALL and heads * sum(long) <= CHUNK_CHAINS * max(long))
+    """Whether a step's long portions go through the chunk kernels rather than the decayed recurrences' walk (see CHUNK_WORK)."""
+    long, rest = [n for n in lens if n >= CHUNK_FROM_TOKENS], max((n for n in lens if n < CHUNK_FROM_TOKENS), default=0)
+    lead = max(long) - rest
+    small = dk * dv < CHUNK_AREA
+    if lead < CHUNK_LEAD and heads * (lead if rest else sum(long)) < (CHUNK_WORK_SMALL if small else CHUNK_WORK):
+        return False
+    return not small or heads * sum(long) <= CHUNK_CHAINS * max(long)
 
 
 def scan_chunks(ctx: StepContext, heads: int, dk: int, dv: int, pays=None) -> "tuple[K.Chunks | None, torch.Tensor | None]":

@@ -76,28 +76,35 @@ def _run(mixer, dtype, seqs, steps, slots, states, planners):
     return [torch.cat(g) for g in got]
 
 
-# a long portion alone; beside a single token and a portion one short of long (heads of 128: of small heads 512 are the least); from a
-# carried state beside others; two at once
-STEPS = [[(0, 0, 530)], [(0, 530, 531), (1, 0, 384), (2, 0, 383)], [(2, 383, 384), (0, 531, 540), (1, 384, 900)], [(0, 540, 1060), (1, 900, 1450)]]
+# a long portion alone; beside a single token and a portion one short of long; from a carried state beside others; two at once (the two
+# heads of these parts are worth the chunk kernels from 1024 tokens on, or so far ahead of the rest)
+STEPS = [[(0, 0, 1100)], [(0, 1100, 1101), (1, 0, 1430), (2, 0, 383)], [(2, 383, 384), (0, 1101, 1110), (1, 1430, 2500)], [(0, 1110, 2140), (1, 2500, 2884)]]
 KINDS = ["gated", "time_mix", "retention", "retention turned", "hgrn2", "delta"]
 
 
 @pytest.mark.parametrize("name, dtype, tol", DTYPES)
 @pytest.mark.parametrize("kind, dk, dv", [(k, 128, 128) for k in KINDS] + [("gated", 70, 100), ("time_mix", 70, 70), ("retention turned", 72, 128),
                                                                         ("hgrn2", 70, 100), ("hgrn2", 127, 65), ("delta", 72, 100)])
-def test_steps_with_long_portions_beside_others(kind, dk, dv, name, dtype, tol):
+def test_steps_with_long_portions_beside_others(kind, dk, dv, name, dtype, tol, monkeypatch):
     """Against the plain recurrence over the whole sequences, and against the same tokens walked in order (a step without the
     planner's lists); a slot of no request stays as it is."""
+    from jax_llm_examples_b200.kernels import api as K
+
     torch.manual_seed(dk + len(kind))
     mixer, plain = _mixer(kind, dtype, 2, dk, dv, 40)
-    seqs = [torch.randn(n, 40).to(dtype) for n in (1060, 1450, 384)]
+    seqs = [torch.randn(n, 40).to(dtype) for n in (2140, 2884, 384)]
     ref = [plain(s.double()) for s in seqs]
     got = {}
+    ran = []
+    for name_of in ("chunk_scan", "delta_chunk"):
+        real = getattr(K, name_of)
+        monkeypatch.setattr(K, name_of, lambda *a, real=real, **k: (ran.append(1), real(*a, **k)))
     for planned in (True, False):
         states = tuple(torch.zeros(5, *n.shape, device=DEV) for n in mixer.state_needs())
         for s in states:
             s[1] = 99.0
         got[planned] = _run(mixer, dtype, seqs, STEPS, [4, 0, 2], states, mixer.step_planners() if planned else ())
+        assert len(ran) == 4  # every step, once
         for r in range(3):
             _close(got[planned][r], ref[r], tol, f"{name} request {r} planned={planned}")
         assert all(torch.equal(s[1], torch.full_like(s[1], 99.0)) for s in states)
@@ -147,7 +154,7 @@ def test_a_decays_bias_off_16_byte_boundaries():
     """Long portions of a gated linear attention take it as ever, whatever of q, k and v is left in place."""
     torch.manual_seed(7)
     mixer, _ = _mixer("gated", torch.float32, 2, 128, 128, 40)
-    seqs, steps, outs = [torch.randn(500, 40)], [[(0, 0, 450)], [(0, 450, 500)]], []
+    seqs, steps, outs = [torch.randn(1150, 40)], [[(0, 0, 1100)], [(0, 1100, 1150)]], []
     for bias in (mixer.a_bias, _off(mixer.a_bias)):
         mixer.a_bias = bias
         states = tuple(torch.zeros(2, *n.shape, device=DEV) for n in mixer.state_needs())
@@ -159,7 +166,7 @@ def test_states_of_the_delta_rule_off_16_byte_boundaries():
     """The kernels for long portions read and write states entry by entry: slabs may start anywhere, as for the walk."""
     torch.manual_seed(7)
     mixer, _ = _mixer("delta", torch.float32, 2, 128, 128, 40)
-    seqs, steps, outs = [torch.randn(500, 40)], [[(0, 0, 450)], [(0, 450, 500)]], []
+    seqs, steps, outs = [torch.randn(1150, 40)], [[(0, 0, 1100)], [(0, 1100, 1150)]], []
     for place in (lambda s: s, _off):
         states = tuple(place(torch.zeros(2, *n.shape, device=DEV)) for n in mixer.state_needs())
         outs.append(_run(mixer, torch.float32, seqs, steps, [1], states, mixer.step_planners())[0])

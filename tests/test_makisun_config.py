@@ -175,10 +175,12 @@ def test_plain_router_takes_the_softmax_over_the_chosen_only():
 
 
 def test_which_long_portions_go_by_chunks():
-    """Heads near 128 x 128 always; smaller ones while the portions are worth few heads of the longest."""
+    """Portions worth enough heads and tokens, or far ahead of the requests beside them; of small heads few."""
     from jax_llm_examples_b200.parts.recurrent import decay_chunks_pay
 
-    for lens, heads, dk, dv, chunks in (([384], 64, 128, 128, True), ([384] * 16, 64, 112, 112, True), ([2048, 1, 300], 16, 72, 72, True),
-                                        ([511], 8, 72, 72, False), ([512], 32, 96, 96, True), ([512], 33, 96, 96, False), ([384] * 5, 32, 72, 72, False),
-                                        ([1024] * 4, 8, 128, 72, True), ([1024] * 4, 16, 72, 128, False), ([777, 500, 600], 16, 72, 72, False)):
+    for lens, heads, dk, dv, chunks in (([767], 16, 128, 128, False), ([768], 16, 128, 128, True), ([384], 32, 128, 128, True), ([1024], 2, 128, 128, True), ([500], 32, 72, 72, False),
+                                        ([384] * 16, 8, 128, 128, True), ([640, 360], 32, 128, 128, False), ([2048, 1, 300], 16, 128, 128, True),
+                                        ([777, 437, 631], 32, 128, 128, True), ([600, 1], 32, 128, 128, True), ([384], 64, 112, 112, True),
+                                        ([2048, 1, 300], 16, 72, 72, True), ([512], 32, 96, 96, True), ([512], 33, 96, 96, False),
+                                        ([384] * 5, 32, 72, 72, False), ([1024] * 4, 8, 128, 72, True), ([1024] * 4, 16, 72, 128, False)):
         assert decay_chunks_pay(lens, heads, dk, dv) == chunks, (lens, heads, dk, dv)
