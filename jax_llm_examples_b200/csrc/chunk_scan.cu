@@ -3,7 +3,8 @@
 //     S_t = diag(d_t) S_(t-1) + k_t v_t^T,   o_t = S_t^T q_t   or   o_t = (S_(t-1) + diag(u) k_t v_t^T)^T q_t.
 //
 // Walked token by token, a request's prompt is a chain of as many dependent steps on the few blocks that its state fills.
-// With chunks almost all of it is products of 64 rows, over all chunks and heads at once:
+// With chunks (the chunkwise form of S. Yang et al., "Gated Linear Attention Transformers with Hardware-Efficient Training", 2023)
+// almost all of it is products of 64 rows, over all chunks and heads at once:
 //
 //   chunk_states   what a chunk adds to a zero state, sum_t (k_t prod_{r>t} d_r) v_t^T, and the product of its decays.
 //   chunk_chain    the chunks' start states, S <- diag(prod d) S + added, chunk after chunk (the one dependent chain, of
@@ -467,11 +468,9 @@ __global__ void __launch_bounds__(CH_THREADS, 2) chunk_outputs_kernel(const __gr
   }
 }
 
-// float32 elements of scratch for n chunks.
-JLX_API long long jlx_chunk_scan_scratch(int n, int H, int dk, int dv) { return (long long)n * H * dk * (dv + 1); }
-
 // chunks: int32 [n, 3] (request, first token row, end row), at most 64 rows each; requests: int32 [m, 3] (request, first chunk,
-// chunks), every chunk in exactly one.  q, k, d, v: row pointers and strides (k null: k = 1 - d); o: [N, H, dv].
+// chunks), every chunk in exactly one.  q, k, d, v: row pointers and strides (k null: k = 1 - d); o: [N, H, dv].  scratch: n H dk
+// (dv + 1) float32 elements.
 JLX_API int jlx_chunk_scan(const float* q, long long ldq, const float* k, long long ldk, const float* d, long long ldd, const float* v,
                            long long ldv, const float* bonus, float* state, const int* slot_ids, float* o, const int* chunks, int n,
                            const int* requests, int m, int H, int dk, int dv, int read_after, float* scratch, cudaStream_t stream) {

@@ -6,7 +6,9 @@
 //
 //     (I + L) U = diag(beta) (V - diag(G) K S0),     L_ts = beta_t D_ts (k_s . k_t) for s < t,
 //
-// so U = X - Y S0 with  (I + L) X = diag(beta) V  and  (I + L) Y = diag(beta G) K,  which need no state:
+// so U = X - Y S0 with  (I + L) X = diag(beta) V  and  (I + L) Y = diag(beta G) K,  which need no state (the chunkwise form of
+// the delta rule: S. Yang et al., "Parallelizing Linear Transformers with the Delta Rule over Sequence Length", 2024; with decays:
+// "Gated Delta Networks", 2024):
 //
 //   delta_solve    X and Y of all chunks and heads at once, by forward substitution, a thread per column.
 //   delta_chain    the one dependent chain: per request, head and slice of value columns, chunk after chunk,
@@ -509,11 +511,9 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_outputs_kernel(const __gr
 
 JLX_API int jlx_delta_chunk_supported(int dk, int dv) { return dk > 64 && dk <= DC_D && dv > 64 && dv <= DC_D && dk % 4 == 0 && dv % 4 == 0; }
 
-// float32 elements of scratch for n chunks.
-JLX_API long long jlx_delta_chunk_scratch(int n, int H, int dk, int dv) { return (long long)n * H * (CHUNK * (dk + dv) + dk * dv + CHUNK + 1); }
-
 // chunks: int32 [n, 3] (request, first token row, end row), at most 64 rows each; requests: int32 [m, 3] (request, first chunk,
-// chunks), every chunk in exactly one.  All rows start on 16-byte boundaries.
+// chunks), every chunk in exactly one.  All rows but the states' start on 16-byte boundaries.  scratch: n H (CHUNK (dk + dv + 1) +
+// dk dv + 1) float32 elements.
 JLX_API int jlx_delta_chunk(const float* q, const float* k, const float* v, const float* beta, const float* decay, float* state, const int* slot_ids,
                             float* o, const int* chunks, int n, const int* requests, int m, int G, int H, int dk, int dv, float* scratch,
                             cudaStream_t stream) {

@@ -9,14 +9,15 @@
 //
 // Three kernels; which one runs is decided by sizes alone (gemm_form below):
 //
-//   gemm_f32_rows   few rows per weight matrix (decode steps, short prompts): every block streams 16 weight rows once for up
+//   gemm_f32_rows   few rows per weight matrix (decode steps, short prompts): every block streams 32 weight rows once for up
 //                   to 8 token rows; bound by the weights' bytes.
 //   gemm_f32_tile   many rows: tiles of 64 (or 32) x 128 outputs, 8 (4) x 8 per thread; bound by the FMA pipe.
 //   gemm_simt       everything that is not float32 throughout or not in whole 16-byte pieces.
 //
-// The order in which an output's K products are added follows from K alone, so that a position's result does not depend on
-// how its prompt was cut into steps.  gemm_simt adds them one by one.  The other two cut K into four parts of whole 32s;
-// a part has a strand of its even and one of its odd K, each one by one; the strands are added, then the parts in order.
+// The order in which an output's K products are added does not depend on the number of rows, so that a position's result does
+// not depend on how its prompt was cut into steps.  The two float32 kernels share one order, which follows from K alone: four
+// parts of whole 32s; a part has a strand of its even and one of its odd K, each one by one; the strands are added, then the
+// parts in order.  gemm_simt adds the products one by one; a product's types, leading dimensions and addresses send it there.
 
 #include "common.cuh"
 
