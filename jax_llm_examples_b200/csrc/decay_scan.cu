@@ -229,6 +229,8 @@ __global__ void decay_prep_kernel(RowsView q, RowsView k, RowsView v, RowsView z
 // A block's chain is longer than the other kernel's (several pieces per thread, partial sums one after the other), so it pays once
 // the tokens fill the GPU: 16 heads, all outputs, us, here and there: 1 token 5.1 and 3.2 (from 8 partial sums 7.2 and 3.3), 64 tokens
 // 5.5 and 3.4, 256 tokens 7.5 and 7.7 (from 8 partial sums 14.3 and 10.0), 512 tokens 8.7 and 13.1.
+// It lets no successor start early: the walk's few large blocks would settle while the SMs are still taken, two on one of them, and
+// stay so (32 heads, 400 tokens: a retention layer 208 us, 178 with the kernel of many blocks).
 #define PREP_MAX_ROT 512
 #define PREP_ROWS_FROM 257
 __global__ void __launch_bounds__(256)
@@ -237,7 +239,6 @@ decay_prep_x4_kernel(RowsView q, RowsView k, RowsView v, RowsView z, const float
                      const float* __restrict__ head_decay, float k_scale, const float* __restrict__ inv_freq, int rot,
                      const int* __restrict__ positions) {
   JLX_TL(TL_OTHER);
-  pdl_launch_dependents_if_small();
   __shared__ __align__(16) float sines[PREP_MAX_ROT / 2], cosines[PREP_MAX_ROT / 2];
   pdl_wait();
   const size_t n = blockIdx.x;
