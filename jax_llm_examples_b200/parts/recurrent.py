@@ -119,9 +119,9 @@ def decay_chunks_pay(lens, heads: int, dk: int, dv: int) -> bool:
 def scan_chunks(ctx: StepContext, heads: int, dk: int, dv: int, pays=None) -> "tuple[K.Chunks | None, torch.Tensor | None]":
     """The step's chunks and the scratch of their states, if it has long portions of heads that the chunk kernels take, and if
     ``pays(lengths, heads, dk, dv)`` says so."""
-    chunks = step_chunks(ctx)
-    if chunks is None or not K.chunk_scan_supported(dk, dv) or (pays is not None and not pays(ctx.host_q_lens, heads, dk, dv)):
+    if "scan_chunks" not in ctx.arrays or not K.chunk_scan_supported(dk, dv) or (pays is not None and not pays(ctx.host_q_lens, heads, dk, dv)):
         return None, None
+    chunks = step_chunks(ctx)
     need = K.chunk_scan_scratch(chunks.n, heads, dk, dv)
     return chunks, ctx.workspace.get("chunk_scan", need, torch.float32) if ctx.workspace is not None else \
         torch.empty(need, dtype=torch.float32, device=chunks.chunks.device)
